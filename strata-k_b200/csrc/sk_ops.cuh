@@ -164,7 +164,7 @@ uint64_t count_distinct_ids(strata_ctx* ctx, const uint32_t* a, uint64_t na, con
                             uint64_t nb, const uint32_t* c, uint64_t nc, uint64_t limit);
 
 // max over columns (synchronizing).
-uint32_t max_u32(strata_ctx* ctx, const uint32_t* a, uint64_t n);
+uint32_t max_u32(strata_ctx* ctx, const uint32_t* a, uint64_t n, const uint32_t* b = nullptr);  // over a and b
 
 // Pack two u32 columns into keys (c0 << shift) | c1, optional weight conversion
 // from (int64 w, u8 inf) to W codes (inf -> WInf<W>, finite v -> v - ctx->wshift).

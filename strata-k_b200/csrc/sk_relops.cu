@@ -692,10 +692,13 @@ __global__ void k_popcount(const uint32_t* __restrict__ bitmap, uint64_t words, 
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
-__global__ void k_max_u32(const uint32_t* __restrict__ a, uint64_t n, uint32_t* out) {
+// The largest value of a (and of b, when given) over n rows.
+__global__ void k_max_u32(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, uint64_t n, uint32_t* out) {
   uint32_t m = 0;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     m = a[i] > m ? a[i] : m;
+    if (b) m = b[i] > m ? b[i] : m;
+  }
   for (int o = 16; o > 0; o >>= 1) {
     const uint32_t t = __shfl_xor_sync(kFull, m, o);
     m = t > m ? t : m;
@@ -1044,11 +1047,11 @@ uint64_t count_distinct_ids(strata_ctx* ctx, const uint32_t* a, uint64_t na, con
   return r;
 }
 
-uint32_t max_u32(strata_ctx* ctx, const uint32_t* a, uint64_t n) {
+uint32_t max_u32(strata_ctx* ctx, const uint32_t* a, uint64_t n, const uint32_t* b) {
   if (n == 0) return 0;
   DBuf<uint64_t> m(ctx, 1);
   SK_CUDA(cudaMemsetAsync(m.p, 0, 8, ctx->stream));
-  k_max_u32<<<grid_for(ctx, n), NT, 0, ctx->stream>>>(a, n, reinterpret_cast<uint32_t*>(m.p));
+  k_max_u32<<<grid_for(ctx, n), NT, 0, ctx->stream>>>(a, b, n, reinterpret_cast<uint32_t*>(m.p));
   after_launch(ctx, "k_max_u32");
   uint64_t r;
   read_u64(ctx, m.p, &r, 1);

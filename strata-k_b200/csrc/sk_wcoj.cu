@@ -11,9 +11,16 @@
 // it stages out(X) in shared memory, expands the concatenation of out(Y) over
 // Y ∈ out(X) with a warp scan so the 32 lanes stream the successor lists with
 // coalesced loads, and probes each candidate Z in the staged list.
+//
+// Graphs with many candidates per edge take the hub-row plan instead
+// (k_tri_edges below): vertices are relabelled by descending degree, the part
+// of out(x) among the first T labels becomes a T-bit row, and an edge (X, Y)
+// is one AND + popcount of two rows plus a short search of the rest.
 #include "sk_ops.cuh"
 #include "sk_prims.cuh"
 #include "sk_rel.cuh"
+
+#include <type_traits>
 
 namespace sk {
 namespace {
@@ -176,6 +183,333 @@ __global__ void __launch_bounds__(TC_NT)
     if (qn > 0 && (uint32_t)lane < qn && bsearch_u32(A, du, q[lane])) count++;
     __syncwarp();
   }
+  count = warp_sum(count);
+  if (lane == 0 && count) atomicAdd(total, count);
+}
+
+// ---- hub rows ----------------------------------------------------------------
+// What bounds the probing kernels above is the candidates: Σ_{(X,Y)} |out(Y)|
+// is 30 G on R-MAT-22 (450 per edge), each costing about one lane-clock.  Most
+// of those candidates are the same few thousand vertices: with labels by
+// descending in-degree, the first 8,192 labels hold 97 % of the candidates of
+// R-MAT-20.  So out(x) is split at label T:
+//   hub part   labels < T: a T-bit row for vertices with more than 32 of them
+//              ("dense"), else the sorted list itself (at most one per lane);
+//   the rest   labels >= T: the sorted list.
+// |out(X) ∩ out(Y)| = hub part + rest, and per edge
+//   dense, dense    AND + popcount of the rows, Q = T / 4,096 uint4 a lane,
+//                   cut at the shorter row's last label;
+//   sparse, dense   one lane per listed label tests its bit of the row;
+//   sparse, sparse  every lane compares its label with the other list's;
+//   rest            X's list as a hashed bitmap in shared memory (built once
+//                   per run of edges of one X), Y's list streamed past it; the
+//                   few entries that pass are queued and binary-searched 32
+//                   at a time (searching every entry of the shorter list in
+//                   the longer one made the kernel 21.4 ms:
+//                   its 32 scattered loads a step fill the L1 pipe).
+// A warp owns a span of consecutive edges of the sorted edge list, so a vertex of any
+// degree is spread over many warps.  Measured on one B200, R-MAT-22 with 16
+// edges a node: 12.5 ms
+// (dense pairs 4.4, sparse 1.7, rest 6.4) against 95.2 ms of k_tri_count_filt;
+// T = 8,192 against 16,384: 12.5 / 14.7 ms (wider rows cost the dense pairs
+// more than they save the rest).
+constexpr uint32_t kHubNone = 0xffffffffu;
+constexpr uint32_t kHubSparse = 32;  // hub labels up to which the list is kept (one per lane)
+
+// Degrees over every step-th row of the raw columns (repeats included: the
+// labels only decide how the work is laid out, never the result).  The sample
+// is at least two rows per vertex; all 67 M rows of R-MAT-22 took 0.91 ms, most
+// of it same-address atomics.  dout may equal din (undirected); self-loops do
+// not count there.
+__global__ void k_hub_degree(const uint32_t* __restrict__ x, const uint32_t* __restrict__ y, uint64_t n, uint32_t step,
+                             uint32_t* din, uint32_t* dout, int undirected) {
+  for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * step; i < n;
+       i += (uint64_t)gridDim.x * blockDim.x * step) {
+    const uint32_t a = x[i], b = y[i];
+    if (undirected && a == b) continue;
+    atomicAdd(&dout[a], 1u);
+    atomicAdd(&din[b], 1u);
+  }
+}
+
+// out[0] = Σ_v in(v)·out(v), the candidates of the probing plan; out[1] = the
+// rows whose Y has at least `heavy` in-edges.
+__global__ void k_hub_candidates(const uint32_t* __restrict__ din, const uint32_t* __restrict__ dout, uint64_t n_nodes,
+                                 uint32_t heavy, unsigned long long* out) {
+  unsigned long long s = 0, h = 0;
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n_nodes; v += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t d = din[v];
+    s += (unsigned long long)d * dout[v];
+    h += d >= heavy ? d : 0u;
+  }
+  s = warp_sum(s);
+  h = warp_sum(h);
+  if ((threadIdx.x & 31) == 0) {
+    if (s) atomicAdd(&out[0], s);
+    if (h) atomicAdd(&out[1], h);
+  }
+}
+
+__global__ void k_hub_sort_keys(const uint32_t* __restrict__ deg, uint64_t n_nodes, uint32_t* __restrict__ keys,
+                                uint32_t* __restrict__ ids) {
+  const uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= n_nodes) return;
+  keys[v] = ~deg[v];  // ascending keys = descending degree
+  ids[v] = (uint32_t)v;
+}
+
+__global__ void k_hub_labels(const uint32_t* __restrict__ order, uint64_t n_nodes, uint32_t* __restrict__ label) {
+  const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < n_nodes) label[order[r]] = (uint32_t)r;
+}
+
+// Labelled edge keys: (label(x) << bits) | label(y) as given, or (undirected)
+// from the larger label, the lower degree, to the smaller; self-loops become
+// the all-ones key, which no real edge can take and which sorts last.
+template <class K>
+__global__ void k_hub_pack(const uint32_t* __restrict__ x, const uint32_t* __restrict__ y, uint64_t n,
+                           const uint32_t* __restrict__ label, int bits, int undirected, K* __restrict__ keys) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t a = label[x[i]], b = label[y[i]];
+  const K sent = (K)((K(1) << bits) - 1);
+  if (!undirected) keys[i] = (K)(((K)a << bits) | b);
+  else if (a == b) keys[i] = (K)((sent << bits) | sent);
+  else keys[i] = a > b ? (K)(((K)a << bits) | b) : (K)(((K)b << bits) | a);
+}
+
+// Per vertex {CSR start, degree, hub count | (128-label blocks used << 16), row slot or none}.
+__global__ void k_hub_meta(const uint32_t* __restrict__ off, const uint32_t* __restrict__ nbr, uint64_t n_nodes,
+                           uint32_t T, uint4* __restrict__ meta, uint32_t* n_dense) {
+  const uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  uint4 mt = make_uint4(0u, 0u, 0u, kHubNone);
+  bool dense = false;
+  if (u < n_nodes) {
+    const uint32_t a = off[u], d = off[u + 1] - a;
+    uint32_t lo = 0, hi = d;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (nbr[a + mid] < T) lo = mid + 1; else hi = mid;
+    }
+    dense = lo > kHubSparse;
+    mt.x = a;
+    mt.y = d;
+    mt.z = lo | (lo ? ((nbr[a + lo - 1] >> 7) + 1) << 16 : 0u);
+  }
+  const unsigned bal = __ballot_sync(kFull, dense);
+  uint32_t base = 0;
+  if (lane == 0 && bal) base = atomicAdd(n_dense, (uint32_t)__popc(bal));
+  base = __shfl_sync(kFull, base, 0);
+  if (dense) mt.w = base + __popc(bal & lanemask_lt());
+  if (u < n_nodes) meta[u] = mt;
+}
+
+// The dense vertices' rows, a warp per `per` vertices, built in shared memory.
+template <int Q>
+__global__ void __launch_bounds__(TC_NT) k_hub_rows(const uint32_t* __restrict__ nbr, const uint4* __restrict__ meta,
+                                                    uint64_t n_nodes, uint32_t per, uint32_t n_rows,
+                                                    uint4* __restrict__ rows) {
+  __shared__ uint4 s_row[TC_WARPS][Q * 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t* w = reinterpret_cast<uint32_t*>(s_row[warp]);
+  const uint64_t nw = (uint64_t)gridDim.x * TC_WARPS;
+  for (uint64_t g = (uint64_t)blockIdx.x * TC_WARPS + warp; g * per < n_nodes; g += nw) {
+    const uint64_t u = g * per + lane;
+    const uint4 mine =
+        (uint32_t)lane < per && u < n_nodes ? meta[u] : make_uint4(0u, 0u, 0u, kHubNone);
+    for (unsigned dm = __ballot_sync(kFull, mine.w < n_rows); dm; dm &= dm - 1) {
+      const int t = __ffs(dm) - 1;
+      const uint32_t a = __shfl_sync(kFull, mine.x, t), h = __shfl_sync(kFull, mine.z, t) & 0xffffu;
+      const uint32_t slot = __shfl_sync(kFull, mine.w, t);
+#pragma unroll
+      for (int q = 0; q < Q; q++) s_row[warp][q * 32 + lane] = make_uint4(0u, 0u, 0u, 0u);
+      __syncwarp();
+      for (uint32_t k = lane; k < h; k += 32) {
+        const uint32_t z = nbr[a + k];  // < T by the split
+        atomicOr(&w[z >> 5], 1u << (z & 31));
+      }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < Q; q++) rows[(uint64_t)slot * (Q * 32) + q * 32 + lane] = s_row[warp][q * 32 + lane];
+      __syncwarp();
+    }
+  }
+}
+
+// Σ over the edges (X, Y) of |out(X) ∩ out(Y)|; with `orig`, only X whose
+// original id lies in [x_lo, x_hi).
+template <class K, int Q>
+__global__ void __launch_bounds__(TC_NT, 4)
+    k_tri_edges(const K* __restrict__ keys, uint64_t m, int bits, uint32_t span, const uint32_t* __restrict__ nbr,
+                const uint4* __restrict__ meta, const uint4* __restrict__ rows, const uint32_t* __restrict__ orig,
+                uint32_t x_lo, uint32_t x_hi, unsigned long long* total) {
+  __shared__ __align__(16) uint32_t s_filt[TC_WARPS][TF_WORDS];
+  __shared__ uint32_t s_q[TC_WARPS][64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = lanemask_lt();
+  uint32_t* F = s_filt[warp];
+  uint32_t* q = s_q[warp];
+  const uint64_t nw = (uint64_t)gridDim.x * TC_WARPS;
+  const K mask = (K)((K(1) << bits) - 1);
+  const uint32_t* rows32 = reinterpret_cast<const uint32_t*>(rows);
+  unsigned long long count = 0;
+  uint32_t cur = kHubNone;  // the X whose row is in ra
+  uint4 ra[Q];
+  uint32_t fx = kHubNone, fn = 0, qn = 0;  // CSR start and length of the filter's list, queued entries
+  for (uint64_t g = ((uint64_t)blockIdx.x * TC_NT + threadIdx.x) >> 5; g * span < m; g += nw) {
+    const uint64_t e1 = (g + 1) * span < m ? (g + 1) * span : m;
+    for (uint64_t e0 = g * span; e0 < e1; e0 += 32) {
+      const uint64_t e = e0 + lane;
+      uint4 a = make_uint4(0u, 0u, 0u, kHubNone), b = a;
+      if (e < e1) {
+        const K k = keys[e];
+        const uint32_t u = (uint32_t)(k >> bits), v = (uint32_t)(k & mask);
+        bool in = true;
+        if (orig) {
+          const uint32_t o = orig[u];
+          in = o >= x_lo && o < x_hi;
+        }
+        if (in) {
+          a = meta[u];
+          b = meta[v];
+        }
+      }
+      const uint32_t ha = a.z & 0xffffu, hb = b.z & 0xffffu;
+      const bool da = a.w != kHubNone, db = b.w != kHubNone;
+      uint32_t c = 0;
+      // dense, dense: four rows of the Y side in flight; the X side changes
+      // rarely (edges are sorted by X) and stays in registers
+      unsigned md = __ballot_sync(kFull, da && db);
+      const uint32_t lim = (a.z >> 16) < (b.z >> 16) ? (a.z >> 16) : (b.z >> 16);  // 128-label blocks both can share
+      while (md) {
+        constexpr int U = Q <= 2 ? 4 : 2;
+        uint4 rb[U][Q];
+        uint32_t sa[U];
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+          const bool live = md != 0;
+          const int t = live ? __ffs(md) - 1 : 0;
+          md &= md - 1;
+          sa[j] = __shfl_sync(kFull, a.w, t);
+          const uint32_t sb = __shfl_sync(kFull, b.w, t);
+          const uint32_t lm = live ? __shfl_sync(kFull, lim, t) : 0u;
+          if (!live) sa[j] = kHubNone;
+#pragma unroll
+          for (int q = 0; q < Q; q++) {
+            rb[j][q] = make_uint4(0u, 0u, 0u, 0u);
+            if ((uint32_t)(q * 32 + lane) < lm) rb[j][q] = rows[(uint64_t)sb * (Q * 32) + q * 32 + lane];
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+          if (sa[j] == kHubNone) break;
+          if (sa[j] != cur) {
+            cur = sa[j];
+#pragma unroll
+            for (int q = 0; q < Q; q++) ra[q] = rows[(uint64_t)cur * (Q * 32) + q * 32 + lane];
+          }
+#pragma unroll
+          for (int q = 0; q < Q; q++)
+            c += __popc(ra[q].x & rb[j][q].x) + __popc(ra[q].y & rb[j][q].y) + __popc(ra[q].z & rb[j][q].z) +
+                 __popc(ra[q].w & rb[j][q].w);
+        }
+      }
+      // one side dense: one lane per label of the sparse side's list
+      const uint32_t l_off = da ? b.x : a.x, l_h = da ? hb : ha, d_slot = da ? a.w : b.w;
+      for (unsigned m1 = __ballot_sync(kFull, da != db && l_h != 0); m1;) {
+        constexpr int U = 4;
+        uint32_t z[U], sl[U];
+        bool on[U];
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+          const bool live = m1 != 0;
+          const int t = live ? __ffs(m1) - 1 : 0;
+          m1 &= m1 - 1;
+          const uint32_t o = __shfl_sync(kFull, l_off, t), h = __shfl_sync(kFull, l_h, t);
+          sl[j] = __shfl_sync(kFull, d_slot, t);
+          on[j] = live && (uint32_t)lane < h;
+          z[j] = on[j] ? nbr[o + lane] : 0u;
+        }
+#pragma unroll
+        for (int j = 0; j < U; j++)
+          if (on[j]) c += (rows32[(uint64_t)sl[j] * (Q * 128) + (z[j] >> 5)] >> (z[j] & 31)) & 1u;
+      }
+      // both sparse: the lists in registers, the shorter one broadcast
+      for (unsigned m2 = __ballot_sync(kFull, !da && !db && ha != 0 && hb != 0); m2; m2 &= m2 - 1) {
+        const int t = __ffs(m2) - 1;
+        const uint32_t oa = __shfl_sync(kFull, a.x, t), na = __shfl_sync(kFull, ha, t);
+        const uint32_t ob = __shfl_sync(kFull, b.x, t), nb = __shfl_sync(kFull, hb, t);
+        const uint32_t za = (uint32_t)lane < na ? nbr[oa + lane] : kHubNone;
+        const uint32_t zb = (uint32_t)lane < nb ? nbr[ob + lane] : kHubNone;
+        const uint32_t zl = na > nb ? za : zb, zs = na > nb ? zb : za, ns = na > nb ? nb : na;
+        for (uint32_t k = 0; k < ns; k++) c += zl == __shfl_sync(kFull, zs, (int)k) ? 1u : 0u;
+      }
+      // labels from T on: X's list as a filter, Y's lists streamed past it
+      const uint32_t la = a.y - ha, lb = b.y - hb;
+      const uint32_t ra0 = a.x + ha, rb0 = b.x + hb;
+      for (unsigned m3 = __ballot_sync(kFull, la != 0 && lb != 0); m3;) {
+        const int t0 = __ffs(m3) - 1;
+        const uint32_t x0 = __shfl_sync(kFull, ra0, t0);
+        if (x0 != fx) {  // a new X: finish the queue against the old list, rebuild the filter
+          if ((uint32_t)lane < qn && bsearch_u32(nbr + fx, fn, q[lane])) c++;
+          qn = 0;
+          fx = x0;
+          fn = __shfl_sync(kFull, la, t0);
+          __syncwarp();
+          reinterpret_cast<uint4*>(F)[lane] = make_uint4(0u, 0u, 0u, 0u);
+          reinterpret_cast<uint4*>(F)[lane + 32] = make_uint4(0u, 0u, 0u, 0u);
+          __syncwarp();
+          for (uint32_t k = lane; k < fn; k += 32) {
+            const uint32_t z = nbr[fx + k];
+            atomicOr(&F[(z >> 5) & (TF_WORDS - 1)], 1u << (z & 31));
+          }
+          __syncwarp();
+        }
+        // this X's edges: their lists as one stream of 32-entry pieces, four in flight
+        unsigned same = m3 & __ballot_sync(kFull, ra0 == fx);
+        m3 &= ~same;
+        uint32_t o = 0, n = 0;  // the rest of the list being streamed
+        while (n != 0 || same != 0) {
+          constexpr int U = 4;
+          uint32_t z[U];
+          bool ok[U];
+#pragma unroll
+          for (int j = 0; j < U; j++) {
+            if (n == 0 && same != 0) {
+              const int t = __ffs(same) - 1;
+              same &= same - 1;
+              o = __shfl_sync(kFull, rb0, t);
+              n = __shfl_sync(kFull, lb, t);
+            }
+            ok[j] = (uint32_t)lane < n;
+            z[j] = ok[j] ? nbr[o + lane] : 0u;
+            const uint32_t took = n < 32 ? n : 32;
+            o += took;
+            n -= took;
+          }
+#pragma unroll
+          for (int j = 0; j < U; j++) {
+            const bool pass = ok[j] && ((F[(z[j] >> 5) & (TF_WORDS - 1)] >> (z[j] & 31)) & 1u);
+            const unsigned bal = __ballot_sync(kFull, pass);
+            if (bal == 0) continue;
+            if (pass) q[qn + __popc(bal & lt)] = z[j];
+            qn += __popc(bal);
+            __syncwarp();
+            if (qn >= 32) {
+              if (bsearch_u32(nbr + fx, fn, q[lane])) c++;
+              __syncwarp();
+              if ((uint32_t)lane + 32 < qn) q[lane] = q[lane + 32];
+              qn -= 32;
+              __syncwarp();
+            }
+          }
+        }
+      }
+      count += c;
+    }
+  }
+  if ((uint32_t)lane < qn && bsearch_u32(nbr + fx, fn, q[lane])) count++;
   count = warp_sum(count);
   if (lane == 0 && count) atomicAdd(total, count);
 }
@@ -420,6 +754,9 @@ __global__ void k_intern_map(const uint64_t* __restrict__ keys, uint64_t n, cons
 }
 
 inline unsigned blocks(uint64_t n, int nt = 256) { return (unsigned)ceil_div(n ? n : 1, nt); }
+inline unsigned grid_of(strata_ctx* ctx, uint64_t n) {  // grid-stride kernels
+  return (unsigned)std::min<uint64_t>(blocks(n), (uint64_t)ctx->num_sms * 16);
+}
 
 // Σ over oriented edges (u, v) of d+(u) + d+(v): the successor-list entries
 // the triangle count streams (its algorithmic bytes; profiling only).
@@ -452,6 +789,17 @@ uint64_t sort_unique(strata_ctx* ctx, DBuf<K>& keys, uint64_t n, int bits, DBuf<
   uint64_t r;
   read_u64(ctx, cnt.p, &r, 1);
   return r;
+}
+
+// The count of sorted unique keys without the self-loops' all-ones key, which sorts last.
+template <class K>
+uint64_t drop_loops(strata_ctx* ctx, const DBuf<K>& keys, uint64_t m, int bits) {
+  if (!m) return 0;
+  K last;
+  SK_CUDA(cudaMemcpyAsync(&last, keys.p + (m - 1), sizeof(K), cudaMemcpyDeviceToHost, ctx->stream));
+  SK_CUDA(cudaStreamSynchronize(ctx->stream));
+  const K sent = (K)((K(1) << bits) - 1);
+  return last == (K)((sent << bits) | sent) ? m - 1 : m;
 }
 
 // Count via the warp-per-vertex kernel over a CSR built from sorted unique keys.
@@ -502,11 +850,160 @@ uint64_t tri_from_sorted(strata_ctx* ctx, const K* keys, uint64_t m, int bits, u
   return r;
 }
 
+// ---- hub-row plan, host side ---------------------------------------------------
+// Where the plan applies (one B200, us a call, hub rows against probing):
+//   pattern   172 k edges with 53 candidates each 353 / 373, 259 k with 40
+//             374 / 319, 1 M with 62 559 / 656, 4.2 M with 95 1,192 / 2,211,
+//             67 M with 450 18,900 / 101,000
+//   both      without skew the labels beyond the rows dominate: uniform graphs
+//             of 4.2 M edges with 11 candidates 1,057 / 674, 12.6 M with 32
+//             3,236 / 2,167
+//   undirected  the labels also save a sort: 15 k edges 327 / 303, 40 k 343 /
+//             365, 172 k 470 / 624, 4.2 M 4,797 / 6,468
+// so: from 2^18 directed and 2^15 undirected edges on, with at least 48
+// candidates an edge (directed), and with the rows covering the columns: few
+// enough vertices, or a quarter of the edges ending in vertices of at least
+// eight times the mean in-degree.
+constexpr uint64_t kHubMinDirected = 1ull << 18, kHubMinUndirected = 1ull << 15;
+constexpr uint64_t kHubMinCandidates = 48;
+constexpr uint64_t kHubMaxNodes = 1ull << 27;  // above, the per-vertex tables outgrow their use
+
+// Device bytes the plan needs beside the edge keys (an upper bound on the rows).
+inline uint64_t hub_bytes(uint64_t n, uint64_t n_nodes, int q) {
+  return n_nodes * (6 * 4 + 16) + (n / (kHubSparse + 1) + 1) * (uint64_t)q * 512 + (1ull << 20);
+}
+
+// Stride of the degree sample.
+inline uint32_t hub_step(uint64_t n, uint64_t n_nodes) {
+  return (uint32_t)std::max<uint64_t>(1, n / std::max<uint64_t>(1ull << 17, 2 * n_nodes));
+}
+
+inline int hub_q(uint64_t n_nodes) { return n_nodes <= 4096 ? 1 : 2; }
+
+// The plan applies: default probe, sizes in range, and its memory within the context's cap.
+inline bool hub_fits(strata_ctx* ctx, uint64_t n, uint64_t n_min, uint64_t n_nodes, size_t key_bytes) {
+  if (ctx->tune_tri_probe != 0 || n < n_min || n_nodes > kHubMaxNodes) return false;
+  return !ctx->cap || ctx->in_use + n * (3 * key_bytes + 4) + hub_bytes(n, n_nodes, hub_q(n_nodes)) <= ctx->cap;
+}
+
+// Sampled degrees (step rows apart) and what they say of the graph: candidates
+// and heavy rows as k_hub_candidates counts them.
+struct HubSample {
+  uint32_t step;
+  uint64_t rows, candidates, heavy;
+  bool covered(uint64_t n_nodes) const { return n_nodes <= hub_q(n_nodes) * 4096ull || heavy * 4 >= rows; }
+};
+HubSample hub_sample(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uint64_t n, uint64_t n_nodes,
+                     bool undirected, DBuf<uint32_t>& deg) {
+  // din, then dout (directed), then the two sums
+  const uint64_t half = (n_nodes + 3) & ~3ull, words = half * (undirected ? 1 : 2);
+  deg.reserve(words + 4);
+  SK_CUDA(cudaMemsetAsync(deg.p, 0, (words + 4) * 4, ctx->stream));
+  uint32_t* din = deg.p;
+  uint32_t* dout = undirected ? deg.p : deg.p + half;
+  auto* sums = reinterpret_cast<unsigned long long*>(deg.p + words);
+  HubSample r{hub_step(n, n_nodes), 0, 0, 0};
+  r.rows = ceil_div(n, r.step);
+  k_hub_degree<<<grid_of(ctx, r.rows), 256, 0, ctx->stream>>>(x, y, n, r.step, din, dout, undirected ? 1 : 0);
+  after_launch(ctx, "k_hub_degree");
+  const uint64_t ends = undirected ? 2 * r.rows : r.rows;
+  k_hub_candidates<<<grid_of(ctx, n_nodes), 256, 0, ctx->stream>>>(
+      din, dout, n_nodes, (uint32_t)std::min<uint64_t>(8 * ceil_div(ends, n_nodes), 0xffffffffull), sums);
+  after_launch(ctx, "k_hub_candidates");
+  uint64_t h[2];
+  read_u64(ctx, reinterpret_cast<const uint64_t*>(sums), h, 2);
+  r.candidates = h[0];
+  r.heavy = undirected ? h[1] / 2 : h[1];
+  return r;
+}
+
+// Labels by descending degree: label[v], and (optional) order[label] = v.
+void hub_labels(strata_ctx* ctx, const uint32_t* deg, uint64_t n_nodes, DBuf<uint32_t>& label, DBuf<uint32_t>* order) {
+  DBuf<uint32_t> k(ctx, n_nodes), ka(ctx, n_nodes), id(ctx, n_nodes), ia(ctx, n_nodes);
+  k_hub_sort_keys<<<blocks(n_nodes), 256, 0, ctx->stream>>>(deg, n_nodes, k.p, id.p);
+  after_launch(ctx, "k_hub_sort_keys");
+  uint32_t *kp = k.p, *kalt = ka.p, *vp = id.p, *valt = ia.p;
+  radix_sort<uint32_t, uint32_t>(ctx, &kp, &kalt, &vp, &valt, true, n_nodes, 32, true);
+  label.reserve(n_nodes);
+  k_hub_labels<<<blocks(n_nodes), 256, 0, ctx->stream>>>(vp, n_nodes, label.p);
+  after_launch(ctx, "k_hub_labels");
+  if (order) *order = vp == id.p ? std::move(id) : std::move(ia);
+}
+
+// Count over sorted unique labelled keys.
+template <class K>
+uint64_t hub_count(strata_ctx* ctx, const K* keys, uint64_t m, int bits, uint64_t n_nodes, const uint32_t* orig,
+                   uint32_t x_lo, uint32_t x_hi) {
+  DBuf<uint32_t> off(ctx, n_nodes + 1), nbr(ctx, m + 1);
+  build_csr<K>(ctx, keys, m, bits, n_nodes, off.p, nbr.p);
+  DBuf<uint64_t> acc(ctx, 3);  // count, dense vertices, list-entry sum (profiling)
+  SK_CUDA(cudaMemsetAsync(acc.p, 0, 24, ctx->stream));
+  DBuf<uint4> meta(ctx, n_nodes);
+  const int q = hub_q(n_nodes);
+  k_hub_meta<<<blocks(n_nodes), 256, 0, ctx->stream>>>(off.p, nbr.p, n_nodes, (uint32_t)q * 4096u, meta.p,
+                                                       reinterpret_cast<uint32_t*>(acc.p + 1));
+  after_launch(ctx, "k_hub_meta");
+  uint64_t nd = 0;
+  read_u64(ctx, acc.p + 1, &nd, 1);
+  DBuf<uint4> rows(ctx, nd * (uint64_t)q * 32 + 1);
+  auto run = [&](auto qt) {
+    constexpr int Q = decltype(qt)::value;
+    if (nd) {
+      // few vertices a warp while the grid is not full, else a lane each
+      const uint32_t per = n_nodes >= (uint64_t)ctx->num_sms * 8 * TC_NT ? 32 : 2;
+      const unsigned rg = (unsigned)std::min<uint64_t>(ceil_div(n_nodes, per * TC_WARPS), (uint64_t)ctx->num_sms * 8);
+      k_hub_rows<Q><<<rg, TC_NT, 0, ctx->stream>>>(nbr.p, meta.p, n_nodes, per, (uint32_t)nd, rows.p);
+      after_launch(ctx, "k_hub_rows");
+    }
+    // consecutive edges a warp takes at a time: as many as leave eight turns per resident warp
+    const uint64_t warps = (uint64_t)ctx->num_sms * 4 * TC_WARPS;
+    const uint32_t span = 32 * (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(16, m / (warps * 32 * 8)));
+    const unsigned g = (unsigned)std::min<uint64_t>(ceil_div(m, (uint64_t)span * TC_WARPS), (uint64_t)ctx->num_sms * 4);
+    const int kh = kprof_begin(ctx, K_TRI_COUNT);
+    k_tri_edges<K, Q><<<g, TC_NT, 0, ctx->stream>>>(keys, m, bits, span, nbr.p, meta.p, rows.p, orig, x_lo, x_hi,
+                                                    reinterpret_cast<unsigned long long*>(acc.p));
+    kprof_end(ctx, kh, 8 * m + 4 * (n_nodes + 1));  // as tri_from_sorted counts them; the list sum is added below
+    after_launch(ctx, "k_tri_edges");
+  };
+  if (q == 1) run(std::integral_constant<int, 1>{});
+  else if (q == 2) run(std::integral_constant<int, 2>{});
+  else run(std::integral_constant<int, 4>{});
+  if (ctx->profiling) {
+    k_tri_list_sum<K><<<(unsigned)std::min<uint64_t>(blocks(m), (uint64_t)ctx->num_sms * 8), 256, 0, ctx->stream>>>(
+        keys, m, bits, off.p, n_nodes, reinterpret_cast<unsigned long long*>(acc.p + 2));
+    after_launch(ctx, "k_tri_list_sum");
+  }
+  SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, acc.p, 24, cudaMemcpyDeviceToHost, ctx->stream));
+  sync_and_check(ctx);
+  const uint64_t r = ctx->h_scalar[0];
+  if (ctx->profiling) kprof_add_last(ctx, K_TRI_COUNT, 4 * ctx->h_scalar[2]);
+  kprof_collect(ctx);
+  return r;
+}
+
 template <class K>
 uint64_t pattern_impl(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uint64_t n, int b,
                       uint64_t n_nodes, uint64_t u_lo = 0, uint64_t u_hi = ~0ull) {
+  if (u_hi > n_nodes) u_hi = n_nodes;
+  if (u_lo >= u_hi) return 0;
   DBuf<K> keys(ctx, n + 1), uniq;
   uniq.ctx = ctx;
+  if (hub_fits(ctx, n, kHubMinDirected, n_nodes, sizeof(K))) {
+    DBuf<uint32_t> deg;
+    deg.ctx = ctx;
+    const HubSample hs = hub_sample(ctx, x, y, n, n_nodes, false, deg);
+    const double cand = (double)hs.candidates * hs.step * hs.step;
+    if (cand >= (double)kHubMinCandidates * (double)n && hs.covered(n_nodes)) {
+      const bool whole = u_lo == 0 && u_hi == n_nodes;
+      DBuf<uint32_t> label, order;
+      label.ctx = order.ctx = ctx;
+      hub_labels(ctx, deg.p, n_nodes, label, whole ? nullptr : &order);
+      k_hub_pack<K><<<blocks(n), 256, 0, ctx->stream>>>(x, y, n, label.p, b, 0, keys.p);
+      after_launch(ctx, "k_hub_pack");
+      const uint64_t m = sort_unique<K>(ctx, keys, n, 2 * b, uniq);
+      return hub_count<K>(ctx, uniq.p, m, b, n_nodes, whole ? nullptr : order.p, (uint32_t)u_lo, (uint32_t)u_hi);
+    }
+  }
   pack_pairs<K, int32_t, false>(ctx, x, y, nullptr, nullptr, n, b, keys.p, nullptr);
   const uint64_t m = sort_unique<K>(ctx, keys, n, 2 * b, uniq);
   return tri_from_sorted<K>(ctx, uniq.p, m, b, n_nodes, u_lo, u_hi);
@@ -521,14 +1018,7 @@ uint64_t oriented_edges(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, u
   uniq.ctx = ctx;
   k_canon<K><<<blocks(n), 256, 0, ctx->stream>>>(a, b, n, bits, keys.p);
   after_launch(ctx, "k_canon");
-  uint64_t m = sort_unique<K>(ctx, keys, n, 2 * bits, uniq);
-  if (m) {
-    K last;
-    SK_CUDA(cudaMemcpyAsync(&last, uniq.p + (m - 1), sizeof(K), cudaMemcpyDeviceToHost, ctx->stream));
-    SK_CUDA(cudaStreamSynchronize(ctx->stream));
-    const K sent = (K)((K(1) << bits) - 1);
-    if (last == (K)((sent << bits) | sent)) m--;
-  }
+  const uint64_t m = drop_loops<K>(ctx, uniq, sort_unique<K>(ctx, keys, n, 2 * bits, uniq), bits);
   if (!by_degree || m == 0) {
     out = std::move(uniq);
     return m;
@@ -555,6 +1045,21 @@ uint64_t tri_undirected_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t*
                              uint64_t n_nodes) {
   DBuf<K> ori;
   ori.ctx = ctx;
+  if (hub_fits(ctx, n, kHubMinUndirected, n_nodes, sizeof(K))) {
+    // Any total order of the vertices counts each triangle of the simple
+    // graph once; the labels are one, so a single sort orients and dedups.
+    DBuf<uint32_t> deg, label;
+    deg.ctx = label.ctx = ctx;
+    const HubSample hs = hub_sample(ctx, a, b, n, n_nodes, true, deg);
+    hub_labels(ctx, deg.p, n_nodes, label, nullptr);
+    DBuf<K> keys(ctx, n + 1);
+    k_hub_pack<K><<<blocks(n), 256, 0, ctx->stream>>>(a, b, n, label.p, bits, 1, keys.p);
+    after_launch(ctx, "k_hub_pack");
+    const uint64_t m = drop_loops<K>(ctx, ori, sort_unique<K>(ctx, keys, n, 2 * bits, ori), bits);
+    if (m == 0) return 0;
+    if (!hs.covered(n_nodes)) return tri_from_sorted<K>(ctx, ori.p, m, bits, n_nodes);
+    return hub_count<K>(ctx, ori.p, m, bits, n_nodes, nullptr, 0, 0);
+  }
   const uint64_t m = oriented_edges<K>(ctx, a, b, n, bits, n_nodes, true, ori);
   if (m == 0) return 0;
   return tri_from_sorted<K>(ctx, ori.p, m, bits, n_nodes);
@@ -626,7 +1131,7 @@ struct Ids {
 };
 
 Ids id_space(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n) {
-  const uint32_t m = std::max(max_u32(ctx, a, n), max_u32(ctx, b, n));
+  const uint32_t m = max_u32(ctx, a, n, b);
   return Ids{std::max(1, bits_for(m)), (uint64_t)m + 1};
 }
 
