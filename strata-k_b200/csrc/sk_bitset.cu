@@ -12,20 +12,38 @@
 // Δ sets and the final relation are those of the tuple plans.
 //
 // Layout (per instance i): rows X ∈ [0, n_rows), each row W4 = ceil(n_cols /
-// 128) uint4 words; three matrices (path F, Δ and Δ' double-buffered) plus a
-// byte flag per row (Δ row non-empty) and an out-edge CSR with local ids.
+// 128) uint4 words; three matrices (path F, Δ and Δ' double-buffered), an
+// out-edge CSR with local ids, and for Δ and Δ' a summary: per row and block of
+// 32 words a mask of its nonzero words, stored block by block
+// (sum_base + block * n_rows + row).  A Δ word is read only where its summary
+// bit is set, so zero words are neither written nor cleared between rounds.
 // All instances of a wave share one pool; instance i starts at vec_base[i]
 // and row_base[i].
 //
-// Work split.  A unit is one warp over (32 / L) consecutive rows of one
-// instance, L = min(32, next power of two >= W4) lanes per row, so a
-// 100-node instance packs 32 rows into a warp and a 50,000-node instance
-// gives each row a whole warp.  Per round one persistent kernel strides its
-// warps over the units of all active instances of the wave (the unit prefix
-// over active instances is rebuilt on the device by a one-block bookkeeping
-// kernel after each round), and the host replays a captured CUDA graph of R
-// (round, bookkeeping) pairs until no instance is active — one launch per
-// semi-naive round for the whole batch, no host round trip inside the graph.
+// Work split.  Rows of at most 16 words share a warp (L = next power of two
+// >= W4 lanes per row, a unit is 32 / L rows).  Wider rows are cut into
+// blocks of 32 words, one uint4 a lane: a unit is one warp over one block of
+// a strip of up to 16 rows, the blocks outermost.  So at any time the resident
+// warps read one or two blocks of Δ (26 MB each at 50,000 nodes), which stay
+// in L2 for all the rows that join them, and one unit's metadata, CSR
+// offsets, neighbour ids and summaries are read once for its strip.
+// Per round one persistent kernel strides its warps over the units of all
+// active instances of the wave; its last block does the bookkeeping (the unit
+// prefix over active instances), and the host replays a captured CUDA graph of
+// R rounds until no instance is active — one launch per semi-naive round for
+// the whole batch, no host round trip inside the graph.  A single closure
+// launches its rounds directly (instantiating a graph costs more than it
+// saves there).
+//
+// What bounds the round: the latency of the Δ loads and, at 40 % of the issue
+// slots, the instructions around them (DRAM at 50 %); the word summaries and
+// blocks took the DRAM bytes of a dense round at 50,000 nodes and 5 edges a
+// node from about 2.6 to 1.6 GB, reading the strip's edges as one list (eight
+// Δ words and the ending rows' path words in flight) the rest.  Measured on
+// one B200 against the form with a byte flag per row and whole rows per warp:
+// that closure 6.7 -> 4.5 ms, 192 ER instances of up to 50,000 nodes (rounds
+// alone) 88.4 -> 70.3 ms.  Three blocks an SM of up to 85 registers: four of
+// 64 spill and lose 5 %, six with four words in flight 12 %.
 //
 // Summary per instance: |path| and  fp = Σ_{(X,Z) ∈ path} mix64(X) · c^Z
 // (mod 2^64, c = 0x9E3779B97F4A7C15), computed from the bit rows one 32-bit
@@ -50,39 +68,53 @@ struct BsView {
   const uint32_t* n_rows;
   const uint32_t* n_cols;
   const uint32_t* w4;
+  const uint32_t* rpu;    // rows per unit
   const uint8_t* lshift;  // log2(lanes per row)
   const uint64_t* row_base;
   const uint64_t* vec_base;
+  const uint64_t* sum_base;
+  const uint64_t* eoff;   // first edge in wave order (n + 1)
+  const uint64_t* ebase;  // first edge in the input columns
+  const uint64_t* fprefix;  // units of the summary kernel (n + 1)
   uint64_t* delta;   // |Δ'| of the current round
   uint64_t* total;   // |path| so far
+  uint64_t* counts;  // summary kernel's |path| and fingerprint
+  uint64_t* fps;
   uint32_t* rounds;
   uint8_t* active;
-  // active list and unit prefix (rebuilt by k_bs_book)
+  // active list and unit prefix (rebuilt by bs_book)
   uint32_t* act;
   uint64_t* uprefix;
-  uint32_t* n_act;
+  uint32_t* n_act;   // [0] active instances, [1] an edge endpoint was out of range
   uint64_t* u_total;
+  uint32_t* ticket;  // blocks of the running round that are done
+  uint32_t n_inst;
   // CSR over global rows, local neighbour ids
   const uint64_t* off;
   const uint32_t* nbr;
-  // matrices and row flags
+  // matrices and summaries
   uint4* F;
   uint4* D0;
   uint4* D1;
-  uint8_t* f0;
-  uint8_t* f1;
+  uint32_t* s0;
+  uint32_t* s1;
   unsigned long long* bytes;  // algorithmic bytes of the rounds (profiling), or null
-  uint32_t* status;
 };
 
 __device__ __forceinline__ uint32_t popc4(const uint4& a) {
   return __popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w);
 }
 __device__ __forceinline__ bool any4(const uint4& a) { return (a.x | a.y | a.z | a.w) != 0u; }
+__device__ __forceinline__ void or4(uint4& a, const uint4& d) {
+  a.x |= d.x;
+  a.y |= d.y;
+  a.z |= d.z;
+  a.w |= d.w;
+}
 
-// Instance slot k of unit u: uprefix[k] <= u < uprefix[k + 1].
-__device__ __forceinline__ uint32_t unit_owner(const uint64_t* uprefix, uint32_t n, uint64_t u) {
-  uint32_t lo = 0, hi = n;
+// Slot k of unit u in [lo, n): uprefix[k] <= u < uprefix[k + 1].
+__device__ __forceinline__ uint32_t unit_owner(const uint64_t* uprefix, uint32_t lo, uint32_t n, uint64_t u) {
+  uint32_t hi = n;
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
     if (uprefix[mid] <= u) lo = mid; else hi = mid;
@@ -90,113 +122,18 @@ __device__ __forceinline__ uint32_t unit_owner(const uint64_t* uprefix, uint32_t
   return lo;
 }
 
-// One semi-naive round over every active instance of the wave.  Reads Δ from
-// (D_PAR, f_PAR), writes Δ' to the other buffer pair and updates F.
-template <int PAR>
-__global__ void __launch_bounds__(BS_NT) k_bs_round(BsView v) {
-  const uint32_t n_act = *v.n_act;
-  const uint64_t U = *v.u_total;
-  const uint4* __restrict__ Dc = PAR ? v.D1 : v.D0;
-  uint4* __restrict__ Dn = PAR ? v.D0 : v.D1;
-  const uint8_t* __restrict__ fc = PAR ? v.f1 : v.f0;
-  uint8_t* __restrict__ fn = PAR ? v.f0 : v.f1;
-  const int lane = threadIdx.x & 31;
-  const uint64_t nwarps = (uint64_t)gridDim.x * (BS_NT / 32);
-  unsigned long long moved = 0;
-  for (uint64_t u = ((uint64_t)blockIdx.x * BS_NT + threadIdx.x) >> 5; u < U; u += nwarps) {
-    const uint32_t k = unit_owner(v.uprefix, n_act, u);
-    const uint32_t i = v.act[k];
-    const uint32_t n = v.n_rows[i], W = v.w4[i];
-    const int ls = v.lshift[i];
-    const uint32_t lpr = 1u << ls, sub = (uint32_t)lane >> ls, sl = (uint32_t)lane & (lpr - 1);
-    const unsigned smask = ls == 5 ? 0xffffffffu : (((1u << lpr) - 1u) << (sub << ls));
-    const uint64_t X = (u - v.uprefix[k]) * (32u >> ls) + sub;
-    const bool valid = X < n;
-    const uint64_t rb = v.row_base[i], vb = v.vec_base[i];
-    const uint64_t e0 = valid ? v.off[rb + X] : 0, e1 = valid ? v.off[rb + X + 1] : 0;
-    // Does the row join any non-empty Δ row?
-    bool any_y = false;
-    for (uint64_t e = e0 + sl; e < e1; e += lpr) {
-      const uint32_t y = v.nbr[e];
-      if (y < n && fc[rb + y]) any_y = true;
-    }
-    // every lane takes part in the ballot (lanes past the last row included)
-    const unsigned bal_y = __ballot_sync(kFull, any_y);
-    const bool row_has = valid && (bal_y & smask) != 0u;
-    bool row_any = false;
-    uint32_t cnt = 0;
-    if (row_has) {
-      uint32_t active_edges = 0, acc_words = 0;
-      for (uint32_t c = sl; c < W; c += lpr) {
-        uint4 acc = make_uint4(0u, 0u, 0u, 0u);
-        active_edges = 0;
-        // four edges at a time: their neighbour, flag and Δ-row loads are
-        // independent, so they are in flight together
-        for (uint64_t e = e0; e < e1; e += 4) {
-          uint32_t y[4];
-          bool on[4];
-#pragma unroll
-          for (int q = 0; q < 4; q++) y[q] = e + q < e1 ? v.nbr[e + q] : 0xffffffffu;
-#pragma unroll
-          for (int q = 0; q < 4; q++) on[q] = y[q] < n && fc[rb + y[q]] != 0;
-          uint4 d[4];
-#pragma unroll
-          for (int q = 0; q < 4; q++) d[q] = on[q] ? Dc[vb + (uint64_t)y[q] * W + c] : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll
-          for (int q = 0; q < 4; q++) {
-            acc.x |= d[q].x;
-            acc.y |= d[q].y;
-            acc.z |= d[q].z;
-            acc.w |= d[q].w;
-            active_edges += on[q] ? 1u : 0u;
-          }
-        }
-        uint4 nw = make_uint4(0u, 0u, 0u, 0u);
-        if (any4(acc)) {
-          acc_words++;
-          uint4* fp = v.F + vb + X * W + c;
-          uint4 f = *fp;
-          nw = make_uint4(acc.x & ~f.x, acc.y & ~f.y, acc.z & ~f.z, acc.w & ~f.w);
-          if (any4(nw)) {
-            f = make_uint4(f.x | nw.x, f.y | nw.y, f.z | nw.z, f.w | nw.w);
-            *fp = f;
-            cnt += popc4(nw);
-            row_any = true;
-          }
-        }
-        Dn[vb + X * W + c] = nw;
-      }
-      if (v.bytes) {
-        // this lane's words: Δ rows read, Δ' written, path read (and written
-        // where bits are new); its share of the edge list and flags
-        const uint64_t lw = (W > sl) ? (W - sl + lpr - 1) / lpr : 0;
-        moved += lw * 16ull * (active_edges + 1) + acc_words * 32ull + (sl == 0 ? (e1 - e0) * 5ull : 0ull);
-      }
-    }
-    const unsigned bal = __ballot_sync(kFull, row_any);
-    if (valid && sl == 0) fn[rb + X] = (bal & smask) != 0u ? 1 : 0;
-    cnt = warp_sum(cnt);
-    if (lane == 0 && cnt) atomicAdd(reinterpret_cast<unsigned long long*>(&v.delta[i]), (unsigned long long)cnt);
-  }
-  if (v.bytes) {
-    moved = warp_sum(moved);
-    if (lane == 0 && moved) atomicAdd(v.bytes, moved);
-  }
-}
-
 // After a round (or the bootstrap): close finished instances, add |Δ'| to
 // |path|, rebuild the active list and its unit prefix.  One block.
-constexpr int BK_NT = 1024;
-__global__ void __launch_bounds__(BK_NT) k_bs_book(BsView v, uint32_t n_inst, int count_round) {
-  __shared__ uint64_t s_scan[BK_NT / 32 + 1];
+__device__ void bs_book(const BsView& v, int count_round) {
+  __shared__ uint64_t s_scan[BS_NT / 32 + 1];
   __shared__ uint64_t s_carry[2];
   if (threadIdx.x == 0) s_carry[0] = s_carry[1] = 0;
   __syncthreads();
-  for (uint32_t base = 0; base < n_inst; base += BK_NT) {
+  for (uint32_t base = 0; base < v.n_inst; base += BS_NT) {
     const uint32_t i = base + threadIdx.x;
     uint64_t units = 0, act = 0;
-    if (i < n_inst && v.active[i]) {
-      const uint64_t d = v.delta[i];
+    if (i < v.n_inst && v.active[i]) {
+      const uint64_t d = __ldcg(reinterpret_cast<const unsigned long long*>(&v.delta[i]));
       v.delta[i] = 0;
       if (count_round) v.rounds[i]++;
       if (d == 0) {
@@ -204,14 +141,14 @@ __global__ void __launch_bounds__(BK_NT) k_bs_book(BsView v, uint32_t n_inst, in
       } else {
         v.total[i] += d;
         act = 1;
-        const uint32_t rpu = 32u >> v.lshift[i];
-        units = (v.n_rows[i] + rpu - 1) / rpu;
+        const uint32_t r = v.rpu[i];
+        units = (v.n_rows[i] + r - 1) / r;
+        if (v.lshift[i] == 5) units *= (v.w4[i] + 31) / 32;
       }
     }
     uint64_t tot_a, tot_u;
-    const uint64_t ex_a = block_excl_sum<BK_NT>(act, s_scan, &tot_a);
-    __syncthreads();
-    const uint64_t ex_u = block_excl_sum<BK_NT>(units, s_scan, &tot_u);
+    const uint64_t ex_a = block_excl_sum<BS_NT>(act, s_scan, &tot_a);
+    const uint64_t ex_u = block_excl_sum<BS_NT>(units, s_scan, &tot_u);
     if (act) {
       v.act[s_carry[0] + ex_a] = i;
       v.uprefix[s_carry[0] + ex_a] = s_carry[1] + ex_u;
@@ -230,6 +167,269 @@ __global__ void __launch_bounds__(BK_NT) k_bs_book(BsView v, uint32_t n_inst, in
   }
 }
 
+__global__ void __launch_bounds__(BS_NT) k_bs_book(BsView v) { bs_book(v, 0); }
+
+// Algorithmic bytes of one lane, counted in profiling runs: Δ words read, path
+// words read, path and Δ' words written.
+template <bool ON>
+struct BsMoved {
+  uint32_t d = 0, f = 0, w = 0;
+  __device__ void delta(bool x) { if (ON) d += x ? 1u : 0u; }
+  __device__ void path() { if (ON) f++; }
+  __device__ void write() { if (ON) w++; }
+  __device__ unsigned long long bytes() const { return 16ull * d + 16ull * f + 32ull * w; }
+};
+
+// The new words of one row word: acc ∖ path, path updated.
+__device__ __forceinline__ uint4 bs_new_word(const uint4& acc, uint4 f, uint4* fp) {
+  const uint4 nw = make_uint4(acc.x & ~f.x, acc.y & ~f.y, acc.z & ~f.z, acc.w & ~f.w);
+  if (any4(nw)) {
+    or4(f, nw);
+    *fp = f;
+  }
+  return nw;
+}
+
+// One semi-naive round over every active instance of the wave.  Reads Δ from
+// (D_PAR, s_PAR), writes Δ' to the other buffer pair and updates F.
+template <int PAR, bool PROF>
+__global__ void __launch_bounds__(BS_NT, 3) k_bs_round(BsView v) {
+  const uint32_t n_act = *v.n_act;
+  const uint64_t U = *v.u_total;
+  const uint4* __restrict__ Dc = PAR ? v.D1 : v.D0;
+  uint4* __restrict__ Dn = PAR ? v.D0 : v.D1;
+  const uint32_t* __restrict__ sc = PAR ? v.s1 : v.s0;
+  uint32_t* __restrict__ sn = PAR ? v.s0 : v.s1;
+  __shared__ uint4 s_ent[BS_NT / 32][32];
+  __shared__ uint32_t s_seen[BS_NT / 32][16];
+  const int lane = threadIdx.x & 31;
+  uint4* ent = s_ent[threadIdx.x >> 5];        // edges with a non-empty Δ block: Δ row, summary, row of the strip
+  uint32_t* seen_of = s_seen[threadIdx.x >> 5];  // per row of the strip: the words any of its edges has
+  const uint64_t nwarps = (uint64_t)gridDim.x * (BS_NT / 32);
+  BsMoved<PROF> mv;
+  unsigned long long moved = 0;
+  uint32_t k = 0;
+  uint64_t k_end = 0;
+  for (uint64_t u = ((uint64_t)blockIdx.x * BS_NT + threadIdx.x) >> 5; u < U; u += nwarps) {
+    if (u >= k_end) {
+      k = unit_owner(v.uprefix, k, n_act, u);
+      k_end = v.uprefix[k + 1];
+    }
+    const uint32_t i = v.act[k];
+    const uint32_t n = v.n_rows[i], W = v.w4[i], R = v.rpu[i];
+    const int ls = v.lshift[i];
+    const uint64_t rb = v.row_base[i], vb = v.vec_base[i], sb = v.sum_base[i];
+    const uint32_t ul = (uint32_t)(u - v.uprefix[k]);
+    uint32_t cnt = 0;
+    if (ls < 5) {
+      // lane group `sub` owns row X, its lane sl the row's word sl
+      const uint32_t lpr = 1u << ls, sub = (uint32_t)lane >> ls, sl = (uint32_t)lane & (lpr - 1);
+      const uint32_t X = ul * (32u >> ls) + sub;
+      const bool valid = X < n;
+      const uint64_t e0 = valid ? v.off[rb + X] : 0, e1 = valid ? v.off[rb + X + 1] : 0;
+      uint4 acc = make_uint4(0u, 0u, 0u, 0u);
+      for (uint64_t e = e0; e < e1; e += 4) {
+        uint32_t y[4], sm[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) y[q] = e + q < e1 ? v.nbr[e + q] : 0xffffffffu;
+#pragma unroll
+        for (int q = 0; q < 4; q++) sm[q] = y[q] < n ? sc[sb + y[q]] : 0u;
+        uint4 d[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const bool on = (sm[q] >> sl) & 1u;
+          d[q] = on ? Dc[vb + (uint64_t)y[q] * W + sl] : make_uint4(0u, 0u, 0u, 0u);
+          mv.delta(on);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) or4(acc, d[q]);
+      }
+      uint4 nw = make_uint4(0u, 0u, 0u, 0u);
+      if (any4(acc)) {
+        uint4* fp = v.F + vb + (uint64_t)X * W + sl;
+        nw = bs_new_word(acc, *fp, fp);
+        mv.path();
+      }
+      const bool has = any4(nw);
+      if (has) {
+        Dn[vb + (uint64_t)X * W + sl] = nw;
+        cnt = popc4(nw);
+        mv.write();
+      }
+      const unsigned bal = __ballot_sync(kFull, has);
+      if (valid && sl == 0) sn[sb + X] = (bal >> (sub << ls)) & ((1u << lpr) - 1u);
+      if (PROF && valid && sl == 0) moved += (e1 - e0) * 8ull + 4ull;
+    } else {
+      const uint32_t strips = (n + R - 1) / R;
+      const uint32_t cb = ul / strips, x0 = (ul - cb * strips) * R;
+      const uint32_t rows = n - x0 < R ? n - x0 : R;
+      const uint32_t c = cb * 32 + lane;  // this lane's word (summary bits exist only below W)
+      const uint32_t* __restrict__ sblk = sc + sb + (uint64_t)cb * n;
+      uint32_t* __restrict__ snblk = sn + sb + (uint64_t)cb * n + x0;
+      const uint4* __restrict__ dcol = Dc + vb + c;
+      uint4* __restrict__ frow = v.F + vb + (uint64_t)x0 * W + c;
+      uint4* __restrict__ drow = Dn + vb + (uint64_t)x0 * W + c;
+      // CSR offsets of the strip, one a lane (rows <= 16)
+      const uint64_t eb = v.off[rb + x0];
+      const uint32_t eo = (uint32_t)lane <= rows ? (uint32_t)(v.off[rb + x0 + lane] - eb) : 0xffffffffu;
+      const uint32_t* __restrict__ nb = v.nbr + eb;
+      uint32_t mine = 0;  // lane r: the summary of row r's new words
+      // row r done: its new words are acc outside the path word f
+      auto finish = [&](uint32_t r, const uint4& acc, const uint4& f, uint32_t seen) {
+        uint4 nw = make_uint4(0u, 0u, 0u, 0u);
+        if ((seen >> lane) & 1u) nw = bs_new_word(acc, f, frow + (uint64_t)r * W);
+        const bool has = any4(nw);
+        if (has) {
+          drow[(uint64_t)r * W] = nw;
+          cnt += popc4(nw);
+          mv.write();
+        }
+        const unsigned bal = __ballot_sync(kFull, has);
+        if ((uint32_t)lane == r) mine = bal;
+      };
+      for (uint32_t r0 = 0; r0 < rows;) {
+        // whole rows of at most 32 edges together
+        const uint32_t p0 = __shfl_sync(kFull, eo, (int)r0);
+        const uint32_t r1 = r0 + __popc(__ballot_sync(kFull, (uint32_t)lane > r0 && (uint32_t)lane <= rows && eo - p0 <= 32u));
+        if (r1 == r0) {  // one row of more than 32 edges: its windows in turn
+          const uint32_t end = __shfl_sync(kFull, eo, (int)r0 + 1);
+          uint4 acc = make_uint4(0u, 0u, 0u, 0u), f = acc;
+          uint32_t seen = 0;
+          for (uint32_t pos = p0; pos < end; pos += 32) {
+            const uint32_t y = pos + lane < end ? nb[pos + lane] : 0xffffffffu;
+            const uint32_t sm = y < n ? sblk[y] : 0u;
+            for (unsigned on = __ballot_sync(kFull, sm != 0u); on;) {
+              uint4 d[8];
+#pragma unroll
+              for (int q = 0; q < 8; q++) {
+                const int t = on ? __ffs(on) - 1 : 0;
+                const uint32_t yt = __shfl_sync(kFull, y, t), st = on ? __shfl_sync(kFull, sm, t) : 0u;
+                on &= on - 1;
+                seen |= st;
+                d[q] = make_uint4(0u, 0u, 0u, 0u);
+                if ((st >> lane) & 1u) {
+                  d[q] = dcol[(uint64_t)yt * W];
+                  mv.delta(true);
+                }
+              }
+#pragma unroll
+              for (int q = 0; q < 8; q++) or4(acc, d[q]);
+            }
+          }
+          if ((seen >> lane) & 1u) {
+            f = frow[(uint64_t)r0 * W];
+            mv.path();
+          }
+          finish(r0, acc, f, seen);
+          r0++;
+          continue;
+        }
+        const uint32_t ne = __shfl_sync(kFull, eo, (int)r1) - p0;
+        const uint32_t y = (uint32_t)lane < ne ? nb[p0 + lane] : 0xffffffffu;
+        const uint32_t sm = y < n ? sblk[y] : 0u;
+        // the row of this lane's edge: the last one that starts at or before it
+        uint32_t row = 0;
+#pragma unroll
+        for (uint32_t st = 8; st > 0; st >>= 1) {
+          const uint32_t o = __shfl_sync(kFull, eo, (int)(row + st));
+          if (row + st < r1 && o <= p0 + lane) row += st;
+        }
+        // the edges whose Δ block is not empty, compacted: N entries, `endm`
+        // those that end their row
+        const bool act = sm != 0u;
+        const unsigned A = __ballot_sync(kFull, act);
+        const uint32_t N = __popc(A), ci = __popc(A & lanemask_lt());
+        const unsigned above = A & ~(lanemask_lt() | (1u << lane));
+        const uint32_t next_row = __shfl_sync(kFull, row, above ? __ffs(above) - 1 : 0);
+        const bool last = act && (above == 0u || next_row != row);
+        const unsigned endm = __reduce_or_sync(kFull, last ? 1u << ci : 0u);
+        if (lane < 16) seen_of[lane] = 0u;
+        __syncwarp();
+        if (act) {
+          ent[ci] = make_uint4(y * W, sm, row, 0u);
+          atomicOr(&seen_of[row], sm);
+        }
+        __syncwarp();
+        // eight entries at a time, at most three row ends among them: their Δ
+        // words and the ending rows' path words are in flight together
+        uint4 acc = make_uint4(0u, 0u, 0u, 0u);
+        for (uint32_t j = 0; j < N;) {
+          uint32_t nq = N - j < 8 ? N - j : 8;
+          unsigned ends = (endm >> j) & ((1u << nq) - 1u);
+          if (__popc(ends) > 3) {
+            const unsigned e3 = ends & (ends - 1) & ((ends & (ends - 1)) - 1);  // without the first two
+            nq = __ffs(e3);
+            ends &= (1u << nq) - 1u;
+          }
+          uint4 d[8];
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            d[q] = make_uint4(0u, 0u, 0u, 0u);
+            if ((uint32_t)q < nq) {
+              const uint4 en = ent[j + q];
+              if ((en.y >> lane) & 1u) {
+                d[q] = dcol[en.x];
+                mv.delta(true);
+              }
+            }
+          }
+          uint4 f[3];
+          uint32_t fr[3], fs[3];
+          unsigned left = ends;
+#pragma unroll
+          for (int t = 0; t < 3; t++) {
+            f[t] = make_uint4(0u, 0u, 0u, 0u);
+            fr[t] = fs[t] = 0u;
+            if (left) {
+              fr[t] = ent[j + __ffs(left) - 1].z;
+              fs[t] = seen_of[fr[t]];
+              left &= left - 1;
+              if ((fs[t] >> lane) & 1u) {
+                f[t] = frow[(uint64_t)fr[t] * W];
+                mv.path();
+              }
+            }
+          }
+          int t = 0;
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            or4(acc, d[q]);
+            if ((ends >> q) & 1u) {
+              finish(t == 0 ? fr[0] : t == 1 ? fr[1] : fr[2], acc, t == 0 ? f[0] : t == 1 ? f[1] : f[2],
+                     t == 0 ? fs[0] : t == 1 ? fs[1] : fs[2]);
+              t++;
+              acc = make_uint4(0u, 0u, 0u, 0u);
+            }
+          }
+          j += nq;
+        }
+        __syncwarp();  // the entries are rewritten for the next rows
+        r0 = r1;
+      }
+      if ((uint32_t)lane < rows) snblk[lane] = mine;
+      if (PROF && (uint32_t)lane == rows) moved += eo * 8ull + rows * 12ull;
+    }
+    cnt = warp_sum(cnt);
+    if (lane == 0 && cnt) atomicAdd(reinterpret_cast<unsigned long long*>(&v.delta[i]), (unsigned long long)cnt);
+  }
+  if (PROF) {
+    moved = warp_sum(moved + mv.bytes());
+    if (lane == 0 && moved) atomicAdd(v.bytes, moved);
+  }
+  // the last block to finish does the bookkeeping (no block waits)
+  __shared__ bool s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(v.ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (threadIdx.x == 0) *v.ticket = 0;
+  bs_book(v, 1);
+}
+
 // Instance of a wave-local edge index (edge offsets relative to the wave).
 __device__ __forceinline__ uint32_t edge_owner(const uint64_t* eoff, uint32_t n_inst, uint64_t g) {
   uint32_t lo = 0, hi = n_inst;
@@ -241,14 +441,14 @@ __device__ __forceinline__ uint32_t edge_owner(const uint64_t* eoff, uint32_t n_
 }
 
 // Out-degree per global row.
-__global__ void k_bs_degree(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t m,
-                            const uint64_t* __restrict__ eoff, uint32_t n_inst, BsView v, uint32_t* deg,
-                            uint32_t* bad) {
+__global__ void k_bs_degree(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t m, BsView v,
+                            uint32_t* deg) {
   for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < m; g += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t i = edge_owner(eoff, n_inst, g);
-    const uint32_t x = src[g], y = dst[g];
+    const uint32_t i = edge_owner(v.eoff, v.n_inst, g);
+    const uint64_t e = v.ebase[i] + (g - v.eoff[i]);
+    const uint32_t x = src[e], y = dst[e];
     if (x >= v.n_rows[i] || y >= v.n_cols[i]) {
-      *bad = 1u;  // an edge endpoint outside its instance's nodes
+      v.n_act[1] = 1u;  // an edge endpoint outside its instance's nodes
       continue;
     }
     atomicAdd(&deg[v.row_base[i] + x], 1u);
@@ -276,8 +476,7 @@ __global__ void __launch_bounds__(BS_NT) k_bs_tile_sums(const uint32_t* __restri
 }
 
 __global__ void __launch_bounds__(BS_NT) k_bs_tile_write(const uint32_t* __restrict__ deg, uint64_t n,
-                                                         const uint64_t* __restrict__ sums, uint64_t* __restrict__ off,
-                                                         uint64_t* __restrict__ cursor) {
+                                                         const uint64_t* __restrict__ sums, uint64_t* __restrict__ off) {
   __shared__ uint64_t s_scan[BS_NT / 32 + 1];
   __shared__ uint64_t s_carry;
   if (threadIdx.x == 0) s_carry = sums[blockIdx.x];
@@ -288,10 +487,7 @@ __global__ void __launch_bounds__(BS_NT) k_bs_tile_write(const uint32_t* __restr
     const uint64_t d = r < n ? deg[r] : 0;
     uint64_t tot;
     const uint64_t ex = block_excl_sum<BS_NT>(d, s_scan, &tot);
-    if (r < n) {
-      off[r] = s_carry + ex;
-      cursor[r] = s_carry + ex;
-    }
+    if (r < n) off[r] = s_carry + ex;
     __syncthreads();
     if (threadIdx.x == 0) s_carry += tot;
     __syncthreads();
@@ -299,26 +495,29 @@ __global__ void __launch_bounds__(BS_NT) k_bs_tile_write(const uint32_t* __restr
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) off[n] = s_carry;
 }
 
-// Scatter edges into the CSR (order within a row is free: the round ORs) and
-// seed path = Δ0 = edge bits, counting distinct edges per instance.
-__global__ void k_bs_seed(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t m,
-                          const uint64_t* __restrict__ eoff, uint32_t n_inst, BsView v, uint64_t* cursor,
-                          uint32_t* nbr) {
+// Scatter edges into the CSR (order within a row is free: the round ORs; deg
+// counts each row's free places down) and seed path = Δ0 = edge bits with
+// their summary, counting distinct edges per instance.
+__global__ void k_bs_seed(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t m, BsView v,
+                          uint32_t* deg, uint32_t* nbr) {
   const int lane = threadIdx.x & 31;
   for (uint64_t g0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; g0 < m;
        g0 += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t g = g0 + lane;
     uint32_t fresh = 0, i = 0xffffffffu;
     if (g < m) {
-      i = edge_owner(eoff, n_inst, g);
-      const uint32_t x = src[g], y = dst[g];
+      i = edge_owner(v.eoff, v.n_inst, g);
+      const uint64_t e = v.ebase[i] + (g - v.eoff[i]);
+      const uint32_t x = src[e], y = dst[e];
       if (x < v.n_rows[i] && y < v.n_cols[i]) {
         const uint64_t row = v.row_base[i] + x;
-        nbr[atomicAdd(reinterpret_cast<unsigned long long*>(&cursor[row]), 1ull)] = y;
+        nbr[v.off[row] + (atomicSub(&deg[row], 1u) - 1u)] = y;
         uint32_t* Fw = reinterpret_cast<uint32_t*>(v.F + v.vec_base[i] + (uint64_t)x * v.w4[i]);
         const uint32_t bit = 1u << (y & 31);
         const uint32_t old = atomicOr(&Fw[y >> 5], bit);
         fresh = (old & bit) ? 0u : 1u;
+        const uint32_t c = y >> 7;
+        if (fresh) atomicOr(&v.s0[v.sum_base[i] + (uint64_t)(c >> 5) * v.n_rows[i] + x], 1u << (c & 31));
       }
     }
     // per-instance distinct-edge counts (warp-aggregated when the warp is one instance)
@@ -333,44 +532,57 @@ __global__ void k_bs_seed(const uint32_t* __restrict__ src, const uint32_t* __re
   }
 }
 
-// Δ0 row flags: a row of path0 is non-empty iff the node has out-edges.
-__global__ void k_bs_flags0(const uint64_t* __restrict__ off, uint64_t rows, uint8_t* f0) {
-  for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (uint64_t)gridDim.x * blockDim.x)
-    f0[r] = off[r + 1] > off[r] ? 1 : 0;
+// Δ0's nonzero words: every edge copies its (finished) path word.
+__global__ void k_bs_delta0(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst, uint64_t m, BsView v) {
+  for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < m; g += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t i = edge_owner(v.eoff, v.n_inst, g);
+    const uint64_t e = v.ebase[i] + (g - v.eoff[i]);
+    const uint32_t x = src[e], y = dst[e];
+    if (x >= v.n_rows[i] || y >= v.n_cols[i]) continue;
+    const uint64_t w = v.vec_base[i] + (uint64_t)x * v.w4[i] + (y >> 7);
+    v.D0[w] = v.F[w];
+  }
 }
 
 // |path| and Σ mix64(X) · c^Z per instance from the final bit rows.
-// tpw[w] = c^(32 w); tables tb[b][v] = Σ_{j ∈ bits(v)} c^(8 b + j).
+// tpw[w] = c^(32 w); tables tb[b][v] = Σ_{j ∈ bits(v)} c^(8 b + j).  Bound by
+// the integer work per 32-bit word (192 ER instances, 4.8 GB of rows: 3.4 ms).
 __global__ void __launch_bounds__(BS_NT) k_bs_final(BsView v, const uint64_t* __restrict__ tpw,
-                                                    const uint64_t* __restrict__ tb_g, uint64_t* counts,
-                                                    uint64_t* fps) {
+                                                    const uint64_t* __restrict__ tb_g) {
   __shared__ uint64_t tb[4][256];
   for (int t = threadIdx.x; t < 1024; t += BS_NT) (&tb[0][0])[t] = tb_g[t];
   __syncthreads();
-  const uint32_t n_act = *v.n_act;
-  const uint64_t U = *v.u_total;
+  const uint64_t U = v.fprefix[v.n_inst];
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = (uint64_t)gridDim.x * (BS_NT / 32);
+  uint32_t i = 0;
   for (uint64_t u = ((uint64_t)blockIdx.x * BS_NT + threadIdx.x) >> 5; u < U; u += nwarps) {
-    const uint32_t k = unit_owner(v.uprefix, n_act, u);
-    const uint32_t i = v.act[k];
+    i = unit_owner(v.fprefix, i, v.n_inst, u);
     const uint32_t n = v.n_rows[i], W = v.w4[i];
     const int ls = v.lshift[i];
     const uint32_t lpr = 1u << ls, sub = (uint32_t)lane >> ls, sl = (uint32_t)lane & (lpr - 1);
-    const uint64_t X = (u - v.uprefix[k]) * (32u >> ls) + sub;
+    const uint64_t X = (u - v.fprefix[i]) * (32u >> ls) + sub;
     uint64_t cnt = 0, poly = 0;
     if (X < n) {
       const uint4* row = v.F + v.vec_base[i] + X * W;
-      for (uint32_t c = sl; c < W; c += lpr) {
-        const uint4 q = row[c];
-        const uint32_t wd[4] = {q.x, q.y, q.z, q.w};
+      for (uint32_t c0 = sl; c0 < W; c0 += 4 * lpr) {
+        uint4 w4[4];  // four words in flight
 #pragma unroll
-        for (int h = 0; h < 4; h++) {
-          const uint32_t x = wd[h];
-          if (!x) continue;
-          cnt += __popc(x);
-          const uint64_t t = tb[0][x & 255] + tb[1][(x >> 8) & 255] + tb[2][(x >> 16) & 255] + tb[3][x >> 24];
-          poly += tpw[4 * (uint64_t)c + h] * t;
+        for (int q = 0; q < 4; q++) {
+          w4[q] = make_uint4(0u, 0u, 0u, 0u);
+          if (c0 + q * lpr < W) w4[q] = __ldcs(&row[c0 + q * lpr]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const uint32_t wd[4] = {w4[q].x, w4[q].y, w4[q].z, w4[q].w};
+          if (!any4(w4[q])) continue;
+          const uint64_t* pw = tpw + 4 * (uint64_t)(c0 + q * lpr);
+#pragma unroll
+          for (int h = 0; h < 4; h++) {
+            const uint32_t x = wd[h];
+            cnt += __popc(x);
+            poly += pw[h] * (tb[0][x & 255] + tb[1][(x >> 8) & 255] + tb[2][(x >> 16) & 255] + tb[3][x >> 24]);
+          }
         }
       }
       // splitmix64 finalizer of X
@@ -383,8 +595,8 @@ __global__ void __launch_bounds__(BS_NT) k_bs_final(BsView v, const uint64_t* __
     cnt = warp_sum(cnt);
     poly = warp_sum(poly);
     if (lane == 0) {
-      if (cnt) atomicAdd(reinterpret_cast<unsigned long long*>(&counts[i]), (unsigned long long)cnt);
-      if (poly) atomicAdd(reinterpret_cast<unsigned long long*>(&fps[i]), (unsigned long long)poly);
+      if (cnt) atomicAdd(reinterpret_cast<unsigned long long*>(&v.counts[i]), (unsigned long long)cnt);
+      if (poly) atomicAdd(reinterpret_cast<unsigned long long*>(&v.fps[i]), (unsigned long long)poly);
     }
   }
 }
@@ -395,45 +607,71 @@ inline uint32_t lanes_shift(uint32_t w4) {
   return (uint32_t)s;
 }
 
-// Fixed buffers of one call, sized for the largest wave.
+// Fixed buffers of one call, sized for the largest wave.  Everything kept per
+// instance lives in one block, which one copy fills (and zeroes) per wave.
 struct BsBuffers {
-  DBuf<uint32_t> n_rows, n_cols, w4, act, n_act, deg, bad;
-  DBuf<uint8_t> lshift, active, f0, f1;
-  DBuf<uint64_t> row_base, vec_base, delta, total, uprefix, u_total, off, cursor, eoff, sums, bytes;
-  DBuf<uint32_t> rounds, nbr;
+  DBuf<uint64_t> inst, off, sums, bytes;
+  DBuf<uint32_t> deg, nbr, s0, s1;
   DBuf<uint4> F, D0, D1;
+  std::vector<uint64_t> host;  // the block as the next wave starts
+  uint32_t n = 0;              // instances the block holds
+  // 64-bit arrays (n + 1 entries each), then 32-bit, then bytes
+  enum { ROW_BASE, VEC_BASE, SUM_BASE, EOFF, EBASE, FPREFIX, UPREFIX, DELTA, TOTAL, COUNTS, FPS, SCALARS, N64 };
+  enum { N_ROWS, N_COLS, W4, RPU, ACT, ROUNDS, N32 };
+  enum { LSHIFT, ACTIVE, N8 };
   explicit BsBuffers(strata_ctx* c) {
-    for (auto* b : {&n_rows, &n_cols, &w4, &act, &n_act, &deg, &bad, &rounds, &nbr}) b->ctx = c;
-    for (auto* b : {&lshift, &active, &f0, &f1}) b->ctx = c;
-    for (auto* b : {&row_base, &vec_base, &delta, &total, &uprefix, &u_total, &off, &cursor, &eoff, &sums, &bytes})
-      b->ctx = c;
+    for (auto* b : {&inst, &off, &sums, &bytes}) b->ctx = c;
+    for (auto* b : {&deg, &nbr, &s0, &s1}) b->ctx = c;
     F.ctx = D0.ctx = D1.ctx = c;
   }
-  BsView view(bool profile) {
-    BsView v;
-    v.n_rows = n_rows.p;
-    v.n_cols = n_cols.p;
-    v.w4 = w4.p;
-    v.lshift = lshift.p;
-    v.row_base = row_base.p;
-    v.vec_base = vec_base.p;
-    v.delta = delta.p;
-    v.total = total.p;
-    v.rounds = rounds.p;
-    v.active = active.p;
-    v.act = act.p;
-    v.uprefix = uprefix.p;
-    v.n_act = n_act.p;
-    v.u_total = u_total.p;
+  uint64_t s64() const { return n + 1; }
+  uint64_t s32() const { return (n + 2) & ~1ull; }   // entries, 8-byte multiples
+  uint64_t s8() const { return (n + 8) & ~7ull; }
+  uint64_t words() const { return N64 * s64() + N32 * s32() / 2 + N8 * s8() / 8; }
+  uint64_t* p64(uint64_t* b, int k) const { return b + k * s64(); }
+  uint32_t* p32(uint64_t* b, int k) const { return reinterpret_cast<uint32_t*>(b + N64 * s64()) + k * s32(); }
+  uint8_t* p8(uint64_t* b, int k) const {
+    return reinterpret_cast<uint8_t*>(b + N64 * s64() + N32 * s32() / 2) + k * s8();
+  }
+  void reserve_inst(uint32_t max_n) {
+    n = std::max<uint32_t>(max_n, 3);  // SCALARS holds three words
+    inst.reserve(words());
+    host.assign(words(), 0);
+  }
+  BsView view(bool profile, uint32_t n_inst) {
+    uint64_t* b = inst.p;
+    BsView v{};
+    v.n_rows = p32(b, N_ROWS);
+    v.n_cols = p32(b, N_COLS);
+    v.w4 = p32(b, W4);
+    v.rpu = p32(b, RPU);
+    v.lshift = p8(b, LSHIFT);
+    v.row_base = p64(b, ROW_BASE);
+    v.vec_base = p64(b, VEC_BASE);
+    v.sum_base = p64(b, SUM_BASE);
+    v.eoff = p64(b, EOFF);
+    v.ebase = p64(b, EBASE);
+    v.fprefix = p64(b, FPREFIX);
+    v.delta = p64(b, DELTA);
+    v.total = p64(b, TOTAL);
+    v.counts = p64(b, COUNTS);
+    v.fps = p64(b, FPS);
+    v.rounds = p32(b, ROUNDS);
+    v.active = p8(b, ACTIVE);
+    v.act = p32(b, ACT);
+    v.uprefix = p64(b, UPREFIX);
+    v.n_act = reinterpret_cast<uint32_t*>(p64(b, SCALARS));
+    v.u_total = p64(b, SCALARS) + 1;
+    v.ticket = reinterpret_cast<uint32_t*>(p64(b, SCALARS) + 2);
+    v.n_inst = n_inst;
     v.off = off.p;
     v.nbr = nbr.p;
     v.F = F.p;
     v.D0 = D0.p;
     v.D1 = D1.p;
-    v.f0 = f0.p;
-    v.f1 = f1.p;
+    v.s0 = s0.p;
+    v.s1 = s1.p;
     v.bytes = profile ? reinterpret_cast<unsigned long long*>(bytes.p) : nullptr;
-    v.status = nullptr;
     return v;
   }
 };
@@ -481,14 +719,24 @@ void poly_tables(uint64_t words, std::vector<uint64_t>& tpw, std::vector<uint64_
 
 int round_grid(strata_ctx* ctx) {
   int per_sm = 0;
-  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bs_round<0>, BS_NT, 0), "occupancy");
+  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bs_round<0, false>, BS_NT, 0), "occupancy");
   if (ctx->tune_bs_blocks > 0) per_sm = std::min(per_sm, ctx->tune_bs_blocks);
   return std::max(1, per_sm) * ctx->num_sms;
 }
 
-// Run instances `order[lo..hi)` as waves within `budget` bytes (mode 0:
-// graph-replayed batched rounds; mode 1: one instance per launch, host-driven
-// rounds).  When `keep_bits` is set (a single instance) F is left in `bufs`.
+// Rows per unit of an instance of rows wider than 16 words: as many (up to 16)
+// as leave each resident warp two units, so that one unit's metadata serves
+// several rows without leaving warps idle on a small instance.
+inline uint32_t strip_rows(uint64_t rows, uint64_t w4, uint64_t warps) {
+  uint32_t r = 1;
+  while (r < 16 && rows * ((w4 + 31) / 32) / (2 * r) >= 2 * warps) r *= 2;
+  return r;
+}
+
+// Run the instances as waves within `budget` bytes.  Mode 0: graph-replayed
+// batched rounds; 1: one instance per launch, host-driven rounds; 2: batched,
+// the rounds launched in groups of R without a graph.  F of the last wave is
+// left in `bufs`.
 void bs_run(strata_ctx* ctx, const std::vector<InstSpec>& spec, const uint32_t* d_src, const uint32_t* d_dst,
             int mode, uint64_t budget, BsBuffers& B, BsResult& R, bool want_fp) {
   const uint32_t n_inst = (uint32_t)spec.size();
@@ -508,228 +756,175 @@ void bs_run(strata_ctx* ctx, const std::vector<InstSpec>& spec, const uint32_t* 
       uint64_t bytes = inst_bytes(spec[order[a]]);
       if (bytes > budget) fail(STRATA_E_OOM, "one instance's bit matrices exceed the memory budget");
       uint32_t b = a + 1;
-      if (mode == 0)
+      if (mode != 1)
         while (b < n_inst && bytes + inst_bytes(spec[order[b]]) <= budget) bytes += inst_bytes(spec[order[b]]), b++;
       waves.push_back({a, b});
       a = b;
     }
   }
   // size the fixed buffers for the largest wave
-  uint64_t max_rows = 1, max_vecs = 1, max_edges = 1, max_w32 = 1;
+  uint64_t max_rows = 1, max_vecs = 1, max_sums = 1, max_edges = 1, max_w32 = 1;
   uint32_t max_n = 1;
   for (auto& w : waves) {
-    uint64_t rows = 0, vecs = 0, edges = 0;
+    uint64_t rows = 0, vecs = 0, sums = 0, edges = 0;
     for (uint32_t k = w.first; k < w.second; k++) {
       const InstSpec& s = spec[order[k]];
       rows += s.rows;
       vecs += inst_vecs(s);
+      sums += s.rows * ceil_div(inst_w4(s), 32);
       edges += s.e1 - s.e0;
       max_w32 = std::max<uint64_t>(max_w32, 4 * inst_w4(s));
     }
     max_rows = std::max(max_rows, rows);
     max_vecs = std::max(max_vecs, vecs);
+    max_sums = std::max(max_sums, sums);
     max_edges = std::max(max_edges, edges);
     max_n = std::max(max_n, w.second - w.first);
   }
-  B.n_rows.reserve(max_n);
-  B.n_cols.reserve(max_n);
-  B.bad.reserve(1);
-  B.w4.reserve(max_n);
-  B.lshift.reserve(max_n);
-  B.row_base.reserve(max_n);
-  B.vec_base.reserve(max_n);
-  B.delta.reserve(max_n);
-  B.total.reserve(max_n);
-  B.rounds.reserve(max_n);
-  B.active.reserve(max_n);
-  B.act.reserve(max_n);
-  B.uprefix.reserve(max_n + 1);
-  B.n_act.reserve(1);
-  B.u_total.reserve(1);
-  B.eoff.reserve(max_n + 1);
+  B.reserve_inst(max_n);
   B.deg.reserve(max_rows + 1);
   B.off.reserve(max_rows + 1);
-  B.cursor.reserve(max_rows + 1);
   B.sums.reserve(ceil_div(max_rows + 1, SC_TILE) + 2);
   B.nbr.reserve(max_edges);
-  B.f0.reserve(max_rows);
-  B.f1.reserve(max_rows);
+  B.s0.reserve(max_sums);
+  B.s1.reserve(max_sums);
   B.F.reserve(max_vecs);
   B.D0.reserve(max_vecs);
   B.D1.reserve(max_vecs);
   B.bytes.reserve(1);
-  DBuf<uint64_t> d_counts(ctx, max_n), d_fps(ctx, max_n), d_tpw(ctx, max_w32), d_tb(ctx, 1024);
-  DBuf<uint32_t> d_src_w(ctx, 1), d_dst_w(ctx, 1);
-  {
+  DBuf<uint64_t> d_tpw, d_tb;
+  d_tpw.ctx = d_tb.ctx = ctx;
+  if (want_fp) {
     std::vector<uint64_t> tpw, tb;
     poly_tables(max_w32, tpw, tb);
+    d_tpw.reserve(max_w32);
+    d_tb.reserve(1024);
     SK_CUDA(cudaMemcpyAsync(d_tpw.p, tpw.data(), tpw.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
     SK_CUDA(cudaMemcpyAsync(d_tb.p, tb.data(), 1024 * 8, cudaMemcpyHostToDevice, ctx->stream));
   }
   const bool profile = ctx->profiling;
   if (profile) SK_CUDA(cudaMemsetAsync(B.bytes.p, 0, 8, ctx->stream));
-  BsView v = B.view(profile);
-  v.status = ctx->d_status;
   const int grid = round_grid(ctx);
-  const int R_graph = ctx->tune_bs_graph_rounds > 0 ? ctx->tune_bs_graph_rounds : 8;
+  const uint64_t warps = (uint64_t)grid * (BS_NT / 32);
+  const int R_group = ctx->tune_bs_graph_rounds > 0 ? ctx->tune_bs_graph_rounds : 8;
+  auto round = [&](const BsView& v, int par) {
+    auto* kern = par == 0 ? (profile ? k_bs_round<0, true> : k_bs_round<0, false>)
+                          : (profile ? k_bs_round<1, true> : k_bs_round<1, false>);
+    kern<<<grid, BS_NT, 0, ctx->stream>>>(v);
+  };
 
-  // The graph of R_graph rounds (even, so buffer parity is the same at every
+  // The graph of R_group rounds (even, so buffer parity is the same at every
   // replay) over the fixed buffers, captured once per call.
   cudaGraphExec_t exec = nullptr;
   uint32_t graph_n_inst = 0;
-  auto capture = [&](uint32_t n_wave) {
-    if (exec && graph_n_inst == n_wave) return;
+  auto capture = [&](const BsView& v) {
+    if (exec && graph_n_inst == v.n_inst) return;
     if (exec) cudaGraphExecDestroy(exec);
     exec = nullptr;
     cudaGraph_t g;
     SK_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    for (int r = 0; r < R_graph; r += 2) {
-      k_bs_round<0><<<grid, BS_NT, 0, ctx->stream>>>(v);
-      k_bs_book<<<1, BK_NT, 0, ctx->stream>>>(v, n_wave, 1);
-      k_bs_round<1><<<grid, BS_NT, 0, ctx->stream>>>(v);
-      k_bs_book<<<1, BK_NT, 0, ctx->stream>>>(v, n_wave, 1);
-    }
+    for (int r = 0; r < R_group; r++) round(v, r & 1);
     SK_CUDA(cudaStreamEndCapture(ctx->stream, &g));
     SK_CUDA(cudaGraphInstantiate(&exec, g, 0));
     cudaGraphDestroy(g);
-    graph_n_inst = n_wave;
+    graph_n_inst = v.n_inst;
   };
 
-  std::vector<uint32_t> h_rows, h_cols, h_w4;
-  std::vector<uint8_t> h_ls, h_act;
-  std::vector<uint64_t> h_rb, h_vb, h_eoff, h_up;
-  std::vector<uint32_t> h_actl;
   for (auto& w : waves) {
     const uint32_t nw = w.second - w.first;
-    h_rows.resize(nw);
-    h_cols.resize(nw);
-    h_w4.resize(nw);
-    h_ls.resize(nw);
-    h_rb.resize(nw);
-    h_vb.resize(nw);
-    h_eoff.resize(nw + 1);
-    uint64_t rows = 0, vecs = 0, edges = 0;
+    uint64_t* h = B.host.data();
+    std::fill(B.host.begin(), B.host.end(), 0);
+    uint64_t rows = 0, vecs = 0, sums = 0, edges = 0, units = 0;
     for (uint32_t k = 0; k < nw; k++) {
       const InstSpec& s = spec[order[w.first + k]];
-      h_rows[k] = s.rows;
-      h_cols[k] = s.cols;
-      h_w4[k] = (uint32_t)inst_w4(s);
-      h_ls[k] = (uint8_t)lanes_shift(h_w4[k]);
-      h_rb[k] = rows;
-      h_vb[k] = vecs;
-      h_eoff[k] = edges;
+      const uint32_t w4 = (uint32_t)inst_w4(s), ls = lanes_shift(w4);
+      B.p32(h, B.N_ROWS)[k] = s.rows;
+      B.p32(h, B.N_COLS)[k] = s.cols;
+      B.p32(h, B.W4)[k] = w4;
+      B.p32(h, B.RPU)[k] = ls < 5 ? 32u >> ls : strip_rows(s.rows, w4, warps);
+      B.p8(h, B.LSHIFT)[k] = (uint8_t)ls;
+      B.p8(h, B.ACTIVE)[k] = 1;
+      B.p64(h, B.ROW_BASE)[k] = rows;
+      B.p64(h, B.VEC_BASE)[k] = vecs;
+      B.p64(h, B.SUM_BASE)[k] = sums;
+      B.p64(h, B.EOFF)[k] = edges;
+      B.p64(h, B.EBASE)[k] = s.e0;
+      B.p64(h, B.FPREFIX)[k] = units;
       rows += s.rows;
       vecs += inst_vecs(s);
+      sums += s.rows * ceil_div(w4, 32);
       edges += s.e1 - s.e0;
+      units += ceil_div(s.rows, 32u >> ls);
     }
-    h_eoff[nw] = edges;
-    // gather this wave's edges (contiguous per instance in the input)
-    SK_CUDA(cudaMemcpyAsync(B.n_rows.p, h_rows.data(), nw * 4, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.n_cols.p, h_cols.data(), nw * 4, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.w4.p, h_w4.data(), nw * 4, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.lshift.p, h_ls.data(), nw, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.row_base.p, h_rb.data(), nw * 8, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.vec_base.p, h_vb.data(), nw * 8, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.eoff.p, h_eoff.data(), (nw + 1) * 8, cudaMemcpyHostToDevice, ctx->stream));
-    d_src_w.reserve(edges + 1);
-    d_dst_w.reserve(edges + 1);
-    for (uint32_t k = 0; k < nw; k++) {
-      const InstSpec& s = spec[order[w.first + k]];
-      if (s.e1 > s.e0) {
-        SK_CUDA(cudaMemcpyAsync(d_src_w.p + h_eoff[k], d_src + s.e0, (s.e1 - s.e0) * 4, cudaMemcpyDeviceToDevice,
-                                ctx->stream));
-        SK_CUDA(cudaMemcpyAsync(d_dst_w.p + h_eoff[k], d_dst + s.e0, (s.e1 - s.e0) * 4, cudaMemcpyDeviceToDevice,
-                                ctx->stream));
-      }
-    }
-    SK_CUDA(cudaMemsetAsync(B.delta.p, 0, nw * 8, ctx->stream));
-    SK_CUDA(cudaMemsetAsync(B.total.p, 0, nw * 8, ctx->stream));
-    SK_CUDA(cudaMemsetAsync(B.rounds.p, 0, nw * 4, ctx->stream));
-    SK_CUDA(cudaMemsetAsync(B.active.p, 1, nw, ctx->stream));
+    B.p64(h, B.EOFF)[nw] = edges;
+    B.p64(h, B.FPREFIX)[nw] = units;
+    const BsView v = B.view(profile, nw);
+    SK_CUDA(cudaMemcpyAsync(B.inst.p, h, B.words() * 8, cudaMemcpyHostToDevice, ctx->stream));
     SK_CUDA(cudaMemsetAsync(B.deg.p, 0, (rows + 1) * 4, ctx->stream));
+    SK_CUDA(cudaMemsetAsync(B.s0.p, 0, sums * 4, ctx->stream));
     SK_CUDA(cudaMemsetAsync(B.F.p, 0, vecs * 16, ctx->stream));
-    SK_CUDA(cudaMemsetAsync(d_counts.p, 0, nw * 8, ctx->stream));
-    SK_CUDA(cudaMemsetAsync(d_fps.p, 0, nw * 8, ctx->stream));
     const unsigned eg = (unsigned)std::min<uint64_t>(ceil_div(std::max<uint64_t>(edges, 1), 256), ctx->num_sms * 16ull);
     if (edges) {
-      SK_CUDA(cudaMemsetAsync(B.bad.p, 0, 4, ctx->stream));
-      k_bs_degree<<<eg, 256, 0, ctx->stream>>>(d_src_w.p, d_dst_w.p, edges, B.eoff.p, nw, v, B.deg.p, B.bad.p);
+      k_bs_degree<<<eg, 256, 0, ctx->stream>>>(d_src, d_dst, edges, v, B.deg.p);
       after_launch(ctx, "k_bs_degree");
-      SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, B.bad.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
-      SK_CUDA(cudaStreamSynchronize(ctx->stream));
-      if ((uint32_t)ctx->h_scalar[0]) fail(STRATA_E_INVALID, "an edge endpoint lies outside its instance's nodes");
     }
     const uint64_t tiles = ceil_div(rows + 1, SC_TILE);
     k_bs_tile_sums<<<(unsigned)tiles, BS_NT, 0, ctx->stream>>>(B.deg.p, rows, B.sums.p);
     after_launch(ctx, "k_bs_tile_sums");
     scan_tile_sums(ctx, B.sums.p, tiles);
-    k_bs_tile_write<<<(unsigned)tiles, BS_NT, 0, ctx->stream>>>(B.deg.p, rows, B.sums.p, B.off.p, B.cursor.p);
+    k_bs_tile_write<<<(unsigned)tiles, BS_NT, 0, ctx->stream>>>(B.deg.p, rows, B.sums.p, B.off.p);
     after_launch(ctx, "k_bs_tile_write");
     if (edges) {
-      k_bs_seed<<<eg, 256, 0, ctx->stream>>>(d_src_w.p, d_dst_w.p, edges, B.eoff.p, nw, v, B.cursor.p, B.nbr.p);
+      k_bs_seed<<<eg, 256, 0, ctx->stream>>>(d_src, d_dst, edges, v, B.deg.p, B.nbr.p);
       after_launch(ctx, "k_bs_seed");
+      k_bs_delta0<<<eg, 256, 0, ctx->stream>>>(d_src, d_dst, edges, v);
+      after_launch(ctx, "k_bs_delta0");
     }
-    k_bs_flags0<<<(unsigned)std::min<uint64_t>(ceil_div(std::max<uint64_t>(rows, 1), 256), ctx->num_sms * 16ull), 256,
-                  0, ctx->stream>>>(B.off.p, rows, B.f0.p);
-    after_launch(ctx, "k_bs_flags0");
-    SK_CUDA(cudaMemcpyAsync(B.D0.p, B.F.p, vecs * 16, cudaMemcpyDeviceToDevice, ctx->stream));
-    k_bs_book<<<1, BK_NT, 0, ctx->stream>>>(v, nw, 0);
+    k_bs_book<<<1, BS_NT, 0, ctx->stream>>>(v);
     after_launch(ctx, "k_bs_book");
-    // rounds
+    // rounds: the host looks at the active count after every group
     const int kh = kprof_begin(ctx, K_BS_ROUND);
+    auto active = [&]() {
+      SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, v.n_act, 8, cudaMemcpyDeviceToHost, ctx->stream));
+      SK_CUDA(cudaStreamSynchronize(ctx->stream));
+      if ((uint32_t)(ctx->h_scalar[0] >> 32)) {
+        if (exec) cudaGraphExecDestroy(exec);
+        fail(STRATA_E_INVALID, "an edge endpoint lies outside its instance's nodes");
+      }
+      return (uint32_t)ctx->h_scalar[0];
+    };
     if (mode == 0) {
-      capture(nw);
-      while (true) {
-        SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, B.n_act.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
-        SK_CUDA(cudaStreamSynchronize(ctx->stream));
-        if ((uint32_t)ctx->h_scalar[0] == 0) break;
-        SK_CUDA(cudaGraphLaunch(exec, ctx->stream));
-        R.graph_launches++;
-        R.round_launches += R_graph;
-        ctx->launches += 2 * (uint64_t)R_graph;
+      if (active()) {
+        capture(v);
+        do {
+          SK_CUDA(cudaGraphLaunch(exec, ctx->stream));
+          R.graph_launches++;
+          R.round_launches += R_group;
+          ctx->launches += (uint64_t)R_group;
+        } while (active());
       }
     } else {
+      const int group = mode == 1 ? 1 : R_group;
       int par = 0;
-      while (true) {
-        SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, B.n_act.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
-        SK_CUDA(cudaStreamSynchronize(ctx->stream));
-        if ((uint32_t)ctx->h_scalar[0] == 0) break;
-        if (par == 0) k_bs_round<0><<<grid, BS_NT, 0, ctx->stream>>>(v);
-        else k_bs_round<1><<<grid, BS_NT, 0, ctx->stream>>>(v);
-        after_launch(ctx, "k_bs_round");
-        k_bs_book<<<1, BK_NT, 0, ctx->stream>>>(v, nw, 1);
-        after_launch(ctx, "k_bs_book");
-        R.round_launches++;
-        par ^= 1;
+      bool more = mode == 2 || active();  // mode 2: the first group runs before the first look
+      while (more) {
+        for (int r = 0; r < group; r++, par ^= 1) {
+          round(v, par);
+          after_launch(ctx, "k_bs_round");
+          R.round_launches++;
+        }
+        more = active() != 0;
       }
     }
     kprof_end(ctx, kh, 0);
-    // summaries: every instance of the wave as a unit range
-    h_up.resize(nw + 1);
-    h_actl.resize(nw);
-    uint64_t acc = 0;
-    for (uint32_t k = 0; k < nw; k++) {
-      h_actl[k] = k;
-      h_up[k] = acc;
-      acc += ceil_div(h_rows[k], 32u >> h_ls[k]);
-    }
-    h_up[nw] = acc;
-    const uint32_t nw32 = nw;
-    SK_CUDA(cudaMemcpyAsync(B.act.p, h_actl.data(), nw * 4, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.uprefix.p, h_up.data(), (nw + 1) * 8, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.n_act.p, &nw32, 4, cudaMemcpyHostToDevice, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(B.u_total.p, &acc, 8, cudaMemcpyHostToDevice, ctx->stream));
     if (want_fp) {
-      k_bs_final<<<grid, BS_NT, 0, ctx->stream>>>(v, d_tpw.p, d_tb.p, d_counts.p, d_fps.p);
+      k_bs_final<<<grid, BS_NT, 0, ctx->stream>>>(v, d_tpw.p, d_tb.p);
       after_launch(ctx, "k_bs_final");
     }
-    std::vector<uint64_t> c(nw), f(nw), t(nw);
-    std::vector<uint32_t> r(nw);
-    SK_CUDA(cudaMemcpyAsync(c.data(), d_counts.p, nw * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(f.data(), d_fps.p, nw * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(t.data(), B.total.p, nw * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    SK_CUDA(cudaMemcpyAsync(r.data(), B.rounds.p, nw * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    SK_CUDA(cudaMemcpyAsync(h, B.inst.p, B.words() * 8, cudaMemcpyDeviceToHost, ctx->stream));
     sync_and_check(ctx);
+    const uint64_t *c = B.p64(h, B.COUNTS), *f = B.p64(h, B.FPS), *t = B.p64(h, B.TOTAL);
+    const uint32_t* r = B.p32(h, B.ROUNDS);
     for (uint32_t k = 0; k < nw; k++) {
       const uint32_t i = order[w.first + k];
       R.counts[i] = want_fp ? c[k] : t[k];
@@ -1002,7 +1197,7 @@ uint64_t tc_bool_bitset(strata_ctx* ctx, const uint32_t* d_src, const uint32_t* 
   std::vector<InstSpec> spec{InstSpec{(uint32_t)n_src, (uint32_t)n_dst, 0, m}};
   BsBuffers B(ctx);
   BsResult R;
-  bs_run(ctx, spec, d_src, d_dst, 0, UINT64_MAX, B, R, false);
+  bs_run(ctx, spec, d_src, d_dst, 2, UINT64_MAX, B, R, false);
   *rounds = R.rounds[0];
   *round_bytes = R.bytes;
   const uint64_t n = R.totals[0];
