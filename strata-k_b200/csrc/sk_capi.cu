@@ -111,7 +111,8 @@ strata_status strata_ctx_create(int device, uint64_t mem_cap_bytes, strata_ctx**
   SK_CUDA(cudaMalloc(&ctx->d_status, 256));
   SK_CUDA(cudaMemset(ctx->d_status, 0, 256));
   SK_CUDA(cudaMallocHost(&ctx->h_status, 64));
-  SK_CUDA(cudaMallocHost(&ctx->h_scalar, 8 * sizeof(uint64_t)));
+  SK_CUDA(cudaMallocHost(&ctx->h_scalar, (8 + 32) * sizeof(uint64_t)));
+  ctx->h_group = ctx->h_scalar + 8;
   SK_CUDA(cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device));
   {
     // A pool of our own whose freed blocks stay mapped: per-round buffers are

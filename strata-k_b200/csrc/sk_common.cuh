@@ -75,6 +75,7 @@ struct strata_ctx {
   uint32_t* d_status = nullptr;     // device status word
   uint32_t* h_status = nullptr;     // pinned mirror
   uint64_t* h_scalar = nullptr;     // pinned scratch for small D2H reads (8 slots)
+  uint64_t* h_group = nullptr;      // pinned, 32 slots: a group of rounds' totals
   int num_sms = 148;
   cudaMemPool_t pool = nullptr;     // this context's pool (kept mapped between calls)
   int plan = 0;                     // 0 auto, 1 sort-merge, 2 direct-addressed

@@ -59,6 +59,32 @@ __global__ void k_tile_splits(const uint64_t* __restrict__ pos, uint64_t n, uint
   splits[t] = mp_before(pos, n, d);
 }
 
+// The same count found by one warp, 32 probes at a time.
+__device__ __forceinline__ uint64_t mp_before_warp(const uint64_t* pos, uint64_t n, uint64_t d) {
+  const int lane = threadIdx.x & 31;
+  uint64_t lo = 0, hi = d < n ? d : n;
+  while (lo < hi) {
+    const uint64_t step = (hi - lo) / 33 + 1;
+    const uint64_t mid = lo + (uint64_t)lane * step;
+    const unsigned below = __ballot_sync(kFull, mid < hi && mid + pos[mid] < d);
+    const int c = __popc(below);  // probes before d: a prefix of the lanes
+    const uint64_t first = lo;
+    if (c < 32 && first + (uint64_t)c * step < hi) hi = first + (uint64_t)c * step;
+    if (c) lo = first + (uint64_t)(c - 1) * step + 1;
+  }
+  return lo;
+}
+
+// A round's totals as the head kernel leaves them: heads and (head, edge)
+// outputs in one word (so that one atomic add reserves places in both), the
+// candidates and the Δ tuples.
+constexpr int kOutBits = 36;
+struct RoundTotals {
+  unsigned long long packed, candidates, tuples, pad;
+};
+__device__ __forceinline__ uint64_t rt_heads(unsigned long long p) { return p >> kOutBits; }
+__device__ __forceinline__ uint64_t rt_outputs(unsigned long long p) { return p & ((1ull << kOutBits) - 1); }
+
 __device__ __forceinline__ uint64_t dense_index(uint64_t key, const DenseLayout& L) {
   const uint64_t c0 = key >> L.b1, c1 = key & L.mask1;
   return L.colmajor ? c1 * L.width + c0 : c0 * L.width + c1;
@@ -117,7 +143,7 @@ __device__ __forceinline__ void atomic_min_w(int64_t* p, int64_t v) {
   atomicMin(reinterpret_cast<long long*>(p), (long long)v);
 }
 
-template <class K, bool TROP, bool WORDS, class IX, class W>
+template <class K, bool TROP, bool WORDS, class IX, class W, bool QUEUED = false>
 __global__ void __launch_bounds__(NT, 5)
     k_expand_dense(const K* __restrict__ dkeys, const W* __restrict__ dw, uint64_t n_rows,
                    const uint32_t* __restrict__ hidx, const uint64_t* __restrict__ pos,
@@ -127,7 +153,7 @@ __global__ void __launch_bounds__(NT, 5)
                    const uint32_t* __restrict__ nbr,
                    uint64_t n_nbr,
                    const W* __restrict__ nbr_w, uint64_t entries, uint32_t* bits, W* D, uint32_t* marks,
-                   int64_t wshift, uint32_t* status) {
+                   int64_t wshift, uint32_t* status, const RoundTotals* __restrict__ rt) {
   using GT = typename std::conditional<WORDS, uint32_t, uint8_t>::type;
   // IX: the index type of entries (32-bit when the index has < 2^32 entries)
   const IX ckx = (IX)ck;
@@ -147,231 +173,255 @@ __global__ void __launch_bounds__(NT, 5)
   uint16_t* s_slot = s_owner + DE_TILE;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint16_t* my_slots = s_slot + warp * (32 * kGroupMax);
+  // One tile per block with host-known sizes and precomputed splits; QUEUED:
+  // the sizes are the head kernel's totals and the blocks stride over the
+  // tiles, finding each tile's splits themselves.
+  if constexpr (QUEUED) {
+    const unsigned long long p = rt->packed;
+    n = rt_heads(p);
+    total = rt_outputs(p);
+  }
   const uint64_t L = n + total;
-  const uint64_t d0 = (uint64_t)blockIdx.x * DE_TILE;
-  const uint64_t d1 = d0 + DE_TILE < L ? d0 + DE_TILE : L;
-  const uint64_t i0 = splits[blockIdx.x], i1 = splits[blockIdx.x + 1];
-  const uint64_t a = i0 > 0 ? i0 - 1 : 0;
-  if (i1 < a || i1 - a > DE_HEADS || i1 > n || d1 < i1 || d0 < i0) {
-    if (tid == 0) atomicOr(status, ST_BOUNDS);
-    return;
-  }
-  const uint64_t o0 = d0 - i0, o1 = d1 - i1;
-  const uint32_t cnt = (uint32_t)(i1 - a);
-  for (uint32_t k = tid; k < cnt; k += NT) {
-    const uint64_t i = a + k;
-    const int64_t rel = (int64_t)pos[i] - (int64_t)o0;  // one head's degree stays below 2^31
-    if (rel < INT32_MIN || rel > INT32_MAX) atomicOr(status, ST_BOUNDS);
-    s_pos[k] = (int32_t)rel;
-    s_seg[k] = hseg[i];
-    s_h[k] = hidx[i];
-    s_g[k] = hg[i];
-  }
-  __syncthreads();
   uint32_t flags = 0;
-  // Serial merge of item events and outputs: thread t walks merged positions
-  // [d0 + t*ITEMS, ...) once and records the owner of every output it meets.
-  // Item a+k sits at merged position (a+k) + pos[a+k]; output o owned by
-  // item i sits at o + i + 1.
-  {
-    const uint64_t p0 = d0 + (uint64_t)tid * DE_ITEMS;
-    if (p0 < d1) {
-      uint32_t lo = 0, hi = cnt;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if ((int64_t)(a + mid + o0) + s_pos[mid] < (int64_t)p0) lo = mid + 1; else hi = mid;
+  for (uint64_t tile = blockIdx.x; QUEUED ? tile * DE_TILE < L : tile == blockIdx.x; tile += gridDim.x) {
+    const uint64_t d0 = tile * DE_TILE;
+    const uint64_t d1 = d0 + DE_TILE < L ? d0 + DE_TILE : L;
+    uint64_t i0, i1;
+    if constexpr (QUEUED) {
+      __shared__ uint64_t s_split[2];
+      __syncthreads();  // the previous tile's readers are done with shared memory
+      if (warp < 2) {
+        const uint64_t x = mp_before_warp(pos, n, warp ? d1 : d0);
+        if (lane == 0) s_split[warp] = x;
       }
-      uint32_t kk = lo;  // local items whose event precedes p0
-      const uint64_t p1 = p0 + DE_ITEMS < d1 ? p0 + DE_ITEMS : d1;
-      for (uint64_t p = p0; p < p1; p++) {
-        if (kk < cnt && (int64_t)(a + kk + o0) + s_pos[kk] == (int64_t)p) {
-          kk++;
-        } else {
-          const uint64_t o = p - (a + kk);
-          if (kk == 0 || o < o0 || o - o0 >= DE_TILE) flags |= ST_BOUNDS;
-          else s_owner[o - o0] = (uint16_t)(kk - 1);
-        }
-      }
+      __syncthreads();
+      i0 = s_split[0];
+      i1 = s_split[1];
+    } else {
+      i0 = splits[tile];
+      i1 = splits[tile + 1];
     }
-  }
-  __syncthreads();
-  const uint64_t o_end = o1 < total ? o1 : total;
-  for (uint64_t c = o0 + (uint64_t)warp * 32; c < o_end; c += NT) {
-    const uint64_t o = c + lane;
-    uint32_t mm = 0, v = 0;
-    W ew = 0;
-    uint64_t h = 0, kb = 0;
-    if (o < o_end) {
-      const uint32_t li = s_owner[o - o0];
-      const uint64_t e = (uint64_t)((int64_t)s_seg[li] + ((int64_t)(o - o0) - s_pos[li]));
-      if (li >= cnt || e >= n_nbr) {
-        flags |= ST_BOUNDS;
-      } else {
-        v = nbr[e];
-        if constexpr (TROP) ew = nbr_w[e];
-        h = s_h[li];
-        if constexpr (WORDS) {
-          // members: the set bits of word h, columns (h mod wpr)*32 + bit of
-          // the head's row; kb = the output index of column 0 of the word
-          mm = s_g[li];
-          const uint32_t wcol = wpr_shift >= 0 ? ((uint32_t)h & (wpr - 1u)) : (uint32_t)h % wpr;
-          kb = (uint64_t)(wcol * 32u) * ck + (uint64_t)v * cv;
-          // every member's entry (and Dprev slot) inside the index: checked
-          // once here for the highest member
-          if (h * 32 + 32 > entries || (mm && kb + (uint64_t)(31 - __clz(mm)) * ck >= entries)) {
-            flags |= ST_BOUNDS;
-            mm = 0;
-          }
-        } else {
-          const uint32_t g = s_g[li];
-          mm = g >= 32 ? kFull : (1u << g) - 1u;  // members h + r for the set bits r
-          if (g > kGroupMax || h + g > n_rows) {
-            flags |= ST_BOUNDS;
-            mm = 0;
+    const uint64_t a = i0 > 0 ? i0 - 1 : 0;
+    if (i1 < a || i1 - a > DE_HEADS || i1 > n || d1 < i1 || d0 < i0) {
+      flags |= ST_BOUNDS;
+      continue;
+    }
+    const uint64_t o0 = d0 - i0, o1 = d1 - i1;
+    const uint32_t cnt = (uint32_t)(i1 - a);
+    for (uint32_t k = tid; k < cnt; k += NT) {
+      const uint64_t i = a + k;
+      const int64_t rel = (int64_t)pos[i] - (int64_t)o0;  // one head's degree stays below 2^31
+      if (rel < INT32_MIN || rel > INT32_MAX) atomicOr(status, ST_BOUNDS);
+      s_pos[k] = (int32_t)rel;
+      s_seg[k] = hseg[i];
+      s_h[k] = hidx[i];
+      s_g[k] = hg[i];
+    }
+    __syncthreads();
+    // Serial merge of item events and outputs: thread t walks merged positions
+    // [d0 + t*ITEMS, ...) once and records the owner of every output it meets.
+    // Item a+k sits at merged position (a+k) + pos[a+k]; output o owned by
+    // item i sits at o + i + 1.
+    {
+      const uint64_t p0 = d0 + (uint64_t)tid * DE_ITEMS;
+      if (p0 < d1) {
+        uint32_t lo = 0, hi = cnt;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if ((int64_t)(a + mid + o0) + s_pos[mid] < (int64_t)p0) lo = mid + 1; else hi = mid;
+        }
+        uint32_t kk = lo;  // local items whose event precedes p0
+        const uint64_t p1 = p0 + DE_ITEMS < d1 ? p0 + DE_ITEMS : d1;
+        for (uint64_t p = p0; p < p1; p++) {
+          if (kk < cnt && (int64_t)(a + kk + o0) + s_pos[kk] == (int64_t)p) {
+            kk++;
+          } else {
+            const uint64_t o = p - (a + kk);
+            if (kk == 0 || o < o0 || o - o0 >= DE_TILE) flags |= ST_BOUNDS;
+            else s_owner[o - o0] = (uint16_t)(kk - 1);
           }
         }
       }
     }
-    if constexpr (WORDS) {
-      // Dense words: lane l takes member bit l, and the warp walks the
-      // outputs (edges) of the dense lanes several at a time; each output's
-      // member weights and probes are one coalesced line.
-      const uint32_t md = mm;
-      unsigned dm = __ballot_sync(kFull, __popc(md) >= dense_members);
-      if ((dm >> lane) & 1u) mm = 0;  // the flattened pass below takes the rest
-      while (dm) {
-        // outputs in flight: four with 32-bit indices and weights, two
-        // otherwise (more would spill under the 51-register bound of five
-        // blocks per SM)
-        constexpr int U = (sizeof(IX) == 4 && sizeof(W) == 4) ? 4 : 2;
-        int t[U];
-        bool live[U];
-        t[0] = __ffs(dm) - 1;
-        live[0] = true;
-        dm &= dm - 1;
-#pragma unroll
-        for (int u = 1; u < U; u++) {
-          live[u] = dm != 0;
-          t[u] = live[u] ? __ffs(dm) - 1 : t[0];
-          dm &= dm - 1;
-        }
-        bool act[U];
-        IX ixd[U];
-        W cwd[U], curd[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          const uint32_t m_t = __shfl_sync(kFull, md, t[u]);
-          const IX kb_t = __shfl_sync(kFull, (IX)kb, t[u]);
-          const W ew_t = TROP ? __shfl_sync(kFull, ew, t[u]) : W(0);
-          const uint32_t w_t = TROP ? __shfl_sync(kFull, (uint32_t)h, t[u]) : 0u;
-          act[u] = ((m_t >> lane) & 1u) && live[u];
-          ixd[u] = kb_t + (IX)lane * ckx;
-          cwd[u] = 0;
-          if constexpr (TROP)
-            if (act[u]) cwd[u] = dw[(IX)w_t * 32 + (IX)lane];
-          if (act[u]) {
-            if constexpr (TROP) curd[u] = D[ixd[u]];
-            else curd[u] = (W)bits[ixd[u] >> 5];
-          }
-          if constexpr (TROP) cwd[u] = trop_mul(cwd[u], ew_t, wshift, &flags);
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-          if (!act[u]) continue;
-          const uint32_t bit = 1u << (ixd[u] & 31);
-          if constexpr (TROP) {
-            if (cwd[u] < curd[u]) {
-              atomic_min_w(&D[ixd[u]], cwd[u]);
-              atomicOr(&marks[ixd[u] >> 5], bit);
+    __syncthreads();
+    const uint64_t o_end = o1 < total ? o1 : total;
+    for (uint64_t c = o0 + (uint64_t)warp * 32; c < o_end; c += NT) {
+      const uint64_t o = c + lane;
+      uint32_t mm = 0, v = 0;
+      W ew = 0;
+      uint64_t h = 0, kb = 0;
+      if (o < o_end) {
+        const uint32_t li = s_owner[o - o0];
+        const uint64_t e = (uint64_t)((int64_t)s_seg[li] + ((int64_t)(o - o0) - s_pos[li]));
+        if (li >= cnt || e >= n_nbr) {
+          flags |= ST_BOUNDS;
+        } else {
+          v = nbr[e];
+          if constexpr (TROP) ew = nbr_w[e];
+          h = s_h[li];
+          if constexpr (WORDS) {
+            // members: the set bits of word h, columns (h mod wpr)*32 + bit of
+            // the head's row; kb = the output index of column 0 of the word
+            mm = s_g[li];
+            const uint32_t wcol = wpr_shift >= 0 ? ((uint32_t)h & (wpr - 1u)) : (uint32_t)h % wpr;
+            kb = (uint64_t)(wcol * 32u) * ck + (uint64_t)v * cv;
+            // every member's entry (and Dprev slot) inside the index: checked
+            // once here for the highest member
+            if (h * 32 + 32 > entries || (mm && kb + (uint64_t)(31 - __clz(mm)) * ck >= entries)) {
+              flags |= ST_BOUNDS;
+              mm = 0;
             }
           } else {
-            if (((uint32_t)curd[u] & bit) == 0) {
-              atomicOr(&bits[ixd[u] >> 5], bit);
-              atomicOr(&marks[ixd[u] >> 5], bit);
-            }
-          }
-        }
-      }
-    }
-    const uint32_t g = __popc(mm);
-    const uint32_t incl = warp_incl_sum(g);
-    const uint32_t T = __shfl_sync(kFull, incl, 31);
-    {
-      uint32_t k = incl - g;
-      for (uint32_t r = mm; r; r &= r - 1) my_slots[k++] = (uint16_t)((lane << 5) | (__ffs(r) - 1));
-    }
-    __syncwarp();
-    // Candidates j = 0..T-1 of this chunk: slot j names the owner lane t and
-    // the member (row offset or bit) of t's head; the edge is v_t.  Four
-    // candidates per lane in flight: their index probes overlap (measured
-    // 3 % faster on MSSP R-MAT-20 than two, together with five resident
-    // blocks of up to 51 registers instead of six of 40).
-    for (uint32_t b0 = 0; b0 < T; b0 += 128) {
-      IX ix[4];
-      W cw[4], cur[4];
-      bool ok[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const uint32_t j = b0 + 32 * u + lane;
-        ok[u] = j < T;
-        const uint32_t sl = ok[u] ? my_slots[j] : 0u;
-        const int t = (int)(sl >> 5);
-        const uint32_t r = sl & 31u;
-        const W ew_t = TROP ? __shfl_sync(kFull, ew, t) : W(0);
-        ix[u] = 0;
-        cw[u] = 0;
-        if constexpr (WORDS) {
-          const IX kb_t = __shfl_sync(kFull, (IX)kb, t);
-          const uint32_t w_t = TROP ? __shfl_sync(kFull, (uint32_t)h, t) : 0u;
-          if (ok[u]) {
-            ix[u] = kb_t + (IX)r * ckx;  // inside the index: checked per output
-            if constexpr (TROP) cw[u] = trop_mul(dw[(IX)w_t * 32 + (IX)r], ew_t, wshift, &flags);
-          }
-        } else {
-          const uint64_t h_t = __shfl_sync(kFull, h, t);
-          const uint32_t v_t = __shfl_sync(kFull, v, t);
-          if (ok[u]) {
-            const uint64_t m = h_t + r;
-            const K mk = dkeys[m];
-            const uint32_t kept = (uint32_t)((mk >> pshift) & (K)pmask);
-            // index of the output key (kept, v) without packing it: one of
-            // the two coefficients is 1, the other the index's row width
-            const uint64_t ix64 = (uint64_t)kept * ck + (uint64_t)v_t * cv;
-            ix[u] = (IX)ix64;
-            if (ix64 >= entries) {
+            const uint32_t g = s_g[li];
+            mm = g >= 32 ? kFull : (1u << g) - 1u;  // members h + r for the set bits r
+            if (g > kGroupMax || h + g > n_rows) {
               flags |= ST_BOUNDS;
-              ok[u] = false;
-            } else if constexpr (TROP) {
-              cw[u] = trop_mul(dw[m], ew_t, wshift, &flags);
+              mm = 0;
             }
           }
         }
       }
+      if constexpr (WORDS) {
+        // Dense words: lane l takes member bit l, and the warp walks the
+        // outputs (edges) of the dense lanes several at a time; each output's
+        // member weights and probes are one coalesced line.
+        const uint32_t md = mm;
+        unsigned dm = __ballot_sync(kFull, __popc(md) >= dense_members);
+        if ((dm >> lane) & 1u) mm = 0;  // the flattened pass below takes the rest
+        while (dm) {
+          // outputs in flight: four with 32-bit indices and weights, two
+          // otherwise (more would spill under the 51-register bound of five
+          // blocks per SM)
+          constexpr int U = (sizeof(IX) == 4 && sizeof(W) == 4) ? 4 : 2;
+          int t[U];
+          bool live[U];
+          t[0] = __ffs(dm) - 1;
+          live[0] = true;
+          dm &= dm - 1;
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        if (ok[u]) {
-          if constexpr (TROP) cur[u] = D[ix[u]];
-          else cur[u] = (W)bits[ix[u] >> 5];
+          for (int u = 1; u < U; u++) {
+            live[u] = dm != 0;
+            t[u] = live[u] ? __ffs(dm) - 1 : t[0];
+            dm &= dm - 1;
+          }
+          bool act[U];
+          IX ixd[U];
+          W cwd[U], curd[U];
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            const uint32_t m_t = __shfl_sync(kFull, md, t[u]);
+            const IX kb_t = __shfl_sync(kFull, (IX)kb, t[u]);
+            const W ew_t = TROP ? __shfl_sync(kFull, ew, t[u]) : W(0);
+            const uint32_t w_t = TROP ? __shfl_sync(kFull, (uint32_t)h, t[u]) : 0u;
+            act[u] = ((m_t >> lane) & 1u) && live[u];
+            ixd[u] = kb_t + (IX)lane * ckx;
+            cwd[u] = 0;
+            if constexpr (TROP)
+              if (act[u]) cwd[u] = dw[(IX)w_t * 32 + (IX)lane];
+            if (act[u]) {
+              if constexpr (TROP) curd[u] = D[ixd[u]];
+              else curd[u] = (W)bits[ixd[u] >> 5];
+            }
+            if constexpr (TROP) cwd[u] = trop_mul(cwd[u], ew_t, wshift, &flags);
+          }
+#pragma unroll
+          for (int u = 0; u < U; u++) {
+            if (!act[u]) continue;
+            const uint32_t bit = 1u << (ixd[u] & 31);
+            if constexpr (TROP) {
+              if (cwd[u] < curd[u]) {
+                atomic_min_w(&D[ixd[u]], cwd[u]);
+                atomicOr(&marks[ixd[u] >> 5], bit);
+              }
+            } else {
+              if (((uint32_t)curd[u] & bit) == 0) {
+                atomicOr(&bits[ixd[u] >> 5], bit);
+                atomicOr(&marks[ixd[u] >> 5], bit);
+              }
+            }
+          }
         }
       }
+      const uint32_t g = __popc(mm);
+      const uint32_t incl = warp_incl_sum(g);
+      const uint32_t T = __shfl_sync(kFull, incl, 31);
+      {
+        uint32_t k = incl - g;
+        for (uint32_t r = mm; r; r &= r - 1) my_slots[k++] = (uint16_t)((lane << 5) | (__ffs(r) - 1));
+      }
+      __syncwarp();
+      // Candidates j = 0..T-1 of this chunk: slot j names the owner lane t and
+      // the member (row offset or bit) of t's head; the edge is v_t.  Four
+      // candidates per lane in flight: their index probes overlap (measured
+      // 3 % faster on MSSP R-MAT-20 than two, together with five resident
+      // blocks of up to 51 registers instead of six of 40).
+      for (uint32_t b0 = 0; b0 < T; b0 += 128) {
+        IX ix[4];
+        W cw[4], cur[4];
+        bool ok[4];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        if (!ok[u]) continue;
-        const uint32_t bit = 1u << (ix[u] & 31);
-        if constexpr (TROP) {
-          if (cw[u] < cur[u]) {
-            atomic_min_w(&D[ix[u]], cw[u]);
-            atomicOr(&marks[ix[u] >> 5], bit);  // changed this round
+        for (int u = 0; u < 4; u++) {
+          const uint32_t j = b0 + 32 * u + lane;
+          ok[u] = j < T;
+          const uint32_t sl = ok[u] ? my_slots[j] : 0u;
+          const int t = (int)(sl >> 5);
+          const uint32_t r = sl & 31u;
+          const W ew_t = TROP ? __shfl_sync(kFull, ew, t) : W(0);
+          ix[u] = 0;
+          cw[u] = 0;
+          if constexpr (WORDS) {
+            const IX kb_t = __shfl_sync(kFull, (IX)kb, t);
+            const uint32_t w_t = TROP ? __shfl_sync(kFull, (uint32_t)h, t) : 0u;
+            if (ok[u]) {
+              ix[u] = kb_t + (IX)r * ckx;  // inside the index: checked per output
+              if constexpr (TROP) cw[u] = trop_mul(dw[(IX)w_t * 32 + (IX)r], ew_t, wshift, &flags);
+            }
+          } else {
+            const uint64_t h_t = __shfl_sync(kFull, h, t);
+            const uint32_t v_t = __shfl_sync(kFull, v, t);
+            if (ok[u]) {
+              const uint64_t m = h_t + r;
+              const K mk = dkeys[m];
+              const uint32_t kept = (uint32_t)((mk >> pshift) & (K)pmask);
+              // index of the output key (kept, v) without packing it: one of
+              // the two coefficients is 1, the other the index's row width
+              const uint64_t ix64 = (uint64_t)kept * ck + (uint64_t)v_t * cv;
+              ix[u] = (IX)ix64;
+              if (ix64 >= entries) {
+                flags |= ST_BOUNDS;
+                ok[u] = false;
+              } else if constexpr (TROP) {
+                cw[u] = trop_mul(dw[m], ew_t, wshift, &flags);
+              }
+            }
           }
-        } else {
-          if (((uint32_t)cur[u] & bit) == 0) {
-            atomicOr(&bits[ix[u] >> 5], bit);
-            atomicOr(&marks[ix[u] >> 5], bit);  // new this round
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          if (ok[u]) {
+            if constexpr (TROP) cur[u] = D[ix[u]];
+            else cur[u] = (W)bits[ix[u] >> 5];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+          if (!ok[u]) continue;
+          const uint32_t bit = 1u << (ix[u] & 31);
+          if constexpr (TROP) {
+            if (cw[u] < cur[u]) {
+              atomic_min_w(&D[ix[u]], cw[u]);
+              atomicOr(&marks[ix[u] >> 5], bit);  // changed this round
+            }
+          } else {
+            if (((uint32_t)cur[u] & bit) == 0) {
+              atomicOr(&bits[ix[u] >> 5], bit);
+              atomicOr(&marks[ix[u] >> 5], bit);  // new this round
+            }
           }
         }
       }
+      __syncwarp();  // the slot table is rewritten for the next chunk
     }
-    __syncwarp();  // the slot table is rewritten for the next chunk
   }
   if (flags) atomicOr(status, flags);
 }
@@ -937,6 +987,85 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
+// The same heads for rounds enqueued without looking at their sizes: one
+// kernel reads the marks once and appends each block's heads at a place
+// reserved by one packed atomic add (the order of the heads is free: every
+// candidate merges by an atomic minimum or OR).  Count, scan and write as
+// three launches are the better form for large indexes, where the reads
+// dominate and the expand wants its heads in index order.
+template <bool TROP, class W>
+__global__ void __launch_bounds__(NT)
+    k_words_append(uint32_t* marks, uint64_t words, uint32_t wpr, const uint32_t* __restrict__ off, uint64_t n_nodes,
+                   uint32_t* __restrict__ hword, uint32_t* __restrict__ hmask, uint64_t* __restrict__ hpos,
+                   uint32_t* __restrict__ hseg, const W* __restrict__ D, W* __restrict__ Dprev, RoundTotals* rt) {
+  __shared__ unsigned long long s_w[NT / 32][3], s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint64_t wb = (uint64_t)blockIdx.x * NT + (uint64_t)warp * 32, i = wb + lane;
+  const uint32_t m = i < words ? marks[i] : 0u;
+  uint32_t d = 0, seg = 0;
+  if (m) {
+    const uint32_t row = (uint32_t)i / wpr;
+    if (row < n_nodes) {
+      seg = off[row];
+      d = off[row + 1] - seg;
+    }
+    marks[i] = 0u;
+  }
+  const unsigned hb = __ballot_sync(kFull, d != 0);
+  const uint64_t incl = warp_incl_sum((uint64_t)d);
+  const uint64_t deg = __shfl_sync(kFull, incl, 31);
+  const uint64_t cands = warp_sum((uint64_t)__popc(m) * d);
+  const uint32_t tuples = warp_sum((uint32_t)__popc(m));
+  if (lane == 0) {
+    s_w[warp][0] = ((unsigned long long)__popc(hb) << kOutBits) + deg;
+    s_w[warp][1] = cands;
+    s_w[warp][2] = tuples;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long t[3] = {0, 0, 0};
+    for (int w = 0; w < NT / 32; w++)
+      for (int q = 0; q < 3; q++) {
+        const unsigned long long x = s_w[w][q];
+        if (q == 0) s_w[w][0] = t[0];  // exclusive over the warps
+        t[q] += x;
+      }
+    if (t[2]) {
+      s_base = t[0] ? atomicAdd(&rt->packed, t[0]) : 0ull;
+      if (t[1]) atomicAdd(&rt->candidates, t[1]);
+      atomicAdd(&rt->tuples, t[2]);
+    }
+  }
+  __syncthreads();
+  if (!hb) return;
+  const unsigned long long at = s_base + s_w[warp][0];
+  if (d) {
+    const uint64_t k = rt_heads(at) + __popc(hb & lanemask_lt());
+    hword[k] = (uint32_t)i;
+    hmask[k] = m;
+    hpos[k] = rt_outputs(at) + incl - d;
+    hseg[k] = seg;
+  }
+  if constexpr (TROP) {
+    // the head words' weights, one line per word, eight in flight
+    for (unsigned left = hb; left;) {
+      int t[8];
+      W val[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        t[q] = left ? __ffs(left) - 1 : -1;
+        left &= left - 1;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (t[q] >= 0) val[q] = D[(wb + t[q]) * 32 + lane];
+#pragma unroll
+      for (int q = 0; q < 8; q++)
+        if (t[q] >= 0) Dprev[(wb + t[q]) * 32 + lane] = val[q];
+    }
+  }
+}
+
 inline unsigned grid1(uint64_t n) { return (unsigned)ceil_div(n ? n : 1, NT); }
 
 size_t dense_expand_smem(bool words) {
@@ -1019,7 +1148,7 @@ void dense_expand(strata_ctx* ctx, const K* dkeys, const W* dw, uint64_t n_rows,
     SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<(unsigned)tiles, NT, smem, ctx->stream>>>(dkeys, dw, n_rows, hidx, hpos, hseg, hg, nh, total, splits_buf,
                                                      pshift, pmask, ck, cv, 1u, 0, 33, nbr, n_nbr, nbr_w, lay.entries,
-                                                     bits, D, marks, ctx->wshift, ctx->d_status);
+                                                     bits, D, marks, ctx->wshift, ctx->d_status, nullptr);
   };
   if (lay.entries <= 0xffffffffull) launch(k_expand_dense<K, TROP, false, uint32_t, W>);
   else launch(k_expand_dense<K, TROP, false, uint64_t, W>);
@@ -1083,7 +1212,7 @@ void dense_expand_words(strata_ctx* ctx, const uint32_t* hword, const uint32_t* 
     SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kern<<<(unsigned)tiles, NT, smem, ctx->stream>>>(nullptr, Dprev, lay.entries, hword, hpos, hseg, hmask, nh, total,
                                                      splits_buf, 0, 0, ck, cv, wpr, wpr_shift, members, nbr, n_nbr,
-                                                     nbr_w, lay.entries, bits, D, marks, ctx->wshift, ctx->d_status);
+                                                     nbr_w, lay.entries, bits, D, marks, ctx->wshift, ctx->d_status, nullptr);
   };
   if (lay.entries <= 0xffffffffull) launch(k_expand_dense<uint32_t, TROP, true, uint32_t, W>);
   else launch(k_expand_dense<uint32_t, TROP, true, uint64_t, W>);
@@ -1094,6 +1223,56 @@ void dense_expand_words(strata_ctx* ctx, const uint32_t* hword, const uint32_t* 
   const uint64_t wsz = TROP ? sizeof(W) : 0;
   kprof_end(ctx, kh, nh * (4 + 4 + 8 + 4) + total * (4 + wsz) + n_delta * wsz + candidates * (TROP ? sizeof(W) : 4));
   after_launch(ctx, "k_expand_dense");
+}
+
+// Whether the rounds over this index and graph can be enqueued in groups: the
+// packed totals hold every size (heads <= words < 2^28, outputs <= words per
+// row × edges < 2^36) and the head buffers for every word are small.  A round
+// enqueued is two launches and no host wait instead of seven operations and
+// one, but its expand strides over unordered heads.  On one B200, whole
+// fixpoints, queued / one by one: 6 k words (MSSP, 2,048 nodes) 742 / 1,128 us,
+// 85 k 1,080 / 1,572, 283 k (paths of 3,000 nodes) 1,518 / 2,208, 536 k 2,402 /
+// 2,667, 1.1 M (MSSP R-MAT-20, 64 sources) 6,759 / 6,520: so up to 2^20 words.
+constexpr uint64_t kQueuedWords = 1ull << 20;
+bool dense_rounds_queued(const DenseLayout& lay, uint64_t n_nbr) {
+  const uint64_t wpr = lay.width / 32;
+  return lay.entries / 32 <= kQueuedWords && n_nbr < (1ull << 36) / (wpr + 1);
+}
+
+// Enqueue rounds [0, count): heads of Δ, then (up to round `expands`) their
+// expand.  totals: count × {heads and outputs packed, candidates, Δ tuples, 0}.
+template <bool TROP, class W>
+void dense_queue_rounds(strata_ctx* ctx, uint32_t* marks, const DenseLayout& lay, const uint32_t* off,
+                        uint64_t n_nodes, uint32_t* hword, uint32_t* hmask, uint64_t* hpos, uint32_t* hseg,
+                        W* D, W* Dprev, int out_pshift, int out_vshift, const uint32_t* nbr, uint64_t n_nbr,
+                        const W* nbr_w, uint32_t* bits, uint64_t* totals, int count, int expands) {
+  const uint64_t words = lay.entries / 32;
+  const uint32_t wpr = (uint32_t)(lay.width / 32);
+  const int wpr_shift = (wpr & (wpr - 1)) == 0 ? __builtin_ctz(wpr) : -1;
+  uint64_t ck, cv;
+  out_coefficients(lay, out_pshift, out_vshift, &ck, &cv);
+  const int members = ctx->tune_dense_members ? ctx->tune_dense_members : kDenseMembers;
+  const size_t smem = dense_expand_smem(true);
+  const bool small_ix = lay.entries <= 0xffffffffull;
+  auto* kern = small_ix ? k_expand_dense<uint32_t, TROP, true, uint32_t, W, true>
+                        : k_expand_dense<uint32_t, TROP, true, uint64_t, W, true>;
+  SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const uint64_t most = words + std::min<uint64_t>(words * n_nbr, (uint64_t)wpr * n_nbr);  // merged positions at most
+  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(most, DE_TILE), (uint64_t)ctx->num_sms * 5));
+  SK_CUDA(cudaMemsetAsync(totals, 0, (uint64_t)count * sizeof(RoundTotals), ctx->stream));
+  auto* rt = reinterpret_cast<RoundTotals*>(totals);
+  for (int r = 0; r < count; r++) {
+    k_words_append<TROP, W><<<grid1(words), NT, 0, ctx->stream>>>(marks, words, wpr, off, n_nodes, hword, hmask, hpos,
+                                                                  hseg, D, Dprev, rt + r);
+    after_launch(ctx, "k_words_append");
+    if (r >= expands) continue;
+    const int kh = kprof_begin(ctx, K_EXPAND_DENSE);
+    kern<<<grid, NT, smem, ctx->stream>>>(nullptr, Dprev, lay.entries, hword, hpos, hseg, hmask, 0, 0, nullptr, 0, 0,
+                                          ck, cv, wpr, wpr_shift, members, nbr, n_nbr, nbr_w, lay.entries, bits, D,
+                                          marks, ctx->wshift, ctx->d_status, rt + r);
+    kprof_end(ctx, kh, 0);  // its bytes are added once the totals are known
+    after_launch(ctx, "k_expand_dense");
+  }
 }
 
 template <class K, bool TROP, class W>
@@ -1190,6 +1369,9 @@ SK_INST_DENSE(uint64_t, true, int32_t)
 SK_INST_DENSE(uint64_t, true, int64_t)
 #undef SK_INST_DENSE
 #define SK_INST_WORDS(T, W)                                                                                     \
+  template void dense_queue_rounds<T, W>(strata_ctx*, uint32_t*, const DenseLayout&, const uint32_t*, uint64_t, \
+                                         uint32_t*, uint32_t*, uint64_t*, uint32_t*, W*, W*, int, int,          \
+                                         const uint32_t*, uint64_t, const W*, uint32_t*, uint64_t*, int, int);  \
   template void dense_word_heads<T, W>(strata_ctx*, uint32_t*, const DenseLayout&, const uint32_t*, uint64_t,   \
                                        uint64_t*, uint32_t*, uint32_t*, uint64_t*, uint32_t*, const W*, W*,     \
                                        uint64_t*);                                                              \

@@ -396,12 +396,20 @@ uint64_t dense_round_keys(strata_ctx* ctx, const K* dk, const W* dw, uint64_t nd
   return cands;
 }
 
+template <bool TROP, class W>
+void fix_loop_queued(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, DenseIdx<W>& X, uint64_t cap,
+                     PhaseTimer& pt, Acct& a, uint64_t* rounds_out);
+
 // Semi-naive rounds with Δ in the marks: word heads (which clear the marks
 // and snapshot Δ's weights), then the expand marks Δ'.  A round runs while
 // Δ is non-empty; `bound` is an upper bound on the entries marked now.
 template <bool TROP, class W>
 void fix_loop_dense(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, DenseIdx<W>& X, uint64_t bound,
                     uint64_t cap, PhaseTimer& pt, Acct& a, uint64_t* rounds_out) {
+  if (dense_rounds_queued(X.lay, csr.m)) {
+    fix_loop_queued<TROP, W>(ctx, csr, js, X, cap, pt, a, rounds_out);
+    return;
+  }
   DBuf<uint64_t> splits;
   splits.ctx = ctx;
   uint64_t rounds = 0;
@@ -439,6 +447,57 @@ void fix_loop_dense(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, Dens
     a.join_l += (uint32_t)(ctx->launches - l0);
     a.cands += cands;
     bound = std::min<uint64_t>(cands, X.entries);
+    if (TROP && cap && rounds > cap)
+      fail(STRATA_E_NEG_CYCLE, "negative-weight cycle: tropical stratum diverges");
+  }
+  *rounds_out = rounds;
+}
+
+// The same rounds in groups: the host enqueues up to kGroup rounds and looks
+// at their totals once.  A round whose Δ is empty costs two empty launches.
+// At the cap the last round's Δ is only counted (its expand would run past
+// the point where the interpreter stops).
+template <bool TROP, class W>
+void fix_loop_queued(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, DenseIdx<W>& X, uint64_t cap,
+                     PhaseTimer& pt, Acct& a, uint64_t* rounds_out) {
+  constexpr int kGroup = 8;
+  const uint64_t hcap = X.words() + 1;
+  X.hidx.reserve(hcap);
+  X.hmask.reserve(hcap);
+  X.hseg.reserve(hcap);
+  X.hpos.reserve(hcap);
+  DBuf<uint64_t> totals(ctx, kGroup * 4 + 1);
+  const uint64_t wsz = TROP ? sizeof(W) : 0;
+  uint64_t rounds = 0;
+  for (bool more = true; more;) {
+    const uint64_t l0 = ctx->launches;
+    const int t = pt.begin(&a.join_ms);
+    // rounds that may still run: the (cap + 1)-th is counted, not expanded
+    const uint64_t left = TROP && cap ? cap + 1 - rounds : kGroup;
+    const int count = (int)std::min<uint64_t>(kGroup, left);
+    const int expands = TROP && cap && left <= (uint64_t)kGroup ? count - 1 : count;
+    const size_t rec0 = ctx->krecs.size();
+    dense_queue_rounds<TROP, W>(ctx, X.marks.p, X.lay, csr.off.p, csr.n_nodes, X.hidx.p, X.hmask.p, X.hpos.p,
+                                X.hseg.p, TROP ? X.D.p : nullptr, TROP ? X.Dprev.p : nullptr, js.out_pshift,
+                                js.out_vshift, csr.nbr.p, csr.m, TROP ? csr.w.p : nullptr, TROP ? nullptr : X.bits.p,
+                                totals.p, count, expands);
+    SK_CUDA(cudaMemcpyAsync(ctx->h_group, totals.p, (size_t)count * 32, cudaMemcpyDeviceToHost, ctx->stream));
+    sync_and_check(ctx);
+    pt.end(t);
+    for (int r = 0; r < count; r++) {
+      const uint64_t *h = ctx->h_group + 4 * r, nh = h[0] >> 36, T = h[0] & ((1ull << 36) - 1), cands = h[1], nd = h[2];
+      a.join_b += X.words() * 4;
+      if (nd == 0) {
+        more = false;
+        break;
+      }
+      rounds++;
+      const uint64_t bytes = nh * 20 + T * (4 + wsz) + nd * wsz + cands * (TROP ? sizeof(W) : 4);
+      if (r < expands && rec0 + r < ctx->krecs.size()) ctx->krecs[rec0 + r].bytes = bytes;
+      a.join_b += X.words() * 4 + nh * 20 + nd * 2 * wsz + bytes;
+      a.cands += cands;
+    }
+    a.join_l += (uint32_t)(ctx->launches - l0);
     if (TROP && cap && rounds > cap)
       fail(STRATA_E_NEG_CYCLE, "negative-weight cycle: tropical stratum diverges");
   }

@@ -92,6 +92,17 @@ void dense_expand_words(strata_ctx* ctx, const uint32_t* hword, const uint32_t* 
                         const W* Dprev, int out_pshift, int out_vshift, const uint32_t* nbr, uint64_t n_nbr,
                         const W* nbr_w, const DenseLayout& lay, uint32_t* bits, W* D, uint32_t* marks,
                         uint64_t* splits_buf);
+// Rounds enqueued without a look at their sizes in between (small indexes).
+// Every round takes the heads of the marks and, for the first `expands` of
+// the `count` rounds, expands them.  `totals` (device, 4 words a round)
+// receives heads << 36 | outputs, candidates and Δ tuples; the head buffers
+// hold one entry per marks word.
+bool dense_rounds_queued(const DenseLayout& lay, uint64_t n_nbr);
+template <bool TROP, class W = int32_t>
+void dense_queue_rounds(strata_ctx* ctx, uint32_t* marks, const DenseLayout& lay, const uint32_t* off,
+                        uint64_t n_nodes, uint32_t* hword, uint32_t* hmask, uint64_t* hpos, uint32_t* hseg,
+                        W* D, W* Dprev, int out_pshift, int out_vshift, const uint32_t* nbr, uint64_t n_nbr,
+                        const W* nbr_w, uint32_t* bits, uint64_t* totals, int count, int expands);
 // out[i] = sum of v[0..i) (exclusive) or v[0..i] (inclusive); *total (if
 // given, synchronizing) = the sum of all n.
 void scan_u64(strata_ctx* ctx, const uint64_t* v, uint64_t n, uint64_t* out, bool inclusive, uint64_t* total);
