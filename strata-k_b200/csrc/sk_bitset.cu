@@ -1120,8 +1120,8 @@ __global__ void __launch_bounds__(BS_NT) k_shard_summary(const uint4* __restrict
   }
 }
 
-uint64_t bs_budget(strata_ctx* ctx) {
-  uint64_t b = (uint64_t)((double)reusable_device_bytes(ctx) * 0.7);
+uint64_t bs_budget(strata_ctx* ctx, uint64_t need) {
+  uint64_t b = device_budget(ctx, 0.7, need);
   if (ctx->cap && ctx->cap > ctx->in_use) b = std::min<uint64_t>(b, ctx->cap - ctx->in_use);
   if (ctx->tune_bs_budget_mb > 0) b = std::min<uint64_t>(b, (uint64_t)ctx->tune_bs_budget_mb << 20);
   return b;
@@ -1150,7 +1150,9 @@ void tc_bool_batch(strata_ctx* ctx, uint32_t n_inst, const uint32_t* nodes, cons
   BsBuffers B(ctx);
   BsResult R;
   try {
-    bs_run(ctx, spec, d_src, d_dst, mode, bs_budget(ctx), B, R, true);
+    uint64_t need = 0;  // of all instances in one wave
+    for (auto& i : spec) need += inst_bytes(i);
+    bs_run(ctx, spec, d_src, d_dst, mode, bs_budget(ctx, need), B, R, true);
   } catch (...) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1188,7 +1190,142 @@ void tc_bool_batch(strata_ctx* ctx, uint32_t n_inst, const uint32_t* nodes, cons
 // do not fit (the caller falls back to another plan).
 bool tc_bool_bitset_fits(strata_ctx* ctx, uint64_t n_src, uint64_t n_dst, uint64_t m) {
   const InstSpec s{(uint32_t)n_src, (uint32_t)n_dst, 0, m};
-  return n_src < (1ull << 32) && n_dst < (1ull << 32) && inst_bytes(s) <= std::min<uint64_t>(bs_budget(ctx), 8ull << 30);
+  const uint64_t need = inst_bytes(s);
+  return n_src < (1ull << 32) && n_dst < (1ull << 32) && need <= (8ull << 30) && need <= bs_budget(ctx, need);
+}
+
+// ---- one small closure in one block --------------------------------------------
+// A graph of a few hundred nodes: the edge CSR, path, Δ and Δ' bit rows fit one
+// block's shared memory, so every round is a pass over them between two block
+// barriers, and the sorted relation is written straight from the final rows.
+// The general form spends 0.6 ms on such a graph in launches and waits; this is
+// bound by the rounds' shared-memory reads (300 nodes, 701 edges, 14 rounds:
+// 49 us on one B200, the call from host columns 639 -> 308 us).
+constexpr int SM_NT = 1024;
+constexpr uint64_t kSmallEdges = 16384, kSmallSmem = 226 * 1024;
+
+inline uint64_t small_smem(uint64_t rows, uint64_t w, uint64_t m) {
+  return 3 * rows * w * 4 + 2 * (rows + 1) * 4 + m * 2 + 16;
+}
+
+__global__ void __launch_bounds__(SM_NT) k_bs_small(const uint32_t* __restrict__ src, const uint32_t* __restrict__ dst,
+                                                    uint32_t m, uint32_t rows, uint32_t cols, int b1,
+                                                    uint32_t* __restrict__ out, uint64_t* res) {
+  extern __shared__ __align__(16) uint32_t s_raw32[];
+  __shared__ uint32_t s_scan[SM_NT / 32 + 1];
+  const uint32_t W = (cols + 31) / 32, N = rows * W;
+  uint32_t* F = s_raw32;
+  uint32_t* D0 = F + N;
+  uint32_t* D1 = D0 + N;
+  uint32_t* off = D1 + N;        // rows + 1
+  uint32_t* deg = off + rows + 1;  // rows + 1
+  uint16_t* nbr = reinterpret_cast<uint16_t*>(deg + rows + 1);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (uint32_t i = tid; i < N; i += SM_NT) F[i] = 0u;
+  for (uint32_t i = tid; i <= rows; i += SM_NT) deg[i] = 0u;
+  __syncthreads();
+  for (uint32_t e = tid; e < m; e += SM_NT) {
+    const uint32_t x = src[e], y = dst[e];
+    if (x >= rows || y >= cols) continue;
+    atomicAdd(&deg[x], 1u);
+    atomicOr(&F[x * W + (y >> 5)], 1u << (y & 31));
+  }
+  __syncthreads();
+  uint32_t carry = 0;
+  for (uint32_t b = 0; b < rows; b += SM_NT) {  // exclusive scan of the degrees
+    const uint32_t d = b + tid < rows ? deg[b + tid] : 0u;
+    uint32_t tot;
+    const uint32_t ex = block_excl_sum<SM_NT>(d, s_scan, &tot);
+    if (b + tid < rows) off[b + tid] = carry + ex;
+    carry += tot;
+  }
+  if (tid == 0) off[rows] = carry;
+  for (uint32_t i = tid; i < N; i += SM_NT) D0[i] = F[i];
+  __syncthreads();
+  for (uint32_t e = tid; e < m; e += SM_NT) {
+    const uint32_t x = src[e], y = dst[e];
+    if (x >= rows || y >= cols) continue;
+    nbr[off[x] + atomicSub(&deg[x], 1u) - 1u] = (uint16_t)y;
+  }
+  __syncthreads();
+  // a round adds a path length, so there are at most rows + 1 of them
+  uint32_t rounds = 0;
+  for (bool more = true; more && rounds <= rows + 1;) {
+    bool any = false;
+    for (uint32_t i = tid; i < N; i += SM_NT) {
+      const uint32_t x = i / W, w = i - x * W, e1 = off[x + 1];
+      uint32_t acc = 0;
+      for (uint32_t e = off[x]; e < e1; e++) {
+        const uint32_t y = nbr[e];
+        if (y < rows) acc |= D0[y * W + w];
+      }
+      const uint32_t f = F[i], nw = acc & ~f;
+      F[i] = f | nw;
+      D1[i] = nw;
+      any |= nw != 0u;
+    }
+    more = __syncthreads_or(any);
+    uint32_t* t = D0;
+    D0 = D1;
+    D1 = t;
+    rounds++;
+  }
+  // rows' sizes, their scan (deg now holds first ordinals), then the keys
+  for (uint32_t x = warp; x < rows; x += SM_NT / 32) {
+    uint32_t c = 0;
+    for (uint32_t w = lane; w < W; w += 32) c += __popc(F[x * W + w]);
+    c = warp_sum(c);
+    if (lane == 0) deg[x] = c;
+  }
+  __syncthreads();
+  carry = 0;
+  for (uint32_t b = 0; b < rows; b += SM_NT) {
+    const uint32_t d = b + tid < rows ? deg[b + tid] : 0u;
+    uint32_t tot;
+    const uint32_t ex = block_excl_sum<SM_NT>(d, s_scan, &tot);
+    if (b + tid < rows) deg[b + tid] = carry + ex;
+    carry += tot;
+  }
+  __syncthreads();
+  for (uint32_t x = warp; x < rows; x += SM_NT / 32) {
+    uint32_t at = deg[x];
+    for (uint32_t w = 0; w < W; w++) {
+      const uint32_t v = F[x * W + w];
+      if ((v >> lane) & 1u) out[at + __popc(v & lanemask_lt())] = (x << b1) | (w * 32 + lane);
+      at += __popc(v);
+    }
+  }
+  if (tid == 0) {
+    res[0] = carry;
+    res[1] = rounds;
+  }
+}
+
+bool tc_bool_small_fits(strata_ctx* ctx, uint64_t n_src, uint64_t n_dst, uint64_t m) {
+  const uint64_t w = ceil_div(n_dst, 32);
+  if (n_src > 1024 || n_dst > 1024 || m > kSmallEdges || small_smem(n_src, w, m) > kSmallSmem) return false;
+  return !ctx->cap || ctx->in_use + 2 * size_class(n_src * n_dst * 4 + 64) <= ctx->cap;
+}
+
+uint64_t tc_bool_small(strata_ctx* ctx, const uint32_t* d_src, const uint32_t* d_dst, uint64_t m, uint64_t n_src,
+                       uint64_t n_dst, int b1, DBuf<uint32_t>& out, uint64_t* rounds) {
+  out.reserve(n_src * n_dst + 1);
+  DBuf<uint64_t> res(ctx, 2);
+  const size_t smem = small_smem(n_src, ceil_div(n_dst, 32), m);
+  SK_CUDA(cudaFuncSetAttribute(k_bs_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_bs_small<<<1, SM_NT, smem, ctx->stream>>>(d_src, d_dst, (uint32_t)m, (uint32_t)n_src, (uint32_t)n_dst, b1, out.p,
+                                              res.p);
+  after_launch(ctx, "k_bs_small");
+  SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, res.p, 16, cudaMemcpyDeviceToHost, ctx->stream));
+  sync_and_check(ctx);
+  *rounds = ctx->h_scalar[1];
+  const uint64_t n = ctx->h_scalar[0];
+  if (n_src * n_dst > 2 * n + 4096) {  // the relation keeps a buffer of its own size
+    DBuf<uint32_t> fit(ctx, n + 1);
+    if (n) SK_CUDA(cudaMemcpyAsync(fit.p, out.p, n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    out = std::move(fit);
+  }
+  return n;
 }
 
 template <class K>

@@ -122,11 +122,8 @@ inline void release_cached(strata_ctx* ctx, uint64_t need) {
   }
 }
 
-// Device bytes this context could obtain now: the device's free memory,
-// plus what its pool holds unused, plus the blocks it keeps cached.
-inline uint64_t reusable_device_bytes(strata_ctx* ctx) {
-  size_t fr = 0, tot = 0;
-  check_cuda(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo");
+// What this context holds unused: its pool's free memory and its cached blocks.
+inline uint64_t held_device_bytes(strata_ctx* ctx) {
   uint64_t extra = ctx->cached;
   if (ctx->pool) {
     unsigned long long reserved = 0, used = 0;  // the attribute value type (cuuint64_t)
@@ -134,7 +131,23 @@ inline uint64_t reusable_device_bytes(strata_ctx* ctx) {
         cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
       extra += reserved - used;
   }
-  return (uint64_t)fr + extra;
+  return extra;
+}
+
+// Device bytes this context could obtain now: the device's free memory,
+// plus what it holds unused.
+inline uint64_t reusable_device_bytes(strata_ctx* ctx) {
+  size_t fr = 0, tot = 0;
+  check_cuda(cudaMemGetInfo(&fr, &tot), "cudaMemGetInfo");
+  return (uint64_t)fr + held_device_bytes(ctx);
+}
+
+// `share` of reusable_device_bytes, or (any call whose need it covers already)
+// the same share of what the context holds: the device query takes 0.1 ms to
+// several ms, and its answer only adds to that.
+inline uint64_t device_budget(strata_ctx* ctx, double share, uint64_t need) {
+  const uint64_t held = (uint64_t)((double)held_device_bytes(ctx) * share);
+  return need <= held ? held : (uint64_t)((double)reusable_device_bytes(ctx) * share);
 }
 
 // Give every cached block back to the pool (before sizing large buffers).

@@ -200,22 +200,31 @@ void fix_loop(strata_ctx* ctx, Rel<K, W>& full, Rel<K, W>& delta, const Csr<W>& 
   *rounds_out = rounds;
 }
 
-// Sort + reduce a packed relation in place into `out` (unique, Trop min).
+// The sorted unique relation (Trop: least weight per key) of columns (c0, c1).
 template <class K, class W, bool TROP>
-void normalize(strata_ctx* ctx, DBuf<K>& keys, DBuf<W>& w, uint64_t n, int key_bits, Rel<K, W>& out) {
+void normalize(strata_ctx* ctx, const uint32_t* c0, const uint32_t* c1, const int64_t* w, const uint8_t* inf,
+               uint64_t n, int shift, int key_bits, Rel<K, W>& out) {
   using V = typename SortVal<W>::type;
-  DBuf<K> ka(ctx, n + 1);
-  DBuf<W> wa;
-  wa.ctx = ctx;
-  if (TROP) wa.reserve(n + 1);
-  K* kp = keys.p;
-  K* kalt = ka.p;
-  V* vp = reinterpret_cast<V*>(w.p);
-  V* valt = reinterpret_cast<V*>(wa.p);
-  radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, TROP, n, key_bits, true);
   out.reserve(n + 1, TROP);
   DBuf<uint64_t> cnt(ctx, 1);
-  reduce_runs<K, W, TROP>(ctx, kp, reinterpret_cast<W*>(vp), n, out.k.p, TROP ? out.w.p : nullptr, cnt.p);
+  if (!small_relation<K, W, TROP>(ctx, c0, c1, w, inf, n, shift, out.k.p, TROP ? out.w.p : nullptr, cnt.p)) {
+    DBuf<K> keys(ctx, n + 1), ka(ctx, n + 1);
+    DBuf<W> kw, wa;
+    kw.ctx = wa.ctx = ctx;
+    if (TROP) {
+      kw.reserve(n + 1);
+      wa.reserve(n + 1);
+    }
+    pack_pairs<K, W, TROP>(ctx, c0, c1, w, inf, n, shift, keys.p, TROP ? kw.p : nullptr);
+    K* kp = keys.p;
+    K* kalt = ka.p;
+    V* vp = reinterpret_cast<V*>(kw.p);
+    V* valt = reinterpret_cast<V*>(wa.p);
+    // skipping constant digits needs a look at the histogram: a wait that a
+    // short sort's passes (5 us each) do not outweigh
+    radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, TROP, n, key_bits, n >= (1u << 18));
+    reduce_runs<K, W, TROP>(ctx, kp, reinterpret_cast<W*>(vp), n, out.k.p, TROP ? out.w.p : nullptr, cnt.p);
+  }
   read_u64(ctx, cnt.p, &out.n, 1);
 }
 
@@ -224,16 +233,11 @@ void normalize(strata_ctx* ctx, DBuf<K>& keys, DBuf<W>& w, uint64_t n, int key_b
 template <class KC, class W, bool TROP>
 void build_edge_csr(strata_ctx* ctx, const EdgeCols& e, int join_col, int jbits, int vbits,
                     uint64_t n_nodes, Csr<W>& csr) {
-  DBuf<KC> keys(ctx, e.n + 1);
-  DBuf<W> w;
-  w.ctx = ctx;
-  if (TROP) w.reserve(e.n + 1);
   const uint32_t* c0 = join_col == 0 ? e.src : e.dst;
   const uint32_t* c1 = join_col == 0 ? e.dst : e.src;
-  pack_pairs<KC, W, TROP>(ctx, c0, c1, e.w, e.inf, e.n, vbits, keys.p, TROP ? w.p : nullptr);
   Rel<KC, W> r;
   r.k.ctx = r.w.ctx = ctx;
-  normalize<KC, W, TROP>(ctx, keys, w, e.n, jbits + vbits, r);
+  normalize<KC, W, TROP>(ctx, c0, c1, e.w, e.inf, e.n, vbits, jbits + vbits, r);
   csr.off.ctx = csr.nbr.ctx = csr.w.ctx = ctx;
   csr.off.reserve(n_nodes + 1);
   csr.nbr.reserve(r.n + 1);
@@ -527,14 +531,7 @@ strata_rel* run_tc_shape(strata_ctx* ctx, const EdgeCols& e, int b0, int b1, int
   // path0 = normalize(edge): every edge is derived by the base rule.
   Rel<K, W> full, delta;
   full.k.ctx = full.w.ctx = delta.k.ctx = delta.w.ctx = ctx;
-  {
-    DBuf<K> keys(ctx, e.n + 1);
-    DBuf<W> w;
-    w.ctx = ctx;
-    if (TROP) w.reserve(e.n + 1);
-    pack_pairs<K, W, TROP>(ctx, e.src, e.dst, e.w, e.inf, e.n, b1, keys.p, TROP ? w.p : nullptr);
-    normalize<K, W, TROP>(ctx, keys, w, e.n, key_bits, full);
-  }
+  normalize<K, W, TROP>(ctx, e.src, e.dst, e.w, e.inf, e.n, b1, key_bits, full);
   // In-CSR: Y -> X (join on the edge's dst), key bits b1 + bsrc.
   Csr<W> csr;
   if (b1 + bsrc <= 32)
@@ -583,8 +580,15 @@ struct Layout {
   bool wide_key;
 };
 
-Layout tc_layout(strata_ctx* ctx, const EdgeCols& e) {
-  const uint32_t ms = max_u32(ctx, e.src, e.n), md = max_u32(ctx, e.dst, e.n);
+// The largest ids of the edge columns alone (a Bool closure needs no more).
+FixScan edge_maxima(strata_ctx* ctx, const EdgeCols& e) {
+  FixScan r{};
+  max_u32_pair(ctx, e.src, e.dst, e.n, &r.max_x, &r.max_y);
+  return r;
+}
+
+Layout tc_layout(const FixScan& fs) {
+  const uint32_t ms = fs.max_x, md = fs.max_y;
   Layout L;
   L.b0 = std::max(1, bits_for(ms));
   L.b1 = std::max(1, bits_for(md));
@@ -635,12 +639,16 @@ bool narrow_ok(uint64_t universe, uint64_t max_edge_w, uint64_t max_seed_w) {
 // final bit rows in (X, Z) order.
 template <class K>
 strata_rel* run_tc_bitset(strata_ctx* ctx, const EdgeCols& e, const Layout& L, strata_fix_stats* st, EventTimer& et,
-                          uint64_t l_start) {
+                          uint64_t l_start, bool small = false) {
   Acct a;
   Rel<K, int32_t> full;
   full.k.ctx = full.w.ctx = ctx;
   uint64_t rounds = 0, round_bytes = 0;
-  full.n = tc_bool_bitset<K>(ctx, e.src, e.dst, e.n, L.n_nodes_src, L.n_nodes, L.b1, full.k, &rounds, &round_bytes);
+  if constexpr (sizeof(K) == 4) {
+    if (small) full.n = tc_bool_small(ctx, e.src, e.dst, e.n, L.n_nodes_src, L.n_nodes, L.b1, full.k, &rounds);
+  }
+  if (!small)
+    full.n = tc_bool_bitset<K>(ctx, e.src, e.dst, e.n, L.n_nodes_src, L.n_nodes, L.b1, full.k, &rounds, &round_bytes);
   a.join_b = round_bytes;
   const double ms = et.stop();
   kprof_collect(ctx);
@@ -664,8 +672,11 @@ strata_rel* fix_tc_bool(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats* st
     strata_rel* rel = new strata_rel();
     return rel;
   }
-  const Layout L = tc_layout(ctx, e);
+  const Layout L = tc_layout(edge_maxima(ctx, e));
   if (ctx->plan == 3 || ctx->plan == 0) {
+    // profiling runs keep the rounds as kernels of their own
+    if (!ctx->profiling && tc_bool_small_fits(ctx, L.n_nodes_src, L.n_nodes, e.n))
+      return run_tc_bitset<uint32_t>(ctx, e, L, st, et, l_start, true);
     const bool fits = tc_bool_bitset_fits(ctx, L.n_nodes_src, L.n_nodes, e.n);
     if (ctx->plan == 3 && !fits) fail(STRATA_E_UNSUPPORTED, "the bit-row plan needs its bit matrices within 8 GB");
     if (fits) {
@@ -693,11 +704,11 @@ strata_rel* fix_trop_paths(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats*
     rel->w_bytes = 8;
     return rel;
   }
-  const Layout L = tc_layout(ctx, e);
-  const uint64_t limit = (uint64_t)std::max(max_u32(ctx, e.src, e.n), (uint32_t)(L.n_nodes - 1)) + 1;
-  const uint64_t universe = count_distinct_ids(ctx, e.src, e.n, e.dst, e.n, nullptr, 0, limit);
+  const FixScan fs = fix_scan(ctx, nullptr, nullptr, nullptr, 0, e.src, e.dst, e.w, e.inf, e.n);
+  const Layout L = tc_layout(fs);
+  const uint64_t universe = fs.universe;
   const uint64_t cap = universe + 2;
-  const bool narrow = !ctx->force_wide && narrow_ok(universe, max_abs_weight(ctx, e.w, e.inf, e.n), 0);
+  const bool narrow = !ctx->force_wide && narrow_ok(universe, fs.mag_w, 0);
   ctx->wshift = narrow ? 0 : wide_shift(ctx, e.w, e.inf, e.n, nullptr, nullptr, 0, cap);
   const bool dense = want_dense(ctx, true, narrow, L.n_nodes_src, L.n_nodes);
   const uint64_t ns = L.n_nodes_src;
@@ -731,12 +742,7 @@ strata_rel* run_mssp(strata_ctx* ctx, const uint32_t* sources, const int64_t* sr
   // src as a unary Trop relation keyed by S (min over duplicate facts).
   Rel<K, W> srcu;
   srcu.k.ctx = srcu.w.ctx = ctx;
-  {
-    DBuf<K> keys(ctx, ns + 1);
-    DBuf<W> w(ctx, ns + 1);
-    pack_pairs<K, W, true>(ctx, nullptr, sources, src_w, src_inf, ns, 0, keys.p, w.p);
-    normalize<K, W, true>(ctx, keys, w, ns, b0, srcu);
-  }
+  normalize<K, W, true>(ctx, nullptr, sources, src_w, src_inf, ns, 0, b0, srcu);
   // Out-CSR: Y -> Z with weights (join on the edge's src), key bits besrc + b1.
   Csr<W> csr;
   if (besrc + b1 <= 32)
@@ -814,16 +820,14 @@ strata_rel* fix_mssp(strata_ctx* ctx, const uint32_t* sources, const int64_t* sr
     }
     return rel;
   }
-  const uint32_t mS = max_u32(ctx, sources, ns);
-  const uint32_t mes = max_u32(ctx, e.src, e.n), med = max_u32(ctx, e.dst, e.n);
+  const FixScan fs = fix_scan(ctx, sources, src_w, src_inf, ns, e.src, e.dst, e.w, e.inf, e.n);
+  const uint32_t mS = fs.max_a, mes = fs.max_x, med = fs.max_y;
   const int b0 = std::max(1, bits_for(mS));
   const int b1 = std::max(1, bits_for(med));
   const int besrc = std::max(1, bits_for(mes));
-  const uint64_t limit = (uint64_t)std::max(mS, std::max(mes, med)) + 1;
-  const uint64_t universe = count_distinct_ids(ctx, sources, ns, e.src, e.n, e.dst, e.n, limit);
+  const uint64_t universe = fs.universe;
   const uint64_t cap = universe + 2;
-  const bool narrow = !ctx->force_wide && narrow_ok(universe, max_abs_weight(ctx, e.w, e.inf, e.n),
-                                                    max_abs_weight(ctx, src_w, src_inf, ns));
+  const bool narrow = !ctx->force_wide && narrow_ok(universe, fs.mag_w, fs.mag_a);
   ctx->wshift = narrow ? 0 : wide_shift(ctx, e.w, e.inf, e.n, src_w, src_inf, ns, cap);
   const uint64_t nn = (uint64_t)mes + 1;
   const uint64_t n0 = (uint64_t)mS + 1, n1 = (uint64_t)med + 1;

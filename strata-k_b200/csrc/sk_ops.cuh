@@ -175,6 +175,7 @@ uint64_t count_distinct_ids(strata_ctx* ctx, const uint32_t* a, uint64_t na, con
                             uint64_t nb, const uint32_t* c, uint64_t nc, uint64_t limit);
 
 // max over columns (synchronizing).
+void max_u32_pair(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, uint32_t* ma, uint32_t* mb);
 uint32_t max_u32(strata_ctx* ctx, const uint32_t* a, uint64_t n, const uint32_t* b = nullptr);  // over a and b
 
 // Pack two u32 columns into keys (c0 << shift) | c1, optional weight conversion
@@ -195,7 +196,19 @@ void unpack_pairs(strata_ctx* ctx, const K* keys, const W* w, uint64_t n, int sh
 bool weight_range(strata_ctx* ctx, const int64_t* w, const uint8_t* inf, uint64_t n, int64_t* mn, int64_t* mx);
 
 // Max |finite weight| over (w, inf) columns (synchronizing); 0 when n == 0.
-uint64_t max_abs_weight(strata_ctx* ctx, const int64_t* w, const uint8_t* inf, uint64_t n);
+// A fixpoint's inputs in one pass: largest ids, largest |finite weight| of the
+// sources' and the edges' columns, and the number of distinct ids.
+struct FixScan {
+  uint32_t max_a, max_x, max_y;
+  uint64_t mag_a, mag_w, universe;
+};
+FixScan fix_scan(strata_ctx* ctx, const uint32_t* a, const int64_t* aw, const uint8_t* ainf, uint64_t na,
+                 const uint32_t* x, const uint32_t* y, const int64_t* w, const uint8_t* winf, uint64_t m);
+// Sorted unique packed rows (Trop: least weight per key) of a relation small
+// enough for one block; false (and nothing done) for a larger one.
+template <class K, class W, bool TROP>
+bool small_relation(strata_ctx* ctx, const uint32_t* c0, const uint32_t* c1, const int64_t* w, const uint8_t* inf,
+                    uint64_t n, int shift, K* out, W* out_w, uint64_t* d_count);
 
 // Order-independent fingerprint of (keys, weight values = codes + ctx->wshift).
 template <class K, class W, bool TROP>

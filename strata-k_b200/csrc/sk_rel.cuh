@@ -82,6 +82,9 @@ uint64_t count_triangle_pattern_range(strata_ctx* ctx, const uint32_t* x, const 
 void tc_bool_batch(strata_ctx* ctx, uint32_t n_inst, const uint32_t* nodes, const uint64_t* edge_off,
                    const uint32_t* d_src, const uint32_t* d_dst, int mode, uint64_t* counts, uint64_t* fps,
                    uint32_t* rounds, strata_batch_stats* st);
+bool tc_bool_small_fits(strata_ctx* ctx, uint64_t n_src, uint64_t n_dst, uint64_t m);
+uint64_t tc_bool_small(strata_ctx* ctx, const uint32_t* d_src, const uint32_t* d_dst, uint64_t m, uint64_t n_src,
+                       uint64_t n_dst, int b1, DBuf<uint32_t>& out, uint64_t* rounds);
 bool tc_bool_bitset_fits(strata_ctx* ctx, uint64_t n_src, uint64_t n_dst, uint64_t m);
 
 void prov_tc_capture(strata_ctx* ctx, uint32_t n, const uint32_t* d_src, const uint32_t* d_dst, uint64_t m,
