@@ -24,11 +24,33 @@
 // round: under the Jacobi schedule its derivation would repeat the previous
 // one exactly, and the buffer being written already holds its set.
 //
+// The same argument skips single batches: while a tuple's set is the one it had
+// throughout the previous round, a batch whose input set did not change either
+// is that round's no-op again.
+//
+// Of the other batches only the candidates that can matter are compared.
+//   * One that contains a proof of the set is rejected, and every candidate
+//     that contains it is rejected with it.
+//   * One that weighs less than all proofs of a full set: with probabilities
+//     in [0, 1] a subset never weighs less than its superset, so it absorbs no
+//     proof and no heavier candidate, and pruning drops it — unless the other
+//     candidates absorb more proofs than they add; then the batch is done
+//     again with it.  (The test keeps a margin of 1e-9 against the rounding of
+//     the products, 4e-15.)
+// What remains (usually a candidate or two of eight) is tested against the set
+// and each other, weighed if accepted, and ranked.
+//
 // Mapping: a half-warp (16 lanes, its own shuffle group) owns one tuple
 // (target, X).  Lanes 0..7 hold the current proof set S, lanes 8..15 the
 // candidates of the batch being applied; each lane keeps its proof's sorted
-// literals in shared memory (double-buffered for the compaction), a 64-bit
-// signature for quick subset rejection, the length and the FP64 weight.
+// literals in one of 16 shared-memory rows (33 words apart, so that lanes at
+// one place of their lists touch different banks; a surviving proof keeps its
+// row), a 64-bit signature for quick subset rejection, the length and the FP64
+// weight.  Bound by instructions at half-warp granularity.  One B200, the
+// rounds of 96 queries over ER 10,000 / 40,000, k = 8: every candidate compared
+// with every proof, lists 32 words apart and copied on every change 65.2 ms;
+// this form 30.3 ms at 8 blocks an SM, 37.6 at 6, 29.8 at 10 with literals
+// loaded in pairs.
 #include "sk_ops.cuh"
 #include "sk_prims.cuh"
 #include "sk_rel.cuh"
@@ -42,6 +64,7 @@ namespace sk {
 namespace {
 
 constexpr int PV_NT = 128;  // 8 half-warps (tuples in flight) per block
+constexpr int PV_BLOCKS = 10;       // resident blocks an SM (48 registers a thread, no spills)
 constexpr uint32_t PV_KMAX = 8;
 constexpr uint32_t PV_LMAX = 32;
 
@@ -99,15 +122,33 @@ struct PvView {
   uint32_t* status;
   uint32_t* last;          // [τ * n + X] last round in which (τ, X) changed (0: never)
   uint32_t round;          // this round, 1-based
+  bool unit_probs;         // every probability lies in [0, 1]
 };
 
-__global__ void __launch_bounds__(PV_NT) k_prov_round(PvView v) {
-  __shared__ uint32_t s_lists[PV_NT / 16][2][16][PV_LMAX];
+// Position of the k-th (0-based) set bit of a 16-bit mask (k < popc).
+__device__ __forceinline__ int nth_bit16(uint32_t m, uint32_t k) {
+  int pos = 0;
+#pragma unroll
+  for (int sh = 8; sh >= 1; sh >>= 1) {
+    const uint32_t c = __popc((m >> pos) & ((1u << sh) - 1u));
+    if (k >= c) {
+      k -= c;
+      pos += sh;
+    }
+  }
+  return pos;
+}
+
+constexpr uint32_t PV_ROW = PV_LMAX + 1;  // words between two lists
+
+__global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_prov_round(PvView v) {
+  __shared__ uint32_t s_lists[PV_NT / 16][16 * PV_ROW];
   const int lane = threadIdx.x & 31;
   const int hw = threadIdx.x >> 4;    // half-warp in the block
   const int hl = lane & 15;           // lane in the half-warp
   const int hbase = lane & 16;
   const unsigned hmask = 0xffffu << hbase;
+  uint32_t* const lists = s_lists[hw];
   const uint64_t pairs = (uint64_t)v.n_tgt * v.n;
   const uint64_t stride = (uint64_t)gridDim.x * (PV_NT / 16);
   uint32_t flags = 0;
@@ -121,36 +162,61 @@ __global__ void __launch_bounds__(PV_NT) k_prov_round(PvView v) {
     // being written still holds that set (it did not change either): skip
     // it.  A stamp read while another half-warp raises it to this round is
     // >= round - 1 and only makes the test conservative.
+    const uint32_t lim = v.round - 1;
+    const uint64_t tbase = (uint64_t)tau * v.n;
+    const uint32_t e0 = v.off[X], e1 = v.off[X + 1];
+    bool steady = false;  // the set is the one of the whole previous round
     if (v.round >= 2) {
-      const uint32_t lim = v.round - 1;
-      bool hot = hl == 0 && v.last[pair] >= lim;
-      for (uint32_t e = v.off[X] + hl; e < v.off[X + 1]; e += 16) {
+      const bool self = v.last[pair] >= lim;
+      steady = !self;
+      bool hot = hl == 0 && self;
+      for (uint32_t e = e0 + hl; e < e1; e += 16) {
         const uint32_t y = v.nbr[e];
-        if (y < v.n && v.last[(uint64_t)tau * v.n + y] >= lim) hot = true;
+        if (y < v.n && v.last[tbase + y] >= lim) hot = true;
       }
       if ((__ballot_sync(hmask, hot) & hmask) == 0u) continue;
     }
     const uint32_t t = v.tgt[tau];
-    int bank = 0;
     uint32_t s_cnt = v.cnt_prev[pair];
-    bool valid = false;
-    uint32_t len = 0;
+    bool valid = hl < (int)s_cnt;
+    uint32_t len = 0, row = (uint32_t)hl;  // this lane's list: lists + row * PV_ROW
     uint64_t sig = 0;
     double w = 0.0;
-    if (hl < (int)s_cnt) {
+    if (valid) {
       const ProofRec& r = v.rec_prev[pair * PV_KMAX + hl];
       len = r.len;
       sig = r.sig;
       w = r.w;
-      for (uint32_t q = 0; q < len; q++) s_lists[hw][0][hl][q] = r.lit[q];
-      valid = true;
+      const uint2* l2 = reinterpret_cast<const uint2*>(r.lit);  // records are 8-byte aligned
+      for (uint32_t q = 0; q < len; q += 2) {
+        const uint2 l = l2[q / 2];
+        lists[row * PV_ROW + q] = l.x;
+        lists[row * PV_ROW + q + 1] = l.y;  // a row has one word more than the longest list
+      }
     }
+    __syncwarp(hmask);
     bool changed = false;
-    const uint32_t e0 = v.off[X], e1 = v.off[X + 1];
+    // candidates below this weight are too light for the full set (0: none is)
+    auto least = [&]() {
+      if (!v.unit_probs || s_cnt < v.k) return 0.0;
+      double m = hl < (int)s_cnt ? w : 2.0;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        const double x = __shfl_xor_sync(hmask, m, o, 16);
+        m = x < m ? x : m;
+      }
+      return m > 1e-290 ? m * (1.0 - 1e-9) : 0.0;
+    };
+    double light = least();
+    bool again = false;  // the batch is done over, light candidates included
+    // a window of 16 edges, one a lane: neighbour, literal, proofs of its set
+    uint32_t wy = 0, wlit = 0, wcnt = 0;
+    bool whot = false;
     for (uint32_t en = 0; en <= e1 - e0; en++) {
       // ---- the batch of this entry (uniform per half-warp)
       uint32_t b_cnt = 0, lit_e = 0, y = 0;
       if (en == 0) {
+        if (steady) continue;  // the edge itself never changes
         uint32_t lo = e0, hi = e1;  // rule 1: is (X, t) an edge?
         while (lo < hi) {
           const uint32_t mid = (lo + hi) >> 1;
@@ -161,140 +227,168 @@ __global__ void __launch_bounds__(PV_NT) k_prov_round(PvView v) {
           lit_e = v.eid[lo] + 1;
         }
       } else {
-        const uint32_t q = e0 + en - 1;
-        y = v.nbr[q];
-        lit_e = v.eid[q] + 1;
-        b_cnt = y < v.n ? v.cnt_prev[(uint64_t)tau * v.n + y] : 0;
+        const uint32_t at = (en - 1) & 15u;
+        if (at == 0) {
+          const uint32_t q = e0 + en - 1 + hl;
+          wcnt = 0;
+          if (q < e1) {
+            wy = v.nbr[q];
+            wlit = v.eid[q] + 1;
+            if (wy < v.n) {
+              wcnt = v.cnt_prev[tbase + wy];
+              whot = v.last[tbase + wy] >= lim;
+            }
+          }
+        }
+        y = __shfl_sync(hmask, wy, (int)at, 16);
+        lit_e = __shfl_sync(hmask, wlit, (int)at, 16);
+        b_cnt = __shfl_sync(hmask, wcnt, (int)at, 16);
+        if (steady && !changed && !__shfl_sync(hmask, whot, (int)at, 16)) continue;
       }
       if (b_cnt == 0) continue;
-      uint32_t* Lc = s_lists[hw][bank][hl];
-      // ---- candidates {e} ∪ P_j into lanes 8..15
+      // ---- candidates {e} ∪ P_j into lanes 8..15, in the rows S does not use
+      uint32_t used = hl < (int)s_cnt ? 1u << row : 0u;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) used |= __shfl_xor_sync(hmask, used, o, 16);
+      bool skipped_light = false;
       if (hl >= 8) {
         valid = false;
+        w = 0.0;
         const uint32_t j = (uint32_t)hl - 8;
+        row = (uint32_t)nth_bit16(~used & 0xffffu, j);
+        uint32_t* Lc = lists + row * PV_ROW;
         if (j < b_cnt) {
           if (en == 0) {
             Lc[0] = lit_e;
             len = 1;
             sig = lit_sig(lit_e);
-            w = 1.0 * v.prob[lit_e - 1];
             valid = true;
           } else {
-            const ProofRec& r = v.rec_prev[((uint64_t)tau * v.n + y) * PV_KMAX + j];
+            const ProofRec& r = v.rec_prev[(tbase + y) * PV_KMAX + j];
             const uint32_t pl = r.len;
-            uint32_t o = 0;
-            bool placed = false;
-            for (uint32_t q = 0; q < pl; q++) {
-              const uint32_t l = r.lit[q];
-              if (!placed && lit_e <= l) {
-                if (lit_e != l) {
-                  if (o < PV_LMAX) Lc[o] = lit_e;
-                  o++;
-                }
-                placed = true;
+            const uint64_t se = lit_sig(lit_e);
+            // without the literal's signature bit the proof cannot hold it; a
+            // proof of full length goes on, to be reported if it is too long
+            skipped_light = !again && pl < PV_LMAX && ((r.sig & se) == 0 ? r.w * v.prob[lit_e - 1] : r.w) < light;
+            if (!skipped_light) {
+              // the literals below e keep their places, those above move up
+              // by one unless e is among them (records are 8-byte aligned:
+              // two literals a load)
+              const uint2* l2 = reinterpret_cast<const uint2*>(r.lit);
+              uint32_t below = 0;
+              bool has = false;
+              auto put = [&](uint32_t l, uint32_t q) {
+                below += l < lit_e ? 1u : 0u;
+                has |= l == lit_e;
+                const uint32_t at = q + (l > lit_e && !has ? 1u : 0u);
+                if (at < PV_LMAX) Lc[at] = l;
+              };
+              for (uint32_t q = 0; q < pl; q += 2) {
+                const uint2 l = l2[q / 2];
+                put(l.x, q);
+                if (q + 1 < pl) put(l.y, q + 1);
               }
-              if (o < PV_LMAX) Lc[o] = l;
-              o++;
-            }
-            if (!placed) {
-              if (o < PV_LMAX) Lc[o] = lit_e;
-              o++;
-            }
-            if (o > PV_LMAX) {
-              flags |= ST_PROOF_LEN;
-            } else {
-              len = o;
-              sig = r.sig | lit_sig(lit_e);
-              double ww = 1.0;
-              for (uint32_t q = 0; q < len; q++) ww = ww * v.prob[Lc[q] - 1];
-              w = ww;
-              valid = true;
+              if (!has && below < PV_LMAX) Lc[below] = lit_e;
+              const uint32_t o = pl + (has ? 0u : 1u);
+              if (o > PV_LMAX) {
+                flags |= ST_PROOF_LEN;
+              } else {
+                len = o;
+                sig = r.sig | se;
+                valid = true;
+              }
             }
           }
         }
       }
+      again = false;
       __syncwarp(hmask);
-      // ---- subset matrix: bit y of subof = proof(y) ⊆ proof(me); eqof = equal
-      // (only the valid lanes are visited: the set bits of the half-warp's
-      // ballot, the same on all its lanes)
+      // ---- rejected: contains a proof of S
+      if (__ballot_sync(hmask, valid && hl >= 8) & hmask) {
+        for (uint32_t q = 0; q < s_cnt; q++) {
+          const uint32_t lq = __shfl_sync(hmask, len, (int)q, 16), rq = __shfl_sync(hmask, row, (int)q, 16);
+          const uint64_t sq = __shfl_sync(hmask, sig, (int)q, 16);
+          if (hl >= 8 && valid && lq <= len && (sq & ~sig) == 0 &&
+              sub_list(lists + rq * PV_ROW, lq, lists + row * PV_ROW, len))
+            valid = false;
+        }
+      }
+      const uint32_t cand = (__ballot_sync(hmask, valid && hl >= 8) >> hbase) & 0xff00u;
+      if (cand == 0) continue;
+      // ---- the remaining candidates against S and each other: bit y of subof
+      // = candidate y ⊆ proof(me); eqof = equal
       uint32_t subof = 0, eqof = 0;
-      const uint32_t vmask = (__ballot_sync(hmask, valid) >> hbase) & 0xffffu;
-      for (uint32_t vm = vmask; vm; vm &= vm - 1) {
+      for (uint32_t vm = cand; vm; vm &= vm - 1) {
         const int yl = __ffs(vm) - 1;
-        const uint32_t ly = __shfl_sync(hmask, len, yl, 16);
+        const uint32_t ly = __shfl_sync(hmask, len, yl, 16), ry = __shfl_sync(hmask, row, yl, 16);
         const uint64_t sy = __shfl_sync(hmask, sig, yl, 16);
         if (valid && yl != hl && ly <= len && (sy & ~sig) == 0 &&
-            sub_list(s_lists[hw][bank][yl], ly, Lc, len)) {
+            sub_list(lists + ry * PV_ROW, ly, lists + row * PV_ROW, len)) {
           subof |= 1u << yl;
           if (ly == len) eqof |= 1u << yl;
         }
       }
       // ---- insert_minimal of the batch: within-batch minimal (equal sets
-      // keep the lowest lane), then rejected by any S proof it contains
-      bool accepted = false;
-      if (valid && hl >= 8) {
-        const uint32_t below = (1u << hl) - 1u;
-        const bool dom = ((subof & ~eqof) & 0xff00u) != 0u || (eqof & 0xff00u & below) != 0u;
-        const bool rej = (subof & 0x00ffu) != 0u;
-        accepted = !dom && !rej;
-      }
+      // keep the lowest lane)
+      const bool accepted = hl >= 8 && valid && (subof & ~eqof) == 0u && (eqof & ((1u << hl) - 1u)) == 0u;
       const uint32_t acc = (__ballot_sync(hmask, accepted) >> hbase) & 0xffffu;
-      const uint32_t s_mask = (1u << s_cnt) - 1u;
       // S proofs absorbed by an accepted candidate (strictly: equal ones were rejected)
-      const bool removed = hl < 8 && valid && (subof & acc) != 0u;
-      const bool surv = (hl < 8 && valid && !removed) || accepted;
+      const bool surv = (hl < 8 && valid && (subof & acc) == 0u) || accepted;
       const uint32_t sv = (__ballot_sync(hmask, surv) >> hbase) & 0xffffu;
-      uint32_t keep = acc ? sv : s_mask;
       const uint32_t ns = __popc(sv);
-      if (acc && ns > v.k) {
+      if (ns < s_cnt && (__ballot_sync(hmask, skipped_light) & hmask)) {
+        // fewer proofs than the full set held: the light candidates count
+        again = true;
+        en--;
+        if (hl >= 8) valid = false;
+        __syncwarp(hmask);
+        continue;
+      }
+      if (accepted) {
+        // the product in ascending literal order
+        double ww = 1.0;
+        const uint32_t* Lc = lists + row * PV_ROW;
+        for (uint32_t q = 0; q < len; q++) ww = ww * v.prob[Lc[q] - 1];
+        w = ww;
+      }
+      uint32_t keep = sv;
+      if (ns > v.k) {
         // prune_top_k: rank by (weight desc, literals asc)
         uint32_t rank = 0;
         for (uint32_t vm = sv; vm; vm &= vm - 1) {
           const int yl = __ffs(vm) - 1;
-          const double wy = __shfl_sync(hmask, w, yl, 16);
-          const uint32_t ly = __shfl_sync(hmask, len, yl, 16);
+          const double wl = __shfl_sync(hmask, w, yl, 16);
+          const uint32_t ly = __shfl_sync(hmask, len, yl, 16), ry = __shfl_sync(hmask, row, yl, 16);
           if (!surv || yl == hl) continue;
-          if (wy > w || (wy == w && lex_less(s_lists[hw][bank][yl], ly, Lc, len))) rank++;
+          if (wl > w || (wl == w && lex_less(lists + ry * PV_ROW, ly, lists + row * PV_ROW, len))) rank++;
         }
         keep = (__ballot_sync(hmask, surv && rank < v.k) >> hbase) & 0xffffu;
       }
-      if (keep == s_mask) {  // S unchanged: drop the candidates
-        if (hl >= 8) {
-          valid = false;
-          len = 0;
-          sig = 0;
-          w = 0.0;
-        }
+      if (keep == (1u << s_cnt) - 1u) {  // S unchanged: drop the candidates
+        if (hl >= 8) valid = false;
         __syncwarp(hmask);
         continue;
       }
       changed = true;
-      // ---- compaction: survivor d moves to lane d, lists to the other bank
+      // ---- survivor d moves to lane d (its list stays where it is)
       const uint32_t cnt = __popc(keep);
-      const int src = hl < (int)cnt ? (int)(__fns(keep, 0, hl + 1)) : hl;
-      const uint32_t nlen = __shfl_sync(hmask, len, src & 15, 16);
-      const uint64_t nsig = __shfl_sync(hmask, sig, src & 15, 16);
-      const double nw = __shfl_sync(hmask, w, src & 15, 16);
-      __syncwarp(hmask);
-      if (hl < (int)cnt) {
-        const uint32_t* from = s_lists[hw][bank][src & 15];
-        uint32_t* to = s_lists[hw][bank ^ 1][hl];
-        for (uint32_t q = 0; q < nlen; q++) to[q] = from[q];
-      }
-      __syncwarp(hmask);
-      bank ^= 1;
+      const int src = hl < (int)cnt ? nth_bit16(keep, (uint32_t)hl) : hl;
+      len = __shfl_sync(hmask, len, src, 16);
+      row = __shfl_sync(hmask, row, src, 16);
+      sig = __shfl_sync(hmask, sig, src, 16);
+      w = __shfl_sync(hmask, w, src, 16);
       s_cnt = cnt;
       valid = hl < (int)cnt;
-      len = valid ? nlen : 0;
-      sig = valid ? nsig : 0;
-      w = valid ? nw : 0.0;
+      light = least();
+      __syncwarp(hmask);
     }
     // ---- write the tuple's new proof set
     if (hl == 0) v.cnt_next[pair] = (uint8_t)s_cnt;
     if (hl < (int)s_cnt) {
       ProofRec* r = &v.rec_next[pair * PV_KMAX + hl];
-      const uint32_t* from = s_lists[hw][bank][hl];
-      for (uint32_t q = 0; q < len; q++) r->lit[q] = from[q];
+      const uint32_t* from = lists + row * PV_ROW;
+      uint2* l2 = reinterpret_cast<uint2*>(r->lit);
+      for (uint32_t q = 0; q < len; q += 2) l2[q / 2] = make_uint2(from[q], from[q + 1]);
       r->len = len;
       r->sig = sig;
       r->w = w;
@@ -327,10 +421,12 @@ __global__ void k_edge_keys(const uint32_t* src, const uint32_t* dst, uint64_t m
   idx[i] = (uint32_t)i;
 }
 
-__global__ void k_dup_check(const uint64_t* keys, uint64_t m, uint32_t* dup) {
+// flags[0]: a duplicate edge; flags[1]: a probability outside [0, 1] (or NaN)
+__global__ void k_edge_check(const uint64_t* keys, const double* prob, uint64_t m, uint32_t* flags) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
-  if (i > 0 && keys[i] == keys[i - 1]) *dup = 1u;
+  if (i > 0 && keys[i] == keys[i - 1]) flags[0] = 1u;
+  if (!(prob[i] >= 0.0 && prob[i] <= 1.0)) flags[1] = 1u;
 }
 
 }  // namespace
@@ -355,8 +451,8 @@ void prov_tc_capture(strata_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     fail(STRATA_E_INVALID, "an edge endpoint is outside [0, n)");
   const int b = std::max(1, bits_for(n ? n - 1 : 0));
   DBuf<uint64_t> keys(ctx, m + 1), kalt(ctx, m + 1);
-  DBuf<uint32_t> idx(ctx, m + 1), ialt(ctx, m + 1), nbr(ctx, m + 1), off(ctx, (uint64_t)n + 1), flag(ctx, 1);
-  SK_CUDA(cudaMemsetAsync(flag.p, 0, 4, ctx->stream));
+  DBuf<uint32_t> idx(ctx, m + 1), ialt(ctx, m + 1), nbr(ctx, m + 1), off(ctx, (uint64_t)n + 1), flag(ctx, 2);
+  SK_CUDA(cudaMemsetAsync(flag.p, 0, 8, ctx->stream));
   if (m) {
     // endpoints are checked against n by the CSR build below
     k_edge_keys<<<(unsigned)ceil_div(m, 256), 256, 0, ctx->stream>>>(d_src, d_dst, m, b, keys.p, idx.p);
@@ -366,15 +462,16 @@ void prov_tc_capture(strata_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     uint32_t* vp = idx.p;
     uint32_t* va = ialt.p;
     radix_sort<uint64_t, uint32_t>(ctx, &kp, &ka, &vp, &va, true, m, 2 * b, false);
-    k_dup_check<<<(unsigned)ceil_div(m, 256), 256, 0, ctx->stream>>>(kp, m, flag.p);
-    after_launch(ctx, "k_dup_check");
+    k_edge_check<<<(unsigned)ceil_div(m, 256), 256, 0, ctx->stream>>>(kp, d_prob, m, flag.p);
+    after_launch(ctx, "k_edge_check");
     build_csr<uint64_t>(ctx, kp, m, b, n, off.p, nbr.p);
     if (vp != idx.p) std::swap(idx, ialt);
   } else {
     SK_CUDA(cudaMemsetAsync(off.p, 0, ((uint64_t)n + 1) * 4, ctx->stream));
   }
-  SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, flag.p, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, flag.p, 8, cudaMemcpyDeviceToHost, ctx->stream));
   sync_and_check(ctx);
+  const bool unit_probs = (uint32_t)(ctx->h_scalar[0] >> 32) == 0;
   if ((uint32_t)ctx->h_scalar[0])
     fail(STRATA_E_UNSUPPORTED, "duplicate probabilistic edge facts (X, Y): each edge tuple must be one leaf");
   // ---- targets and waves
@@ -416,7 +513,7 @@ void prov_tc_capture(strata_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     std::fill(h_live.begin(), h_live.end(), 1u);
     SK_CUDA(cudaMemcpyAsync(d_live.p, h_live.data(), nt * 4, cudaMemcpyHostToDevice, ctx->stream));
     PvView v{n, off.p, nbr.p, idx.p, d_prob, d_tgt.p, nt, k, cntA.p, recA.p, cntB.p, recB.p,
-             d_live.p, d_changed.p, ctx->d_status, d_last.p, 0};
+             d_live.p, d_changed.p, ctx->d_status, d_last.p, 0, unit_probs};
     bool a_is_prev = true;
     uint32_t live_count = nt;
     uint32_t r = 0;
