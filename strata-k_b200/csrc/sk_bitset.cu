@@ -1146,13 +1146,14 @@ void tc_bool_batch(strata_ctx* ctx, uint32_t n_inst, const uint32_t* nodes, cons
   check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
   check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
   check_cuda(cudaEventRecord(e0, ctx->stream), "cudaEventRecord");
-  release_all_cached(ctx);  // the waves are sized from what this context can reuse
+  uint64_t need = 0;  // of all instances in one wave
+  for (auto& i : spec) need += inst_bytes(i);
+  const uint64_t budget = bs_budget(ctx, need);  // the waves are sized from what this context can reuse
+  release_all_cached(ctx);
   BsBuffers B(ctx);
   BsResult R;
   try {
-    uint64_t need = 0;  // of all instances in one wave
-    for (auto& i : spec) need += inst_bytes(i);
-    bs_run(ctx, spec, d_src, d_dst, mode, bs_budget(ctx, need), B, R, true);
+    bs_run(ctx, spec, d_src, d_dst, mode, budget, B, R, true);
   } catch (...) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
