@@ -142,12 +142,13 @@ inline uint64_t reusable_device_bytes(strata_ctx* ctx) {
   return (uint64_t)fr + held_device_bytes(ctx);
 }
 
-// `share` of reusable_device_bytes, or (any call whose need it covers already)
-// the same share of what the context holds: the device query takes 0.1 ms to
-// several ms, and its answer only adds to that.
+// `share` of reusable_device_bytes; or `need` itself when the context holds
+// that much unused already (with a tenth to spare): the device query takes
+// 0.1 ms to several ms, and the need then takes nothing new from the device.
 inline uint64_t device_budget(strata_ctx* ctx, double share, uint64_t need) {
-  const uint64_t held = (uint64_t)((double)held_device_bytes(ctx) * share);
-  return need <= held ? held : (uint64_t)((double)reusable_device_bytes(ctx) * share);
+  const uint64_t held = held_device_bytes(ctx);
+  if (need <= held - held / 10) return need;
+  return (uint64_t)((double)reusable_device_bytes(ctx) * share);
 }
 
 // Give every cached block back to the pool (before sizing large buffers).
