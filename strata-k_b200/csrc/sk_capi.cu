@@ -857,6 +857,12 @@ void strata_rel_free(strata_ctx* ctx, strata_rel* rel) {
 
 // ---- operator surface ---------------------------------------------------------------
 
+// [a, a + an) and [b, b + bn) share a byte (null or empty spans share none).
+static bool spans_overlap(const void* a, uint64_t an, const void* b, uint64_t bn) {
+  const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return a && b && an && bn && x < y + bn && y < x + an;
+}
+
 strata_status strata_op_sort(strata_ctx* ctx, int key_bytes, int val_bytes, const void* d_keys_in,
                              const void* d_vals_in, void* d_keys_out, void* d_vals_out, uint64_t n,
                              int key_bits) {
@@ -871,10 +877,15 @@ strata_status strata_op_sort(strata_ctx* ctx, int key_bytes, int val_bytes, cons
   SK_GUARD_BEGIN
   sk::reset_status(ctx);
   if (n == 0) return STRATA_OK;
-  // Copy the inputs into the output buffers, sort between output and scratch.
-  SK_CUDA(cudaMemcpyAsync(d_keys_out, d_keys_in, n * key_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
-  if (val_bytes)
-    SK_CUDA(cudaMemcpyAsync(d_vals_out, d_vals_in, n * val_bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+  // The first pass reads the inputs and the last writes the outputs; buffers
+  // that overlap are copied first and sorted between output and scratch.
+  const uint64_t kb = n * (uint64_t)key_bytes, vb = n * (uint64_t)val_bytes;
+  const bool apart = !spans_overlap(d_keys_in, kb, d_keys_out, kb) && !spans_overlap(d_keys_in, kb, d_vals_out, vb) &&
+                     !spans_overlap(d_vals_in, vb, d_keys_out, kb) && !spans_overlap(d_vals_in, vb, d_vals_out, vb);
+  if (!apart) {
+    SK_CUDA(cudaMemcpyAsync(d_keys_out, d_keys_in, kb, cudaMemcpyDeviceToDevice, ctx->stream));
+    if (val_bytes) SK_CUDA(cudaMemcpyAsync(d_vals_out, d_vals_in, vb, cudaMemcpyDeviceToDevice, ctx->stream));
+  }
   auto run = [&](auto kt, auto vt) {
     using K = decltype(kt);
     using V = decltype(vt);
@@ -886,7 +897,9 @@ strata_status strata_op_sort(strata_ctx* ctx, int key_bytes, int val_bytes, cons
     K* kalt = ka.p;
     V* vp = static_cast<V*>(d_vals_out);
     V* valt = va.p;
-    sk::radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, val_bytes != 0, n, key_bits, true);
+    sk::radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, val_bytes != 0, n, key_bits, true,
+                         apart ? static_cast<const K*>(d_keys_in) : nullptr,
+                         apart && val_bytes ? static_cast<const V*>(d_vals_in) : nullptr);
     if (kp != d_keys_out) {
       SK_CUDA(cudaMemcpyAsync(d_keys_out, kp, n * sizeof(K), cudaMemcpyDeviceToDevice, ctx->stream));
       if (val_bytes) SK_CUDA(cudaMemcpyAsync(d_vals_out, vp, n * sizeof(V), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -899,12 +912,6 @@ strata_status strata_op_sort(strata_ctx* ctx, int key_bytes, int val_bytes, cons
     if (val_bytes == 8) run(uint64_t(), uint64_t()); else run(uint64_t(), uint32_t());
   }
   SK_GUARD_END(ctx)
-}
-
-// [a, a + an) and [b, b + bn) share a byte (null or empty spans share none).
-static bool spans_overlap(const void* a, uint64_t an, const void* b, uint64_t bn) {
-  const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-  return a && b && an && bn && x < y + bn && y < x + an;
 }
 
 strata_status strata_op_dedup_diff(strata_ctx* ctx, int key_bytes, const void* d_cand, uint64_t n,

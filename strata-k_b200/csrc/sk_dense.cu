@@ -59,22 +59,6 @@ __global__ void k_tile_splits(const uint64_t* __restrict__ pos, uint64_t n, uint
   splits[t] = mp_before(pos, n, d);
 }
 
-// The same count found by one warp, 32 probes at a time.
-__device__ __forceinline__ uint64_t mp_before_warp(const uint64_t* pos, uint64_t n, uint64_t d) {
-  const int lane = threadIdx.x & 31;
-  uint64_t lo = 0, hi = d < n ? d : n;
-  while (lo < hi) {
-    const uint64_t step = (hi - lo) / 33 + 1;
-    const uint64_t mid = lo + (uint64_t)lane * step;
-    const unsigned below = __ballot_sync(kFull, mid < hi && mid + pos[mid] < d);
-    const int c = __popc(below);  // probes before d: a prefix of the lanes
-    const uint64_t first = lo;
-    if (c < 32 && first + (uint64_t)c * step < hi) hi = first + (uint64_t)c * step;
-    if (c) lo = first + (uint64_t)(c - 1) * step + 1;
-  }
-  return lo;
-}
-
 // A round's totals as the head kernel leaves them: heads and (head, edge)
 // outputs in one word (so that one atomic add reserves places in both), the
 // candidates and the Δ tuples.

@@ -220,9 +220,8 @@ void normalize(strata_ctx* ctx, const uint32_t* c0, const uint32_t* c1, const in
     K* kalt = ka.p;
     V* vp = reinterpret_cast<V*>(kw.p);
     V* valt = reinterpret_cast<V*>(wa.p);
-    // skipping constant digits needs a look at the histogram: a wait that a
-    // short sort's passes (5 us each) do not outweigh
-    radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, TROP, n, key_bits, n >= (1u << 18));
+    // packed ids: every digit of the key's bits varies, so no look at the keys
+    radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, TROP, n, key_bits, false);
     reduce_runs<K, W, TROP>(ctx, kp, reinterpret_cast<W*>(vp), n, out.k.p, TROP ? out.w.p : nullptr, cnt.p);
   }
   read_u64(ctx, cnt.p, &out.n, 1);

@@ -16,12 +16,13 @@ constexpr uint64_t kMaxSortKeys = (1ull << 32) - 1;
 // Stable LSD radix sort (onesweep) of `n` keys on their low `bits` bits, with
 // optional values (V = uint32_t or uint64_t; has_vals selects them).  keys/alt
 // (and vals/valt) are a double buffer: on return `*keys` (and `*vals`) point at
-// the sorted data and `*alt` at the scratch half.  When `skip_trivial` is set
-// the global digit histogram is read back (one synchronization) and passes
-// whose digit is constant are skipped.
+// the sorted data and `*alt` at the scratch half.  With `look` the bits in
+// which the keys differ are read back first (one synchronization) and only
+// those are sorted.  With kin (and vin) the data comes from there, untouched,
+// and the result lies in the buffers that *keys and *vals name on entry.
 template <class K, class V>
 void radix_sort(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has_vals,
-                uint64_t n, int bits, bool skip_trivial = true);
+                uint64_t n, int bits, bool look = true, const K* kin = nullptr, const V* vin = nullptr);
 
 // Keys-per-thread choices of the onesweep tile for 4- or 8-byte keys
 // (strata_ctx_set_knob); returns how many, writes up to max_out.
@@ -135,7 +136,7 @@ template <class K, class W, bool TROP>
 void expand_emit(strata_ctx* ctx, const K* dkeys, const W* dw, uint64_t n, const uint64_t* pos,
                  uint64_t total, int jshift, uint64_t jmask, int pshift, uint64_t pmask,
                  int out_pshift, int out_vshift, const uint32_t* off, uint64_t n_nodes,
-                 const uint32_t* nbr, uint64_t n_nbr, const W* nbr_w, K* out, W* out_w);
+                 const uint32_t* nbr, uint64_t n_nbr, const W* nbr_w, K* out, W* out_w, bool op_weights = false);
 
 // Reduce sorted keys with duplicates to one row per key (Trop: the minimum
 // weight).  Writes count to *d_count (device).  `out`/`out_w` capacity >= n.
@@ -166,6 +167,12 @@ void diff_improve(strata_ctx* ctx, const K* cand, const W* cand_w, uint64_t nc, 
 
 // CSR offsets from keys sorted by (join << vbits) | v:
 // off[j] = first index with join >= j, for j in [0, n_nodes]; nbr[i] = key & vmask.
+// The two halves of build_csr; op_w (optional): the rows' operator-surface
+// weights, checked on the way (a finite one without a code sets the status).
+template <class K>
+void csr_offsets(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint64_t n_nodes, uint32_t* off);
+template <class K>
+void csr_neighbours(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint32_t* nbr, const int64_t* op_w);
 template <class K>
 void build_csr(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint64_t n_nodes,
                uint32_t* off, uint32_t* nbr);

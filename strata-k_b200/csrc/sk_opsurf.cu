@@ -44,27 +44,6 @@ constexpr uint32_t AG_TILE = NT * AG_ITEMS;
 
 inline unsigned grid_of(uint64_t n, uint64_t per) { return (unsigned)ceil_div(n ? n : 1, per); }
 
-// The operator surface carries Trop weights as int64 with INT64_MAX = +inf;
-// the kernels use codes with +inf = WInf (sk_prims.cuh).  Finite weights
-// above WFinMax have no code on this surface.
-__global__ void k_op_to_codes(const int64_t* __restrict__ in, uint64_t n, int64_t* __restrict__ out,
-                              uint32_t* status) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int64_t v = in[i];
-  if (v == INT64_MAX) {
-    out[i] = WInf<int64_t>::v;
-  } else {
-    if (v > WFinMax<int64_t>::v) atomicOr(status, ST_SENTINEL);
-    out[i] = v;
-  }
-}
-
-__global__ void k_op_from_codes(int64_t* w, uint64_t n) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && w[i] == WInf<int64_t>::v) w[i] = INT64_MAX;
-}
-
 template <class KI, class KO>
 __global__ void k_project(const KI* __restrict__ in, uint64_t n, int in_shift, int sel_hi, int sel_lo,
                           uint64_t const_hi, uint64_t const_lo, int out_shift, KO* __restrict__ out) {
@@ -320,32 +299,39 @@ uint64_t op_join(strata_ctx* ctx, const K* dk, const int64_t* dw, uint64_t nd, i
   SK_CUDA(cudaStreamSynchronize(ctx->stream));
   const uint64_t n_nodes = (r_shift >= (int)(8 * sizeof(K)) ? 0ull : ((uint64_t)last >> r_shift)) + 1;
   if (n_nodes > (1ull << 32)) fail(STRATA_E_UNSUPPORTED, "join column values must be below 2^32");
-  DBuf<uint32_t> off(ctx, n_nodes + 1), nbr(ctx, nr + 1);
-  build_csr<K>(ctx, rk, nr, r_shift, n_nodes, off.p, nbr.p);
+  DBuf<uint32_t> off(ctx, n_nodes + 1);
+  csr_offsets<K>(ctx, rk, nr, r_shift, n_nodes, off.p);
   DBuf<uint64_t> pos(ctx, nd + 1);
   const uint64_t dmask = d_shift >= 64 ? ~0ull : ((1ull << d_shift) - 1);
   expand_offsets<K>(ctx, dk, nd, 0, dmask, off.p, n_nodes, pos.p);
-  uint64_t T = 0;
-  read_u64(ctx, pos.p + nd, &T, 1);
+  SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, pos.p + nd, 8, cudaMemcpyDeviceToHost, ctx->stream));
   sync_and_check(ctx);  // an unsorted `b` shows up here as a bounds status
+  const uint64_t T = ctx->h_scalar[0];
   if (!out || out_cap < T) return T;
   *written = true;
   if (T == 0) return 0;
   ctx->wshift = 0;
+  DBuf<uint32_t> nbr(ctx, nr + 1);
+  // an output weight column over an input one: the inputs are read from copies
+  DBuf<int64_t> cd, cr;
+  cd.ctx = cr.ctx = ctx;
+  auto apart = [&](const int64_t* w, uint64_t n, DBuf<int64_t>& copy) -> const int64_t* {
+    if (!w || out_w >= w + n || w >= out_w + T) return w;
+    copy.reserve(n);
+    SK_CUDA(cudaMemcpyAsync(copy.p, w, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+    return copy.p;
+  };
   if (trop) {
-    DBuf<int64_t> cd(ctx, nd), cr(ctx, nr);
-    k_op_to_codes<<<grid_of(nd, NT), NT, 0, ctx->stream>>>(dw, nd, cd.p, ctx->d_status);
-    after_launch(ctx, "k_op_to_codes");
-    k_op_to_codes<<<grid_of(nr, NT), NT, 0, ctx->stream>>>(rw, nr, cr.p, ctx->d_status);
-    after_launch(ctx, "k_op_to_codes");
-    expand_emit<K, int64_t, true>(ctx, dk, cd.p, nd, pos.p, T, 0, dmask, d_shift, ~0ull, out_shift, 0, off.p, n_nodes,
-                                  nbr.p, nr, cr.p, out, out_w);
-    k_op_from_codes<<<grid_of(T, NT), NT, 0, ctx->stream>>>(out_w, T);
-    after_launch(ctx, "k_op_from_codes");
-  } else {
+    dw = apart(dw, nd, cd);
+    rw = apart(rw, nr, cr);
+  }
+  csr_neighbours<K>(ctx, rk, nr, r_shift, nbr.p, rw);
+  if (trop)
+    expand_emit<K, int64_t, true>(ctx, dk, dw, nd, pos.p, T, 0, dmask, d_shift, ~0ull, out_shift, 0, off.p, n_nodes,
+                                  nbr.p, nr, rw, out, out_w, true);
+  else
     expand_emit<K, int32_t, false>(ctx, dk, nullptr, nd, pos.p, T, 0, dmask, d_shift, ~0ull, out_shift, 0, off.p,
                                    n_nodes, nbr.p, nr, nullptr, out, nullptr);
-  }
   sync_and_check(ctx);
   return T;
 }

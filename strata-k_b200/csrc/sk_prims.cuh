@@ -145,6 +145,22 @@ __device__ __forceinline__ uint64_t upper_bound_dev(const K* a, uint64_t lo, uin
   return lo;
 }
 
+// #items i of n with i + pos[i] < d (i + pos[i] strictly increasing), found by
+// one warp 32 probes at a time: four dependent loads for a million items where
+// one thread's binary search takes twenty.
+__device__ __forceinline__ uint64_t mp_before_warp(const uint64_t* pos, uint64_t n, uint64_t d) {
+  const int lane = threadIdx.x & 31;
+  uint64_t lo = 0, hi = d < n ? d : n;
+  while (lo < hi) {
+    const uint64_t step = (hi - lo) / 33 + 1;
+    const uint64_t mid = lo + (uint64_t)lane * step;
+    const int c = __popc(__ballot_sync(kFull, mid < hi && mid + pos[mid] < d));  // a prefix of the lanes
+    if (c < 32 && lo + (uint64_t)c * step < hi) hi = lo + (uint64_t)c * step;
+    if (c) lo += (uint64_t)(c - 1) * step + 1;
+  }
+  return lo;
+}
+
 // ---- Trop weights ----------------------------------------------------------------
 // A device lane holds a weight CODE.  The reference's Weight is Finite(i64) |
 // PosInf (strata-ir/src/trop.rs:35-40), so +inf must stay distinct from every

@@ -16,7 +16,10 @@
 //     written out in runs (coalesced per digit), values fetched through the
 //     source slot — no per-key value state stays in registers;
 //   * only the significant `bits` of the key are sorted (a 26-bit key takes 4
-//     passes, not 64) and passes whose digit is constant are skipped.
+//     passes, not 64), and where the host may look at the keys first only the
+//     bits that differ between them: a digit is up to eight such bits, from two
+//     separate windows of the key where one ends and the next begins (a packed
+//     pair (c0 << 32) | c1 of 19-bit ids takes 5 passes, not 6 or 8).
 #include "sk_ops.cuh"
 #include "sk_prims.cuh"
 
@@ -44,14 +47,40 @@ template <class K> struct RCfg;
 template <> struct RCfg<uint32_t> { static constexpr int ITEMS = 15; };
 template <> struct RCfg<uint64_t> { static constexpr int ITEMS = 9; };
 
+// A digit: l1 bits of the key from s1, and (m2 != 0) more from s2 above them.
+struct Digit {
+  int s1, s2, l1, bits;
+  uint32_t m1, m2;
+};
+struct Digits4 {
+  Digit d[4];
+};
+template <bool TWO, class K>
+__device__ __forceinline__ uint32_t digit_of(K k, const Digit& g) {
+  const uint32_t a = (uint32_t)(k >> g.s1) & g.m1;
+  return TWO ? a | (((uint32_t)(k >> g.s2) & g.m2) << g.l1) : a;
+}
+
+// The bits in which keys differ from keys[0].
+template <class K>
+__global__ void __launch_bounds__(NT) k_radix_varying(const K* __restrict__ keys, uint64_t n, unsigned long long* out) {
+  const K k0 = keys[0];
+  unsigned long long m = 0;
+  for (uint64_t i = (uint64_t)blockIdx.x * NT + threadIdx.x; i < n; i += (uint64_t)gridDim.x * NT)
+    m |= (unsigned long long)(keys[i] ^ k0);
+  const uint32_t lo = __reduce_or_sync(kFull, (uint32_t)m), hi = __reduce_or_sync(kFull, (uint32_t)(m >> 32));
+  m = ((unsigned long long)hi << 32) | lo;
+  if ((threadIdx.x & 31) == 0 && (m & ~*reinterpret_cast<volatile unsigned long long*>(out))) atomicOr(out, m);
+}
+
 // Digit histograms of passes [p0, p0 + np), np <= 4.  Each warp loads HI
 // keys per lane warp-striped (coalesced) and counts into its own shared
 // counters; when all 32 lanes of a full row hold the same digit (long runs of
 // equal high digits are the common case for packed keys) one add of 32
 // replaces 32 atomics.
-template <class K>
+template <class K, bool TWO>
 __global__ void __launch_bounds__(NT) k_radix_hist(const K* __restrict__ keys, uint64_t n, int p0,
-                                                   int np, uint32_t* __restrict__ hist) {
+                                                   int np, Digits4 dg, uint32_t* __restrict__ hist) {
   constexpr int HI = 8;
   __shared__ uint32_t sh[4][NW][RADIX];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -66,12 +95,13 @@ __global__ void __launch_bounds__(NT) k_radix_hist(const K* __restrict__ keys, u
       const uint64_t i = wb + j * 32 + lane;
       k[j] = i < n ? keys[i] : K(0);
     }
-    for (int p = 0; p < np; p++) {
-      const int sh_bits = 8 * (p0 + p);
+#pragma unroll
+    for (int p = 0; p < 4; p++) {  // unrolled: the digits stay in the constant bank
+      if (p >= np) break;
 #pragma unroll
       for (int j = 0; j < HI; j++) {
         const uint64_t row = wb + j * 32;
-        const uint32_t d = (uint32_t)(k[j] >> sh_bits) & 0xffu;
+        const uint32_t d = digit_of<TWO>(k[j], dg.d[p]);
         if (row + 31 < n) {  // warp-uniform: the whole row is in range
           const uint32_t d0 = __shfl_sync(kFull, d, 0);
           if (__all_sync(kFull, d == d0)) {
@@ -168,10 +198,10 @@ constexpr size_t onesweep_smem() {
 //  4. keys are staged in digit order (with their source slot when values
 //     ride along) and written out in runs, each value fetched from shared
 //     memory through its source slot.
-template <class K, class V, bool HAS_V, int ITEMS, int RANK, class LB = uint32_t>
+template <class K, class V, bool HAS_V, int ITEMS, int RANK, class LB = uint32_t, bool TWO = false>
 __global__ void __launch_bounds__(NT, 4) k_onesweep(const K* __restrict__ kin, K* __restrict__ kout,
                                                  const V* __restrict__ vin, V* __restrict__ vout,
-                                                 uint32_t n, int shift, int dbits,
+                                                 uint32_t n, Digit dg,
                                                  const uint32_t* __restrict__ binoff,
                                                  LB* lookback, uint32_t* tile_counter,
                                                  uint32_t* status, int bulk_ok) {
@@ -220,7 +250,7 @@ __global__ void __launch_bounds__(NT, 4) k_onesweep(const K* __restrict__ kin, K
       if constexpr (HAS_V) s_vin[i] = vin[base + i];
     }
   }
-  const uint32_t dmask = (1u << dbits) - 1;
+  const int dbits = dg.bits;
   const uint32_t wloc = (uint32_t)warp * 32u * ITEMS;  // this warp's first tile slot
   const unsigned lt = lanemask_lt();
   // every thread sees the keys (barrier phase, or the block barrier itself)
@@ -244,7 +274,7 @@ __global__ void __launch_bounds__(NT, 4) k_onesweep(const K* __restrict__ kin, K
 #pragma unroll
   for (int j = 0; j < ITEMS; j++) {
     const bool valid = wloc + j * 32 + lane < tile_n;
-    const uint32_t d = (uint32_t)(key[j] >> shift) & dmask;
+    const uint32_t d = digit_of<TWO>(key[j], dg);
     unsigned peers;
     if (rank_mode == 2) {
       // shared-mask ranking: each lane ORs its bit into its digit's mask;
@@ -320,7 +350,7 @@ __global__ void __launch_bounds__(NT, 4) k_onesweep(const K* __restrict__ kin, K
   for (int j = 0; j < ITEMS; j++) {
     const uint32_t li = wloc + j * 32 + lane;
     if (li < tile_n) {
-      const uint32_t d = (uint32_t)(key[j] >> shift) & dmask;
+      const uint32_t d = digit_of<TWO>(key[j], dg);
       const uint32_t pos = s_dstart[d] + s_whist[warp][d] + rank[j];
       s_keys[pos] = key[j];
       if constexpr (HAS_V) s_src[pos] = (uint16_t)li;
@@ -335,7 +365,7 @@ __global__ void __launch_bounds__(NT, 4) k_onesweep(const K* __restrict__ kin, K
     const uint32_t i = j * NT + tid;
     if (i < tile_n) {
       const K k = s_keys[i];
-      const uint32_t d = (uint32_t)(k >> shift) & dmask;
+      const uint32_t d = digit_of<TWO>(k, dg);
       const uint32_t dst = s_goff[d] + i;
       if (dst < n) {
         kout[dst] = k;
@@ -351,11 +381,67 @@ __global__ void __launch_bounds__(NT, 4) k_onesweep(const K* __restrict__ kin, K
 
 namespace {
 
+// `bits` low bits in contiguous 8-bit digits.
+std::vector<Digit> plain_digits(int bits) {
+  std::vector<Digit> g;
+  for (int s = 0; s < bits; s += 8) {
+    const int l = std::min(8, bits - s);
+    g.push_back(Digit{s, 0, l, l, (1u << l) - 1, 0u});
+  }
+  return g;
+}
+
+// Digits over the set bits of `vary`, lowest first: a window of at most eight
+// bits from the lowest one left (up to its last varying bit), then a second
+// window where the first leaves room.
+std::vector<Digit> varying_digits(uint64_t vary) {
+  std::vector<Digit> g;
+  auto window = [&](int room, int* s, uint32_t* m) {  // takes it off `vary`
+    *s = __builtin_ctzll(vary);
+    const uint64_t w = (vary >> *s) & ((1ull << room) - 1);
+    const int l = 64 - __builtin_clzll(w);
+    *m = (1u << l) - 1;
+    vary &= ~((uint64_t)*m << *s);
+    return l;
+  };
+  while (vary) {
+    Digit d{0, 0, 0, 0, 0u, 0u};
+    d.l1 = window(8, &d.s1, &d.m1);
+    d.bits = d.l1;
+    if (d.l1 < 8 && vary) d.bits += window(8 - d.l1, &d.s2, &d.m2);
+    g.push_back(d);
+  }
+  return g;
+}
+
+// kin / vin (optional): sort from these buffers, which stay as they are, into
+// *keys / *vals (the result is there on return).
 template <class K, class V, int ITEMS>
 void radix_sort_impl(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has_vals,
-                     uint64_t n, int bits, bool skip_trivial) {
+                     uint64_t n, int bits, bool look, const K* kin, const V* vin) {
   constexpr uint32_t TILE = NT * ITEMS;
-  const int passes = (bits + 7) / 8;
+  const K* src = kin ? kin : *keys;
+  const V* vsrc = vin ? vin : *vals;
+  std::vector<Digit> dg;
+  if (look) {
+    DBuf<uint64_t> m(ctx, 1);
+    SK_CUDA(cudaMemsetAsync(m.p, 0, 8, ctx->stream));
+    k_radix_varying<K><<<(unsigned)std::min<uint64_t>(ceil_div(n, NT * 8), (uint64_t)ctx->num_sms * 8), NT, 0,
+                         ctx->stream>>>(src, n, reinterpret_cast<unsigned long long*>(m.p));
+    after_launch(ctx, "k_radix_varying");
+    uint64_t vary;
+    read_u64(ctx, m.p, &vary, 1);
+    if (bits < 64) vary &= (1ull << bits) - 1;
+    dg = varying_digits(vary);
+  } else {
+    dg = plain_digits(bits);
+  }
+  const int passes = (int)dg.size();
+  if (passes == 0) {
+    if (kin) SK_CUDA(cudaMemcpyAsync(*keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, ctx->stream));
+    if (vin && has_vals) SK_CUDA(cudaMemcpyAsync(*vals, vin, n * sizeof(V), cudaMemcpyDeviceToDevice, ctx->stream));
+    return;
+  }
 
   DBuf<uint32_t> hist(ctx, passes * RADIX + passes);
   uint32_t* counters = hist.p + passes * RADIX;
@@ -363,25 +449,21 @@ void radix_sort_impl(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, boo
   const int hblocks = (int)std::min<uint64_t>(ceil_div(n, NT * 16), (uint64_t)ctx->num_sms * 4);
   for (int p0 = 0; p0 < passes; p0 += 4) {
     const int np = std::min(4, passes - p0);
+    Digits4 d4{};
+    bool two = false;
+    for (int p = 0; p < np; p++) {
+      d4.d[p] = dg[p0 + p];
+      two |= d4.d[p].m2 != 0;
+    }
     const int kh = kprof_begin(ctx, K_RADIX_HIST);
-    k_radix_hist<K><<<hblocks, NT, 0, ctx->stream>>>(*keys, n, p0, np, hist.p);
+    auto* count = two ? k_radix_hist<K, true> : k_radix_hist<K, false>;
+    count<<<hblocks, NT, 0, ctx->stream>>>(src, n, p0, np, d4, hist.p);
     kprof_end(ctx, kh, n * sizeof(K));
     after_launch(ctx, "k_radix_hist");
   }
   DBuf<uint32_t> binoff(ctx, passes * RADIX);
   k_radix_bins<<<passes, NT, 0, ctx->stream>>>(hist.p, binoff.p);
   after_launch(ctx, "k_radix_bins");
-
-  bool trivial[8] = {false, false, false, false, false, false, false, false};
-  if (skip_trivial) {
-    std::vector<uint32_t> h(passes * RADIX);
-    SK_CUDA(cudaMemcpyAsync(h.data(), hist.p, sizeof(uint32_t) * passes * RADIX,
-                            cudaMemcpyDeviceToHost, ctx->stream));
-    SK_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (int p = 0; p < passes; p++)
-      for (int d = 0; d < RADIX; d++)
-        if (h[p * RADIX + d] == n) trivial[p] = true;
-  }
 
   const uint32_t ntiles = (uint32_t)ceil_div(n, TILE);
   // 64-bit look-back words once a digit's count can reach 2^30
@@ -390,41 +472,55 @@ void radix_sort_impl(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, boo
   const size_t lb_bytes = lb_words * (wide_lb ? 8 : 4);
   DBuf<uint64_t> lookback(ctx, (lb_bytes + 7) / 8);
   const size_t smem = has_vals ? onesweep_smem<K, V, true, ITEMS>() : onesweep_smem<K, V, false, ITEMS>();
+  // the passes alternate between the two buffers; from kin the last one ends
+  // in *keys, in place the buffers swap with every pass
+  K* kdst = kin && passes % 2 ? *keys : *alt;
+  V* vdst = kin && passes % 2 ? *vals : *valt;
   for (int p = 0; p < passes; p++) {
-    if (trivial[p]) continue;
     SK_CUDA(cudaMemsetAsync(lookback.p, 0, lb_bytes, ctx->stream));
-    const int dbits = std::min(8, bits - 8 * p);
     const int kh = kprof_begin(ctx, K_ONESWEEP);
-    auto go = [&](auto rank_tag, auto lb_tag) {
+    auto go = [&](auto rank_tag, auto lb_tag, auto two_tag) {
       constexpr int RK = decltype(rank_tag)::value;
+      constexpr bool TWO = decltype(two_tag)::value;
       using LB = typename decltype(lb_tag)::type;
       LB* lbp = reinterpret_cast<LB*>(lookback.p);
       if (has_vals) {
-        auto kern = k_onesweep<K, V, true, ITEMS, RK, LB>;
+        auto kern = k_onesweep<K, V, true, ITEMS, RK, LB, TWO>;
         SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<ntiles, NT, smem, ctx->stream>>>(*keys, *alt, *vals, *valt, (uint32_t)n, 8 * p, dbits,
-                                                binoff.p + p * RADIX, lbp, counters + p, ctx->d_status,
-                                                aligned16(*keys) && aligned16(*vals) ? 1 : 0);
+        kern<<<ntiles, NT, smem, ctx->stream>>>(src, kdst, vsrc, vdst, (uint32_t)n, dg[p], binoff.p + p * RADIX, lbp,
+                                                counters + p, ctx->d_status,
+                                                aligned16(src) && aligned16(vsrc) ? 1 : 0);
       } else {
-        auto kern = k_onesweep<K, V, false, ITEMS, RK, LB>;
+        auto kern = k_onesweep<K, V, false, ITEMS, RK, LB, TWO>;
         SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<ntiles, NT, smem, ctx->stream>>>(*keys, *alt, nullptr, nullptr, (uint32_t)n, 8 * p, dbits,
+        kern<<<ntiles, NT, smem, ctx->stream>>>(src, kdst, nullptr, nullptr, (uint32_t)n, dg[p],
                                                 binoff.p + p * RADIX, lbp, counters + p, ctx->d_status,
-                                                aligned16(*keys) ? 1 : 0);
+                                                aligned16(src) ? 1 : 0);
       }
     };
-    if (wide_lb)  // the large sorts take the default ranking
-      go(std::integral_constant<int, 2>{}, LbTag<uint64_t>{});
-    else
+    using One = std::false_type;
+    if (dg[p].m2) {  // two windows, and the large sorts, take the default ranking
+      if (wide_lb) go(std::integral_constant<int, 2>{}, LbTag<uint64_t>{}, std::true_type{});
+      else go(std::integral_constant<int, 2>{}, LbTag<uint32_t>{}, std::true_type{});
+    } else if (wide_lb) {
+      go(std::integral_constant<int, 2>{}, LbTag<uint64_t>{}, One{});
+    } else {
       switch (ctx->tune_sort_rank) {
-        case 0: go(std::integral_constant<int, 0>{}, LbTag<uint32_t>{}); break;
-        case 1: go(std::integral_constant<int, 1>{}, LbTag<uint32_t>{}); break;
-        default: go(std::integral_constant<int, 2>{}, LbTag<uint32_t>{}); break;
+        case 0: go(std::integral_constant<int, 0>{}, LbTag<uint32_t>{}, One{}); break;
+        case 1: go(std::integral_constant<int, 1>{}, LbTag<uint32_t>{}, One{}); break;
+        default: go(std::integral_constant<int, 2>{}, LbTag<uint32_t>{}, One{}); break;
       }
+    }
     kprof_end(ctx, kh, 2 * n * (sizeof(K) + (has_vals ? sizeof(V) : 0)));
     after_launch(ctx, "k_onesweep");
-    std::swap(*keys, *alt);
-    if (has_vals) std::swap(*vals, *valt);
+    if (!kin) {
+      std::swap(*keys, *alt);
+      if (has_vals) std::swap(*vals, *valt);
+    }
+    src = kdst;
+    vsrc = vdst;
+    kdst = kdst == *keys ? *alt : *keys;
+    vdst = vdst == *vals ? *valt : *vals;
   }
 }
 
@@ -443,28 +539,36 @@ int radix_items_choices(int key_bytes, int* out, int max_out) {
 
 template <class K, class V>
 void radix_sort(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has_vals,
-                uint64_t n, int bits, bool skip_trivial) {
-  if (n <= 1 || bits <= 0) return;
+                uint64_t n, int bits, bool look, const K* kin, const V* vin) {
+  if (n <= 1 || bits <= 0) {
+    if (kin && n) SK_CUDA(cudaMemcpyAsync(*keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, ctx->stream));
+    if (vin && n && has_vals)
+      SK_CUDA(cudaMemcpyAsync(*vals, vin, n * sizeof(V), cudaMemcpyDeviceToDevice, ctx->stream));
+    return;
+  }
   if (n > kMaxSortKeys) fail(STRATA_E_UNSUPPORTED, "radix sort call limited to 2^32-1 keys");
   if (bits > (int)(8 * sizeof(K))) bits = 8 * sizeof(K);
+  auto run = [&](auto items) {
+    radix_sort_impl<K, V, decltype(items)::value>(ctx, keys, alt, vals, valt, has_vals, n, bits, look, kin, vin);
+  };
   if constexpr (sizeof(K) == 4) {
     switch (ctx->tune_items4) {
-      case 11: return radix_sort_impl<K, V, 11>(ctx, keys, alt, vals, valt, has_vals, n, bits, skip_trivial);
-      case 19: return radix_sort_impl<K, V, 19>(ctx, keys, alt, vals, valt, has_vals, n, bits, skip_trivial);
-      case 23: return radix_sort_impl<K, V, 23>(ctx, keys, alt, vals, valt, has_vals, n, bits, skip_trivial);
-      default: return radix_sort_impl<K, V, 15>(ctx, keys, alt, vals, valt, has_vals, n, bits, skip_trivial);
+      case 11: return run(std::integral_constant<int, 11>{});
+      case 19: return run(std::integral_constant<int, 19>{});
+      case 23: return run(std::integral_constant<int, 23>{});
+      default: return run(std::integral_constant<int, 15>{});
     }
   } else {
     switch (ctx->tune_items8) {
-      case 7: return radix_sort_impl<K, V, 7>(ctx, keys, alt, vals, valt, has_vals, n, bits, skip_trivial);
-      case 13: return radix_sort_impl<K, V, 13>(ctx, keys, alt, vals, valt, has_vals, n, bits, skip_trivial);
-      default: return radix_sort_impl<K, V, 9>(ctx, keys, alt, vals, valt, has_vals, n, bits, skip_trivial);
+      case 7: return run(std::integral_constant<int, 7>{});
+      case 13: return run(std::integral_constant<int, 13>{});
+      default: return run(std::integral_constant<int, 9>{});
     }
   }
 }
 
 #define SK_INST_SORT(K, V)                                                                   \
-  template void radix_sort<K, V>(strata_ctx*, K**, K**, V**, V**, bool, uint64_t, int, bool);
+  template void radix_sort<K, V>(strata_ctx*, K**, K**, V**, V**, bool, uint64_t, int, bool, const K*, const V*);
 SK_INST_SORT(uint32_t, uint32_t)
 SK_INST_SORT(uint32_t, uint64_t)
 SK_INST_SORT(uint64_t, uint32_t)
@@ -496,7 +600,12 @@ void radix_sort_u32_static(cudaStream_t stream, const uint32_t* in, uint32_t* ou
   // Everything that must start at zero is cleared on every call.
   check_cuda(cudaMemsetAsync(hist, 0, (4 * RADIX + 4 * RADIX + 32) * 4, stream), "cudaMemsetAsync");
   const int hblocks = (int)std::min<uint64_t>(ceil_div(n, NT * 16), 148 * 4);
-  k_radix_hist<uint32_t><<<hblocks, NT, 0, stream>>>(in, n, 0, passes, hist);
+  Digits4 d4{};
+  for (int p = 0; p < passes; p++) {
+    const int l = std::min(8, bits - 8 * p);
+    d4.d[p] = Digit{8 * p, 0, l, l, (1u << l) - 1, 0u};
+  }
+  k_radix_hist<uint32_t, false><<<hblocks, NT, 0, stream>>>(in, n, 0, passes, d4, hist);
   k_radix_bins<<<passes, NT, 0, stream>>>(hist, binoff);
   const size_t smem = onesweep_smem<uint32_t, uint32_t, false, ITEMS>();
   const uint32_t* src = in;
@@ -505,7 +614,7 @@ void radix_sort_u32_static(cudaStream_t stream, const uint32_t* in, uint32_t* ou
     uint32_t* dst = ((passes - 1 - p) % 2 == 0) ? out : alt;
     check_cuda(cudaMemsetAsync(lookback, 0, sizeof(uint32_t) * ntiles * RADIX, stream), "cudaMemsetAsync");
     auto kern = k_onesweep<uint32_t, uint32_t, false, ITEMS, 2>;
-    kern<<<ntiles, NT, smem, stream>>>(src, dst, nullptr, nullptr, (uint32_t)n, 8 * p, std::min(8, bits - 8 * p),
+    kern<<<ntiles, NT, smem, stream>>>(src, dst, nullptr, nullptr, (uint32_t)n, d4.d[p],
                                        binoff + p * RADIX, lookback, counters + p, status,
                                        aligned16(src) ? 1 : 0);
     src = dst;

@@ -196,17 +196,21 @@ __global__ void __launch_bounds__(NT)
 constexpr int EE_ITEMS = 6;
 constexpr uint32_t EE_TILE = NT * EE_ITEMS;
 
-// #items i with i + pos[i] < d  (i + pos[i] is strictly increasing).
-__device__ __forceinline__ uint64_t mp_items_before(const uint64_t* pos, uint64_t n, uint64_t d) {
-  uint64_t lo = 0, hi = d < n ? d : n;
-  while (lo < hi) {
-    const uint64_t mid = (lo + hi) >> 1;
-    if (mid + pos[mid] < d) lo = mid + 1; else hi = mid;
-  }
-  return lo;
+// OP: the weights are the operator surface's (int64, INT64_MAX = +inf), turned
+// into codes as they are read and back as they are written; a finite weight
+// without a code is reported for every Δ row, joined or not.  The tile's splits
+// are found by two warps in parallel (one thread's two binary searches kept
+// the block waiting for most of its time: 1 M rows with 4 M outputs of 16
+// bytes, one B200, 90 -> 67 us, the conversions that were three more launches
+// included).
+template <class W>
+__device__ __forceinline__ W op_code(W v, uint32_t* flags) {
+  if (v == WAbs<W>::v) return WInf<W>::v;  // the surface's +inf is the type's maximum
+  if (v > WFinMax<W>::v) *flags |= ST_SENTINEL;
+  return v;
 }
 
-template <class K, class W, bool TROP>
+template <class K, class W, bool TROP, bool OP>
 __global__ void __launch_bounds__(NT)
     k_expand_emit(const K* __restrict__ dkeys, const W* __restrict__ dw, uint64_t n,
                   const uint64_t* __restrict__ pos, uint64_t total, int jshift, uint64_t jmask,
@@ -223,14 +227,17 @@ __global__ void __launch_bounds__(NT)
   const uint64_t L = n + total;
   const uint64_t d0 = (uint64_t)blockIdx.x * EE_TILE;
   const uint64_t d1 = d0 + EE_TILE < L ? d0 + EE_TILE : L;
-  if (tid == 0) {
-    const uint64_t i0 = mp_items_before(pos, n, d0);
-    const uint64_t i1 = mp_items_before(pos, n, d1);
-    s_r[0] = i0 > 0 ? i0 - 1 : 0;  // first item that may own an output here
-    s_r[1] = i1;
-    s_r[2] = d0 - i0;              // first output of the tile
-    s_r[3] = d1 - i1;              // one past the last output
+  if (tid < 64) {
+    const uint64_t x = mp_before_warp(pos, n, tid < 32 ? d0 : d1);
+    if (tid == 0) {
+      s_r[0] = x > 0 ? x - 1 : 0;  // first item that may own an output here
+      s_r[2] = d0 - x;             // first output of the tile
+    } else if (tid == 32) {
+      s_r[1] = x;
+      s_r[3] = d1 - x;             // one past the last output
+    }
   }
+  uint32_t flags = 0;
   __syncthreads();
   const uint64_t a = s_r[0], i1 = s_r[1], o0 = s_r[2], o1 = s_r[3];
   if (i1 - a > EE_TILE + 1) {  // cannot happen for a valid pos[]; never index past smem
@@ -245,10 +252,9 @@ __global__ void __launch_bounds__(NT)
     s_pos[k] = pos[i];
     s_seg[k] = jv < n_nodes ? off[jv] : 0u;
     s_kept[k] = (K)(((uint64_t)key >> pshift) & pmask);
-    if constexpr (TROP) s_w[k] = dw[i];
+    if constexpr (TROP) s_w[k] = OP ? op_code(dw[i], &flags) : dw[i];
   }
   __syncthreads();
-  uint32_t flags = 0;
   const uint64_t o_end = o1 < total ? o1 : total;  // o1 <= total for a valid pos[]
   for (uint64_t o = o0 + tid; o < o_end; o += NT) {
     // owner = last loaded item with pos <= o
@@ -263,7 +269,10 @@ __global__ void __launch_bounds__(NT)
     if (e >= n_nbr) { flags |= ST_BOUNDS; continue; }
     const uint32_t v = nbr[e];
     out[o] = (K)(((K)s_kept[li] << out_pshift) | ((K)v << out_vshift));
-    if constexpr (TROP) out_w[o] = trop_mul(s_w[li], nbr_w[e], wshift, &flags);
+    if constexpr (TROP) {
+      const W r = trop_mul(s_w[li], OP ? op_code(nbr_w[e], &flags) : nbr_w[e], wshift, &flags);
+      out_w[o] = OP && r == WInf<W>::v ? WAbs<W>::v : r;
+    }
   }
   if (flags) atomicOr(status, flags);
 }
@@ -458,42 +467,46 @@ __global__ void __launch_bounds__(NT)
 }
 
 // ---------------------------------------------------------------------------
-// merge_diff: full ∪ cand and the delta, one merge-path pass
+// merge_diff: full ∪ cand and the delta over merge-path tiles
 // ---------------------------------------------------------------------------
 constexpr int MD_ITEMS = 6;
 constexpr uint32_t MD_TILE = NT * MD_ITEMS;
+constexpr int MD_PER = MD_ITEMS + 1;  // merged positions a thread (a tile holds up to MD_TILE + 1)
 
-// Merge-path split of diagonal d: #A among the first d merged elements (A wins
-// ties), then moved so that an equal pair A[i-1] == B[j] stays in one tile.
+// Merge-path split of every tile boundary, one warp each: the rows of A among
+// the first d merged ones (A wins ties), found 32 probes at a time, then moved
+// so that an equal pair A[i-1] == B[j] stays in one tile.  splits[2t],
+// splits[2t + 1] = the rows of A and B before diagonal min(t * MD_TILE, na + nb).
 template <class K>
-__device__ void md_split(const K* A, uint64_t na, const K* B, uint64_t nb, uint64_t d,
-                         uint64_t* oi, uint64_t* oj) {
-  uint64_t lo = d > nb ? d - nb : 0, hi = d < na ? d : na;
-  while (lo < hi) {
-    const uint64_t mid = (lo + hi) >> 1;
-    if (A[mid] <= B[d - mid - 1]) lo = mid + 1; else hi = mid;
-  }
-  uint64_t i = lo, j = d - lo;
-  if (i > 0 && j < nb && A[i - 1] == B[j]) j++;
-  *oi = i;
-  *oj = j;
-}
-
-// Merge-path splits of every tile boundary at once (one thread per
-// diagonal): splits[2t], splits[2t+1] = md_split of diagonal min(t*MD_TILE, na+nb).
-template <class K>
-__global__ void k_md_bounds(const K* __restrict__ A, uint64_t na, const K* __restrict__ B, uint64_t nb,
-                            uint32_t tiles, uint64_t* __restrict__ splits) {
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(NT) k_md_bounds(const K* __restrict__ A, uint64_t na, const K* __restrict__ B,
+                                                  uint64_t nb, uint32_t tiles, uint64_t* __restrict__ splits) {
+  const uint64_t t = ((uint64_t)blockIdx.x * NT + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   if (t > tiles) return;
   const uint64_t L = na + nb, d = t * MD_TILE < L ? t * MD_TILE : L;
-  md_split(A, na, B, nb, d, &splits[2 * t], &splits[2 * t + 1]);
+  uint64_t lo = d > nb ? d - nb : 0, hi = d < na ? d : na;
+  while (lo < hi) {
+    const uint64_t step = (hi - lo) / 33 + 1, mid = lo + (uint64_t)lane * step;
+    const int c = __popc(__ballot_sync(kFull, mid < hi && A[mid] <= B[d - mid - 1]));  // a prefix of the lanes
+    if (c < 32 && lo + (uint64_t)c * step < hi) hi = lo + (uint64_t)c * step;
+    if (c) lo += (uint64_t)(c - 1) * step + 1;
+  }
+  if (lane == 0) {
+    const uint64_t i = lo, j = d - lo;
+    splits[2 * t] = i;
+    splits[2 * t + 1] = j + (i > 0 && j < nb && A[i - 1] == B[j] ? 1 : 0);
+  }
 }
 
 // Two passes over the same tiles, reduce-then-scan (no tile waits on
 // another): PASS 0 counts each tile's full-out rows and Δ' rows into
 // tile_full / tile_delta; after their exclusive scan, PASS 1 recomputes the tile
-// and writes its rows at the scanned offsets.
+// and writes its rows at the scanned offsets.  A thread finds its place on the
+// tile's merge path with one binary search and then merges MD_PER rows in
+// turn (a binary search for every row, 2 x 11 shared-memory reads each, bound
+// the earlier form); the rows leave through shared memory, coalesced.  Delta
+// round of 2 M rows against 3.2 M candidates of 16 bytes, one B200: both
+// passes 225 -> 140 us.
 template <class K, class W, bool TROP, bool WRITE_FULL, bool WRITE_DELTA, bool INPLACE, int PASS>
 __global__ void __launch_bounds__(NT)
     k_merge_diff(const K* __restrict__ A, W* Aw, uint64_t na, const K* __restrict__ B,
@@ -502,137 +515,122 @@ __global__ void __launch_bounds__(NT)
                  uint64_t* tile_full, uint64_t* tile_delta, uint32_t* status) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   constexpr uint32_t CAP = MD_TILE + 2;
-  K* s_a = reinterpret_cast<K*>(s_raw);
-  K* s_b = s_a + CAP;
-  W* s_aw = reinterpret_cast<W*>(s_b + CAP);
-  W* s_bw = s_aw + (TROP ? CAP : 0);
-  uint32_t* s_mpre = reinterpret_cast<uint32_t*>(s_bw + (TROP ? CAP : 0));  // CAP + 1
-  uint32_t* s_dpre = s_mpre + CAP + 1;                                      // CAP
+  // keys of A, then of B; on the way out the full rows' keys, then Δ's (at
+  // most acnt + bcnt and bcnt of them); the weights beside them
+  K* s_k = reinterpret_cast<K*>(s_raw);
+  W* s_w = reinterpret_cast<W*>(s_k + 2 * CAP);
   __shared__ uint32_t s_scan[NT / 32 + 1];
   const int tid = threadIdx.x;
   const uint32_t tile = blockIdx.x;
-  const uint64_t s_r[4] = {splits[2 * tile], splits[2 * tile + 1], splits[2 * tile + 2], splits[2 * tile + 3]};
-  const uint64_t i0 = s_r[0], j0 = s_r[1];
+  const uint64_t i0 = splits[2 * tile], j0 = splits[2 * tile + 1];
+  const uint64_t i1 = splits[2 * tile + 2], j1 = splits[2 * tile + 3];
   // Impossible for sorted unique inputs; checked so unsorted input cannot
   // index past shared memory.
-  const bool oversize = s_r[2] < i0 || s_r[3] < j0 || (s_r[2] - i0) > MD_TILE + 1 ||
-                        (s_r[3] - j0) > MD_TILE + 1 || (s_r[2] - i0) + (s_r[3] - j0) > MD_TILE + 1;
+  const bool oversize = i1 < i0 || j1 < j0 || i1 - i0 > MD_TILE + 1 || j1 - j0 > MD_TILE + 1 ||
+                        (i1 - i0) + (j1 - j0) > MD_TILE + 1;
   if (oversize && tid == 0) atomicOr(status, ST_BOUNDS);
-  const uint32_t acnt = oversize ? 0u : (uint32_t)(s_r[2] - i0);
-  const uint32_t bcnt = oversize ? 0u : (uint32_t)(s_r[3] - j0);
-  constexpr int BI = (MD_TILE + 2 + NT - 1) / NT;
+  const uint32_t acnt = oversize ? 0u : (uint32_t)(i1 - i0);
+  const uint32_t bcnt = oversize ? 0u : (uint32_t)(j1 - j0);
+  const uint32_t n = acnt + bcnt;
 #pragma unroll
-  for (int q = 0; q < BI; q++) {
+  for (int q = 0; q < MD_PER; q++) {
     const uint32_t k = q * NT + tid;
-    if (k < acnt) {
-      s_a[k] = A[i0 + k];
-      if constexpr (TROP) s_aw[k] = Aw[i0 + k];
-    }
-    if (k < bcnt) {
-      s_b[k] = B[j0 + k];
-      if constexpr (TROP) s_bw[k] = Bw[j0 + k];
+    if (k < n) {
+      s_k[k] = k < acnt ? A[i0 + k] : B[j0 + (k - acnt)];
+      if constexpr (TROP) s_w[k] = k < acnt ? Aw[i0 + k] : Bw[j0 + (k - acnt)];
     }
   }
   __syncthreads();
-  // Per B element: rank in A, matched?, delta?
-  uint32_t b_ra[BI];
-  uint32_t mflag = 0, dflag = 0;  // bit per item
-  uint32_t mcount = 0, dcount = 0;
-  const uint32_t bb = tid * BI;
+  const K* a = s_k;
+  const K* b = s_k + acnt;
+  const W* aw = s_w;
+  const W* bw = s_w + acnt;
+  // this thread's place on the merge path (A first on ties)
+  const uint32_t d = min((uint32_t)tid * MD_PER, n);
+  uint32_t lo = d > bcnt ? d - bcnt : 0, hi = d < acnt ? d : acnt;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (a[mid] <= b[d - mid - 1]) lo = mid + 1; else hi = mid;
+  }
+  uint32_t i = lo, j = d - lo;
+  K kk[MD_PER];
+  W ww[MD_PER];
+  uint32_t fm = 0, dm = 0;  // positions that go to the full relation / to Δ'
 #pragma unroll
-  for (int q = 0; q < BI; q++) {
-    const uint32_t jb = bb + q;
-    b_ra[q] = 0;
-    if (jb < bcnt) {
-      const K x = s_b[jb];
-      uint32_t lo = 0, hi = acnt;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (s_a[mid] < x) lo = mid + 1; else hi = mid;
+  for (int q = 0; q < MD_PER; q++) {
+    kk[q] = K(0);
+    ww[q] = W(0);
+    if (d + q >= n) continue;
+    if (i < acnt && (j >= bcnt || a[i] <= b[j])) {
+      kk[q] = a[i];
+      fm |= 1u << q;
+      if constexpr (TROP) {
+        ww[q] = aw[i];
+        if (j < bcnt && b[j] == a[i] && bw[j] < ww[q]) ww[q] = bw[j];
       }
-      b_ra[q] = lo;
-      const bool m = lo < acnt && s_a[lo] == x;
-      bool dl = !m;
-      if constexpr (TROP) dl = dl || (s_bw[jb] < s_aw[lo]);
-      if (m) { mflag |= 1u << q; mcount++; }
-      if (dl) { dflag |= 1u << q; dcount++; }
+      i++;
+    } else {
+      const bool match = i > 0 && a[i - 1] == b[j];
+      kk[q] = b[j];
+      bool changed = !match;
+      if constexpr (TROP) {
+        ww[q] = bw[j];
+        if (match && bw[j] < aw[i - 1]) {
+          changed = true;
+          if constexpr (INPLACE && PASS == 1) Aw[i0 + i - 1] = bw[j];
+        }
+      }
+      if (!match) fm |= 1u << q;
+      if (changed) dm |= 1u << q;
+      j++;
     }
   }
-  uint32_t mtot, dtot;
-  const uint32_t mex = block_excl_sum<NT>(mcount, s_scan, &mtot);
-  const uint32_t dex = block_excl_sum<NT>(dcount, s_scan, &dtot);
-  {
-    uint32_t mr = mex, dr = dex;
-#pragma unroll
-    for (int q = 0; q < BI; q++) {
-      const uint32_t jb = bb + q;
-      if (jb < bcnt) {
-        s_mpre[jb] = mr;
-        s_dpre[jb] = dr;
-        mr += (mflag >> q) & 1u;
-        dr += (dflag >> q) & 1u;
-      }
-    }
-    if (tid == 0) s_mpre[bcnt] = mtot;
-  }
-  const uint32_t fcnt = acnt + bcnt - mtot;
+  // both counts in one scan (a tile has fewer than 2^16 rows)
+  uint32_t tot;
+  const uint32_t ex = block_excl_sum<NT>((uint32_t)__popc(fm) | ((uint32_t)__popc(dm) << 16), s_scan, &tot);
+  const uint32_t ftot = tot & 0xffffu, dtot = tot >> 16;
   if constexpr (PASS == 0) {
     if (tid == 0) {
-      tile_full[tile] = fcnt;
+      tile_full[tile] = ftot;
       tile_delta[tile] = dtot;
     }
     return;
   }
-  const uint64_t fex = tile_full[tile], dexg = tile_delta[tile];
-  __syncthreads();  // every thread's s_mpre / s_dpre entries are read below
-  // B elements: unmatched -> full_out; delta -> delta out.
+  // every thread has read its rows (the scan's barriers); stage and write
+  uint32_t f = ex & 0xffffu, e = ftot + (ex >> 16);
 #pragma unroll
-  for (int q = 0; q < BI; q++) {
-    const uint32_t jb = bb + q;
-    if (jb < bcnt) {
-      const bool m = (mflag >> q) & 1u;
-      if (WRITE_FULL && !m) {
-        const uint64_t p = fex + b_ra[q] + (jb - s_mpre[jb]);
-        if (p < na + nb) {
-          fout[p] = s_b[jb];
-          if constexpr (TROP) fout_w[p] = s_bw[jb];
-        } else {
-          atomicOr(status, ST_BOUNDS);
-        }
-      }
-      if (WRITE_DELTA && ((dflag >> q) & 1u)) {
-        const uint64_t p = dexg + s_dpre[jb];
-        if (p < nb) {
-          dout[p] = s_b[jb];
-          if constexpr (TROP) dout_w[p] = s_bw[jb];
-        } else {
-          atomicOr(status, ST_BOUNDS);
-        }
-      }
-      if constexpr (TROP && INPLACE) {
-        if (m && s_bw[jb] < s_aw[b_ra[q]]) Aw[i0 + b_ra[q]] = s_bw[jb];
-      }
+  for (int q = 0; q < MD_PER; q++) {
+    if (WRITE_FULL && ((fm >> q) & 1u)) {
+      s_k[f] = kk[q];
+      if constexpr (TROP) s_w[f] = ww[q];
+      f++;
+    }
+    if (WRITE_DELTA && ((dm >> q) & 1u)) {
+      s_k[e] = kk[q];
+      if constexpr (TROP) s_w[e] = ww[q];
+      e++;
     }
   }
+  __syncthreads();
+  const uint64_t fex = tile_full[tile], dex = tile_delta[tile];
   if constexpr (WRITE_FULL) {
-    for (uint32_t ia = tid; ia < acnt; ia += NT) {
-      const K x = s_a[ia];
-      uint32_t lo = 0, hi = bcnt;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (s_b[mid] < x) lo = mid + 1; else hi = mid;
-      }
-      const uint64_t p = fex + ia + (lo - s_mpre[lo]);
-      if (p >= na + nb) {
+    for (uint32_t k = tid; k < ftot; k += NT) {
+      if (fex + k >= na + nb) {
         atomicOr(status, ST_BOUNDS);
-        continue;
+        break;
       }
-      fout[p] = x;
-      if constexpr (TROP) {
-        W wv = s_aw[ia];
-        if (lo < bcnt && s_b[lo] == x && s_bw[lo] < wv) wv = s_bw[lo];
-        fout_w[p] = wv;
+      fout[fex + k] = s_k[k];
+      if constexpr (TROP) fout_w[fex + k] = s_w[k];
+    }
+  }
+  if constexpr (WRITE_DELTA) {
+    for (uint32_t k = tid; k < dtot; k += NT) {
+      if (dex + k >= nb) {
+        atomicOr(status, ST_BOUNDS);
+        break;
       }
+      dout[dex + k] = s_k[ftot + k];
+      if constexpr (TROP) dout_w[dex + k] = s_w[ftot + k];
     }
   }
 }
@@ -655,10 +653,14 @@ __global__ void k_csr_offsets(const K* __restrict__ keys, uint64_t m, int vbits,
   off[j] = (uint32_t)lo;
 }
 
+// op_w (optional): operator-surface weights of the rows, checked for a code.
 template <class K>
-__global__ void k_csr_nbr(const K* __restrict__ keys, uint64_t m, uint64_t vmask, uint32_t* __restrict__ nbr) {
+__global__ void k_csr_nbr(const K* __restrict__ keys, uint64_t m, uint64_t vmask, uint32_t* __restrict__ nbr,
+                          const int64_t* __restrict__ op_w, uint32_t* status) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < m) nbr[i] = (uint32_t)((uint64_t)keys[i] & vmask);
+  if (i >= m) return;
+  nbr[i] = (uint32_t)((uint64_t)keys[i] & vmask);
+  if (op_w && op_w[i] > WFinMax<int64_t>::v && op_w[i] != INT64_MAX) atomicOr(status, ST_SENTINEL);
 }
 
 __global__ void k_mark_ids(const uint32_t* __restrict__ a, uint64_t n, uint32_t* bitmap, uint64_t limit) {
@@ -1006,12 +1008,17 @@ template <class K, class W, bool TROP>
 void expand_emit(strata_ctx* ctx, const K* dkeys, const W* dw, uint64_t n, const uint64_t* pos,
                  uint64_t total, int jshift, uint64_t jmask, int pshift, uint64_t pmask,
                  int out_pshift, int out_vshift, const uint32_t* off, uint64_t n_nodes,
-                 const uint32_t* nbr, uint64_t n_nbr, const W* nbr_w, K* out, W* out_w) {
+                 const uint32_t* nbr, uint64_t n_nbr, const W* nbr_w, K* out, W* out_w, bool op_weights) {
   if (total == 0 || n == 0) return;
   const uint64_t tiles = ceil_div(n + total, EE_TILE);
   if (tiles > 0x7fffffffull) fail(STRATA_E_UNSUPPORTED, "expand too large for one launch");
   const int kh = kprof_begin(ctx, K_EXPAND_EMIT);
-  k_expand_emit<K, W, TROP><<<(unsigned)tiles, NT, 0, ctx->stream>>>(
+  // only the operator surface's weights (int64) need the conversion
+  auto* kern = k_expand_emit<K, W, TROP, false>;
+  if constexpr (TROP && sizeof(W) == 8) {
+    if (op_weights) kern = k_expand_emit<K, W, TROP, true>;
+  }
+  kern<<<(unsigned)tiles, NT, 0, ctx->stream>>>(
       dkeys, dw, n, pos, total, jshift, jmask, pshift, pmask, out_pshift, out_vshift, off, n_nodes,
       nbr, n_nbr, nbr_w, out, out_w, ctx->wshift, ctx->d_status);
   const uint64_t wsz = TROP ? sizeof(W) : 0;
@@ -1059,10 +1066,11 @@ static void launch_merge(strata_ctx* ctx, const K* full, W* full_w, uint64_t nf,
   uint64_t* fcount = buf.p;
   uint64_t* dcount = buf.p + tiles + 1;
   uint64_t* splits = buf.p + 2ull * (tiles + 1);
-  k_md_bounds<K><<<(unsigned)ceil_div(tiles + 1, NT), NT, 0, ctx->stream>>>(full, nf, cand, nc, tiles, splits);
+  k_md_bounds<K><<<(unsigned)ceil_div((uint64_t)tiles + 1, NT / 32), NT, 0, ctx->stream>>>(full, nf, cand, nc, tiles,
+                                                                                           splits);
   after_launch(ctx, "k_md_bounds");
   constexpr uint32_t CAP = MD_TILE + 2;
-  const size_t smem = 2 * CAP * sizeof(K) + (TROP ? 2 * CAP * sizeof(W) : 0) + (2 * CAP + 1) * sizeof(uint32_t);
+  const size_t smem = 2 * CAP * (sizeof(K) + (TROP ? sizeof(W) : 0));
   auto count = k_merge_diff<K, W, TROP, WF, WD, IP, 0>;
   auto write = k_merge_diff<K, W, TROP, WF, WD, IP, 1>;
   SK_CUDA(cudaFuncSetAttribute(count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1111,16 +1119,25 @@ void diff_improve(strata_ctx* ctx, const K* cand, const W* cand_w, uint64_t nc, 
 }
 
 template <class K>
-void build_csr(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint64_t n_nodes,
-               uint32_t* off, uint32_t* nbr) {
+void csr_offsets(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint64_t n_nodes, uint32_t* off) {
   if (m >= 0xffffffffull) fail(STRATA_E_UNSUPPORTED, "CSR limited to 2^32-1 edges");
   k_csr_offsets<K><<<(unsigned)ceil_div(n_nodes + 1, NT), NT, 0, ctx->stream>>>(keys, m, vbits, n_nodes, off);
   after_launch(ctx, "k_csr_offsets");
-  if (m) {
-    const uint64_t vmask = vbits >= 64 ? ~0ull : ((1ull << vbits) - 1);
-    k_csr_nbr<K><<<(unsigned)ceil_div(m, NT), NT, 0, ctx->stream>>>(keys, m, vmask, nbr);
-    after_launch(ctx, "k_csr_nbr");
-  }
+}
+
+template <class K>
+void csr_neighbours(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint32_t* nbr, const int64_t* op_w) {
+  if (!m) return;
+  const uint64_t vmask = vbits >= 64 ? ~0ull : ((1ull << vbits) - 1);
+  k_csr_nbr<K><<<(unsigned)ceil_div(m, NT), NT, 0, ctx->stream>>>(keys, m, vmask, nbr, op_w, ctx->d_status);
+  after_launch(ctx, "k_csr_nbr");
+}
+
+template <class K>
+void build_csr(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint64_t n_nodes,
+               uint32_t* off, uint32_t* nbr) {
+  csr_offsets<K>(ctx, keys, m, vbits, n_nodes, off);
+  csr_neighbours<K>(ctx, keys, m, vbits, nbr, nullptr);
 }
 
 uint64_t count_distinct_ids(strata_ctx* ctx, const uint32_t* a, uint64_t na, const uint32_t* b,
@@ -1277,6 +1294,10 @@ template void expand_offsets<uint32_t>(strata_ctx*, const uint32_t*, uint64_t, i
                                        uint64_t*, uint32_t, uint64_t*);
 template void expand_offsets<uint64_t>(strata_ctx*, const uint64_t*, uint64_t, int, uint64_t, const uint32_t*, uint64_t,
                                        uint64_t*, uint32_t, uint64_t*);
+template void csr_offsets<uint32_t>(strata_ctx*, const uint32_t*, uint64_t, int, uint64_t, uint32_t*);
+template void csr_neighbours<uint32_t>(strata_ctx*, const uint32_t*, uint64_t, int, uint32_t*, const int64_t*);
+template void csr_offsets<uint64_t>(strata_ctx*, const uint64_t*, uint64_t, int, uint64_t, uint32_t*);
+template void csr_neighbours<uint64_t>(strata_ctx*, const uint64_t*, uint64_t, int, uint32_t*, const int64_t*);
 template void build_csr<uint32_t>(strata_ctx*, const uint32_t*, uint64_t, int, uint64_t, uint32_t*, uint32_t*);
 template void build_csr<uint64_t>(strata_ctx*, const uint64_t*, uint64_t, int, uint64_t, uint32_t*, uint32_t*);
 
@@ -1284,7 +1305,7 @@ template void build_csr<uint64_t>(strata_ctx*, const uint64_t*, uint64_t, int, u
   template void expand_emit<K, W, T>(strata_ctx*, const K*, const W*, uint64_t, const uint64_t*,     \
                                      uint64_t, int, uint64_t, int, uint64_t, int, int,               \
                                      const uint32_t*, uint64_t, const uint32_t*, uint64_t, const W*, \
-                                     K*, W*);                                                        \
+                                     K*, W*, bool);                                                        \
   template void reduce_runs<K, W, T>(strata_ctx*, const K*, const W*, uint64_t, K*, W*, uint64_t*);  \
   template void merge_diff<K, W, T>(strata_ctx*, const K*, const W*, uint64_t, const K*, const W*,   \
                                     uint64_t, K*, W*, K*, W*, uint64_t*);                            \

@@ -775,14 +775,15 @@ __global__ void k_tri_list_sum(const K* __restrict__ keys, uint64_t m, int bits,
 }
 
 // Sort + dedup packed keys in `keys` (n), result in out (returns count).
+// `look`: the keys may vary in few of their bits (packed ids vary in all).
 template <class K>
-uint64_t sort_unique(strata_ctx* ctx, DBuf<K>& keys, uint64_t n, int bits, DBuf<K>& out) {
+uint64_t sort_unique(strata_ctx* ctx, DBuf<K>& keys, uint64_t n, int bits, DBuf<K>& out, bool look = false) {
   DBuf<K> alt(ctx, n + 1);
   K* kp = keys.p;
   K* ka = alt.p;
   uint32_t* vp = nullptr;
   uint32_t* va = nullptr;
-  radix_sort<K, uint32_t>(ctx, &kp, &ka, &vp, &va, false, n, bits, true);
+  radix_sort<K, uint32_t>(ctx, &kp, &ka, &vp, &va, false, n, bits, look);
   out.reserve(n + 1);
   DBuf<uint64_t> cnt(ctx, 1);
   reduce_runs<K, int32_t, false>(ctx, kp, nullptr, n, out.p, nullptr, cnt.p);
@@ -1034,7 +1035,7 @@ uint64_t oriented_edges(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, u
   K* ka = alt.p;
   uint32_t* vp = nullptr;
   uint32_t* va = nullptr;
-  radix_sort<K, uint32_t>(ctx, &kp, &ka, &vp, &va, false, m, 2 * bits, true);
+  radix_sort<K, uint32_t>(ctx, &kp, &ka, &vp, &va, false, m, 2 * bits, false);
   if (kp == uniq.p) out = std::move(uniq);
   else out = std::move(alt);
   return m;
@@ -1191,7 +1192,7 @@ uint64_t intern_terms(strata_ctx* ctx, const uint64_t* keys, uint64_t n, uint32_
   DBuf<uint64_t> copy(ctx, n + 1), table;
   table.ctx = ctx;
   SK_CUDA(cudaMemcpyAsync(copy.p, keys, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-  const uint64_t m = sort_unique<uint64_t>(ctx, copy, n, std::max(1, bits_for(maxk)), table);
+  const uint64_t m = sort_unique<uint64_t>(ctx, copy, n, std::max(1, bits_for(maxk)), table, true);
   k_intern_map<<<blocks(n), 256, 0, ctx->stream>>>(keys, n, table.p, m, ids);
   after_launch(ctx, "k_intern_map");
   sync_and_check(ctx);
