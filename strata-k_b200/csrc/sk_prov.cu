@@ -33,9 +33,9 @@
 //     that contains it is rejected with it.
 //   * One that weighs less than all proofs of a full set: with probabilities
 //     in [0, 1] a subset never weighs less than its superset, so it absorbs no
-//     proof and no heavier candidate, and pruning drops it — unless the other
-//     candidates absorb more proofs than they add; then the batch is done
-//     again with it.  (The test keeps a margin of 1e-9 against the rounding of
+//     proof and no heavier candidate, and pruning drops it — unless fewer than k
+//     heavier proofs are left once the other candidates have absorbed theirs;
+//     then the batch is done again with it.  (The test keeps a margin of 1e-9 against the rounding of
 //     the products, 4e-15.)
 // What remains (usually a candidate or two of eight) is tested against the set
 // and each other, weighed if accepted, and ranked.
@@ -336,20 +336,24 @@ __global__ void __launch_bounds__(PV_NT, PV_BLOCKS) k_prov_round(PvView v) {
       const bool surv = (hl < 8 && valid && (subof & acc) == 0u) || accepted;
       const uint32_t sv = (__ballot_sync(hmask, surv) >> hbase) & 0xffffu;
       const uint32_t ns = __popc(sv);
-      if (ns < s_cnt && (__ballot_sync(hmask, skipped_light) & hmask)) {
-        // fewer proofs than the full set held: the light candidates count
-        again = true;
-        en--;
-        if (hl >= 8) valid = false;
-        __syncwarp(hmask);
-        continue;
-      }
       if (accepted) {
         // the product in ascending literal order
         double ww = 1.0;
         const uint32_t* Lc = lists + row * PV_ROW;
         for (uint32_t q = 0; q < len; q++) ww = ww * v.prob[Lc[q] - 1];
         w = ww;
+      }
+      if (__ballot_sync(hmask, skipped_light) & hmask) {
+        // fewer proofs that outweigh the skipped candidates than the full set
+        // held (an accepted one may be as light as they are): these count
+        const bool heavy = surv && w > light * (1.0 + 5e-10);
+        if (__popc(__ballot_sync(hmask, heavy) & hmask) < (int)v.k) {
+          again = true;
+          en--;
+          if (hl >= 8) valid = false;
+          __syncwarp(hmask);
+          continue;
+        }
       }
       uint32_t keep = sv;
       if (ns > v.k) {
