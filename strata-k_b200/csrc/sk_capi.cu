@@ -857,12 +857,6 @@ void strata_rel_free(strata_ctx* ctx, strata_rel* rel) {
 
 // ---- operator surface ---------------------------------------------------------------
 
-// [a, a + an) and [b, b + bn) share a byte (null or empty spans share none).
-static bool spans_overlap(const void* a, uint64_t an, const void* b, uint64_t bn) {
-  const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-  return a && b && an && bn && x < y + bn && y < x + an;
-}
-
 strata_status strata_op_sort(strata_ctx* ctx, int key_bytes, int val_bytes, const void* d_keys_in,
                              const void* d_vals_in, void* d_keys_out, void* d_vals_out, uint64_t n,
                              int key_bits) {
@@ -878,10 +872,15 @@ strata_status strata_op_sort(strata_ctx* ctx, int key_bytes, int val_bytes, cons
   sk::reset_status(ctx);
   if (n == 0) return STRATA_OK;
   // The first pass reads the inputs and the last writes the outputs; buffers
-  // that overlap are copied first and sorted between output and scratch.
+  // that overlap, or whose inputs lie off their own type's alignment, are
+  // copied first and sorted between output and scratch.
   const uint64_t kb = n * (uint64_t)key_bytes, vb = n * (uint64_t)val_bytes;
-  const bool apart = !spans_overlap(d_keys_in, kb, d_keys_out, kb) && !spans_overlap(d_keys_in, kb, d_vals_out, vb) &&
-                     !spans_overlap(d_vals_in, vb, d_keys_out, kb) && !spans_overlap(d_vals_in, vb, d_vals_out, vb);
+  auto aligned = [](const void* p, int b) { return b == 0 || reinterpret_cast<uintptr_t>(p) % b == 0; };
+  const bool apart = aligned(d_keys_in, key_bytes) && aligned(d_vals_in, val_bytes) &&
+                     !sk::spans_overlap(d_keys_in, kb, d_keys_out, kb) &&
+                     !sk::spans_overlap(d_keys_in, kb, d_vals_out, vb) &&
+                     !sk::spans_overlap(d_vals_in, vb, d_keys_out, kb) &&
+                     !sk::spans_overlap(d_vals_in, vb, d_vals_out, vb);
   if (!apart) {
     SK_CUDA(cudaMemcpyAsync(d_keys_out, d_keys_in, kb, cudaMemcpyDeviceToDevice, ctx->stream));
     if (val_bytes) SK_CUDA(cudaMemcpyAsync(d_vals_out, d_vals_in, vb, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -967,8 +966,8 @@ strata_status strata_op_reduce(strata_ctx* ctx, int key_bytes, const void* d_key
   {
     // tiles write their output while other tiles still read their input
     const uint64_t kb = n * (uint64_t)key_bytes, wb = n * 8;
-    if (spans_overlap(d_keys, kb, d_out, kb) || spans_overlap(d_keys, kb, d_out_w, wb) ||
-        spans_overlap(d_w, wb, d_out, kb) || spans_overlap(d_w, wb, d_out_w, wb))
+    if (sk::spans_overlap(d_keys, kb, d_out, kb) || sk::spans_overlap(d_keys, kb, d_out_w, wb) ||
+        sk::spans_overlap(d_w, wb, d_out, kb) || sk::spans_overlap(d_w, wb, d_out_w, wb))
       return bad(ctx, "the output buffers overlap the input buffers");
   }
   if (set_device(ctx) != STRATA_OK) return STRATA_E_CUDA;
@@ -1008,7 +1007,7 @@ strata_status strata_op_merge_diff(strata_ctx* ctx, int key_bytes, const void* d
     const uint64_t out_b[4] = {fo * kb, fo * 8, n_cand * kb, n_cand * 8};
     for (int a = 0; a < 4; a++)
       for (int b = 0; b < 4; b++)
-        if (spans_overlap(in[a], in_b[a], out[b], out_b[b]))
+        if (sk::spans_overlap(in[a], in_b[a], out[b], out_b[b]))
           return bad(ctx, "the output buffers overlap the input buffers");
   }
   if (set_device(ctx) != STRATA_OK) return STRATA_E_CUDA;

@@ -103,6 +103,12 @@ namespace sk {
 
 // ---- allocation -------------------------------------------------------------
 
+// [a, a + an) and [b, b + bn) share a byte (null or empty spans share none).
+inline bool spans_overlap(const void* a, uint64_t an, const void* b, uint64_t bn) {
+  const auto x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return a && b && an && bn && x < y + bn && y < x + an;
+}
+
 // Size classes: 256 B granules below 1 MiB, then steps of 1/8 of the power of
 // two, so a block freed by one call fits the same request of the next call.
 inline uint64_t size_class(uint64_t bytes) {

@@ -312,11 +312,11 @@ uint64_t op_join(strata_ctx* ctx, const K* dk, const int64_t* dw, uint64_t nd, i
   if (T == 0) return 0;
   ctx->wshift = 0;
   DBuf<uint32_t> nbr(ctx, nr + 1);
-  // an output weight column over an input one: the inputs are read from copies
+  // an output column over an input weight column: the inputs are read from copies
   DBuf<int64_t> cd, cr;
   cd.ctx = cr.ctx = ctx;
   auto apart = [&](const int64_t* w, uint64_t n, DBuf<int64_t>& copy) -> const int64_t* {
-    if (!w || out_w >= w + n || w >= out_w + T) return w;
+    if (!spans_overlap(w, n * 8, out, T * sizeof(K)) && !spans_overlap(w, n * 8, out_w, T * 8)) return w;
     copy.reserve(n);
     SK_CUDA(cudaMemcpyAsync(copy.p, w, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
     return copy.p;
