@@ -687,6 +687,11 @@ inline uint64_t inst_bytes(const InstSpec& s) {
   return 3 * inst_vecs(s) * 16 + (uint64_t)s.rows * (2 + 4 + 16) + (s.e1 - s.e0) * 4 + 64;
 }
 
+// With the Δ summaries of rows wider than 32 words (inst_bytes has room for narrower ones).
+inline uint64_t wave_bytes(const InstSpec& s) {
+  return inst_bytes(s) + (uint64_t)s.rows * 8 * (ceil_div(inst_w4(s), 32) - 1);
+}
+
 struct BsResult {
   std::vector<uint64_t> counts, fps, totals;
   std::vector<uint32_t> rounds;
@@ -753,11 +758,11 @@ void bs_run(strata_ctx* ctx, const std::vector<InstSpec>& spec, const uint32_t* 
   {
     uint32_t a = 0;
     while (a < n_inst) {
-      uint64_t bytes = inst_bytes(spec[order[a]]);
-      if (bytes > budget) fail(STRATA_E_OOM, "one instance's bit matrices exceed the memory budget");
+      if (inst_bytes(spec[order[a]]) > budget) fail(STRATA_E_OOM, "one instance's bit matrices exceed the memory budget");
+      uint64_t bytes = wave_bytes(spec[order[a]]);
       uint32_t b = a + 1;
       if (mode != 1)
-        while (b < n_inst && bytes + inst_bytes(spec[order[b]]) <= budget) bytes += inst_bytes(spec[order[b]]), b++;
+        for (; b < n_inst && bytes + wave_bytes(spec[order[b]]) <= budget; b++) bytes += wave_bytes(spec[order[b]]);
       waves.push_back({a, b});
       a = b;
     }
@@ -1147,7 +1152,7 @@ void tc_bool_batch(strata_ctx* ctx, uint32_t n_inst, const uint32_t* nodes, cons
   check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
   check_cuda(cudaEventRecord(e0, ctx->stream), "cudaEventRecord");
   uint64_t need = 0;  // of all instances in one wave
-  for (auto& i : spec) need += inst_bytes(i);
+  for (auto& i : spec) need += wave_bytes(i);
   const uint64_t budget = bs_budget(ctx, need);  // the waves are sized from what this context can reuse
   release_all_cached(ctx);
   BsBuffers B(ctx);

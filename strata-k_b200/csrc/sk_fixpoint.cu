@@ -409,7 +409,10 @@ void fix_loop_queued(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, Den
 template <bool TROP, class W>
 void fix_loop_dense(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, DenseIdx<W>& X, uint64_t bound,
                     uint64_t cap, PhaseTimer& pt, Acct& a, uint64_t* rounds_out) {
-  if (dense_rounds_queued(X.lay, csr.m)) {
+  // the queued rounds hold a head per marks word: under a memory cap only where those fit
+  const uint64_t heads = X.words() + 1;
+  if (dense_rounds_queued(X.lay, csr.m) &&
+      (!ctx->cap || ctx->in_use + 3 * size_class(heads * 4) + size_class(heads * 8) + size_class(4096) <= ctx->cap)) {
     fix_loop_queued<TROP, W>(ctx, csr, js, X, cap, pt, a, rounds_out);
     return;
   }
@@ -504,6 +507,9 @@ void fix_loop_queued(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, Den
     if (TROP && cap && rounds > cap)
       fail(STRATA_E_NEG_CYCLE, "negative-weight cycle: tropical stratum diverges");
   }
+  // a head per word is more than the rounds one by one would hold: not while the result is built
+  for (auto* b : {&X.hidx, &X.hmask, &X.hseg}) b->release();
+  X.hpos.release();
   *rounds_out = rounds;
 }
 
