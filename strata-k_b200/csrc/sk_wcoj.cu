@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(TC_NT, 4)
       unsigned md = __ballot_sync(kFull, da && db);
       const uint32_t lim = (a.z >> 16) < (b.z >> 16) ? (a.z >> 16) : (b.z >> 16);  // 128-label blocks both can share
       while (md) {
-        constexpr int U = Q <= 2 ? 4 : 2;
+        constexpr int U = 4;
         uint4 rb[U][Q];
         uint32_t sa[U];
 #pragma unroll
@@ -937,8 +937,8 @@ uint64_t hub_count(strata_ctx* ctx, const K* keys, uint64_t m, int bits, uint64_
                    uint32_t x_lo, uint32_t x_hi) {
   DBuf<uint32_t> off(ctx, n_nodes + 1), nbr(ctx, m + 1);
   build_csr<K>(ctx, keys, m, bits, n_nodes, off.p, nbr.p);
-  DBuf<uint64_t> acc(ctx, 3);  // count, dense vertices, list-entry sum (profiling)
-  SK_CUDA(cudaMemsetAsync(acc.p, 0, 24, ctx->stream));
+  DBuf<uint64_t> acc(ctx, 2);  // count, dense vertices
+  SK_CUDA(cudaMemsetAsync(acc.p, 0, 16, ctx->stream));
   DBuf<uint4> meta(ctx, n_nodes);
   const int q = hub_q(n_nodes);
   k_hub_meta<<<blocks(n_nodes), 256, 0, ctx->stream>>>(off.p, nbr.p, n_nodes, (uint32_t)q * 4096u, meta.p,
@@ -963,21 +963,14 @@ uint64_t hub_count(strata_ctx* ctx, const K* keys, uint64_t m, int bits, uint64_
     const int kh = kprof_begin(ctx, K_TRI_COUNT);
     k_tri_edges<K, Q><<<g, TC_NT, 0, ctx->stream>>>(keys, m, bits, span, nbr.p, meta.p, rows.p, orig, x_lo, x_hi,
                                                     reinterpret_cast<unsigned long long*>(acc.p));
-    kprof_end(ctx, kh, 8 * m + 4 * (n_nodes + 1));  // as tri_from_sorted counts them; the list sum is added below
+    kprof_end(ctx, kh, m * sizeof(K) + n_nodes * 16 + nd * (uint64_t)Q * 512 + 4 * m);  // keys, meta, rows, lists once
     after_launch(ctx, "k_tri_edges");
   };
   if (q == 1) run(std::integral_constant<int, 1>{});
-  else if (q == 2) run(std::integral_constant<int, 2>{});
-  else run(std::integral_constant<int, 4>{});
-  if (ctx->profiling) {
-    k_tri_list_sum<K><<<(unsigned)std::min<uint64_t>(blocks(m), (uint64_t)ctx->num_sms * 8), 256, 0, ctx->stream>>>(
-        keys, m, bits, off.p, n_nodes, reinterpret_cast<unsigned long long*>(acc.p + 2));
-    after_launch(ctx, "k_tri_list_sum");
-  }
-  SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, acc.p, 24, cudaMemcpyDeviceToHost, ctx->stream));
+  else run(std::integral_constant<int, 2>{});
+  SK_CUDA(cudaMemcpyAsync(ctx->h_scalar, acc.p, 8, cudaMemcpyDeviceToHost, ctx->stream));
   sync_and_check(ctx);
   const uint64_t r = ctx->h_scalar[0];
-  if (ctx->profiling) kprof_add_last(ctx, K_TRI_COUNT, 4 * ctx->h_scalar[2]);
   kprof_collect(ctx);
   return r;
 }
