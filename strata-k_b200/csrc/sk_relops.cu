@@ -12,8 +12,8 @@
 //       and the concat + full re-sort of tc.rs:124-144 / trop.rs:177-213).
 //   build_csr, pack/unpack, distinct-id count, fingerprint : plumbing.
 //
-// Every kernel is single-pass over its inputs; cross-tile offsets come from
-// the bounded decoupled look-back in sk_prims.cuh.
+// Cross-tile offsets come from the bounded decoupled look-back in sk_prims.cuh
+// (merge_diff) or a scan of per-tile sums (the others).
 #include "sk_ops.cuh"
 #include "sk_prims.cuh"
 
@@ -28,68 +28,9 @@ constexpr int NT = 256;
 constexpr int EO_ITEMS = 16;
 constexpr uint32_t EO_TILE = NT * EO_ITEMS;
 
-template <class K>
-__global__ void __launch_bounds__(NT)
-    k_expand_offsets(const K* __restrict__ dkeys, uint64_t n, int jshift, uint64_t jmask,
-                     const uint32_t* __restrict__ off, uint64_t n_nodes, uint64_t* __restrict__ pos,
-                     uint64_t* states, uint32_t* counter, uint32_t* status, uint32_t gmax,
-                     unsigned long long* cand_total) {
-  __shared__ uint32_t s_tile;
-  __shared__ uint64_t s_warp[NT / 32 + 1];
-  __shared__ uint64_t s_excl;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t tile = claim_tile(counter, &s_tile);
-  const uint64_t wbase = (uint64_t)tile * EO_TILE + (uint64_t)warp * 32 * EO_ITEMS;
-  uint64_t vals[EO_ITEMS];
-  uint64_t carry = 0;
-  unsigned long long cands = 0;
-#pragma unroll
-  for (int j = 0; j < EO_ITEMS; j++) {
-    const uint64_t idx = wbase + j * 32 + lane;
-    uint64_t deg = 0;
-    if (idx < n) {
-      const uint64_t jv = ((uint64_t)dkeys[idx] >> jshift) & jmask;
-      if (jv < n_nodes) deg = (uint64_t)(off[jv + 1] - off[jv]);
-      cands += deg;
-      // grouped: a follower of a run (same join value, same gmax block) has no outputs
-      if (gmax && idx % gmax != 0 && (((uint64_t)dkeys[idx - 1] >> jshift) & jmask) == jv) deg = 0;
-    }
-    const uint64_t incl = warp_incl_sum(deg);
-    vals[j] = carry + incl - deg;
-    carry += __shfl_sync(kFull, incl, 31);
-  }
-  if (lane == 0) s_warp[warp] = carry;
-  if (cand_total) {
-    cands = warp_sum(cands);
-    if (lane == 0 && cands) atomicAdd(cand_total, cands);
-  }
-  __syncthreads();
-  if (warp == 0) {
-    uint64_t w = (lane < NT / 32) ? s_warp[lane] : 0;
-    uint64_t wi = warp_incl_sum(w);
-    if (lane < NT / 32) s_warp[lane] = wi - w;
-    const uint64_t agg = __shfl_sync(kFull, wi, NT / 32 - 1);
-    const uint64_t ex = warp_lookback(states, tile, agg, status);
-    if (lane == 0) {
-      s_excl = ex;
-      if (tile == gridDim.x - 1) pos[n] = ex + agg;
-    }
-  }
-  __syncthreads();
-  const uint64_t base = s_excl + s_warp[warp];
-#pragma unroll
-  for (int j = 0; j < EO_ITEMS; j++) {
-    const uint64_t idx = wbase + j * 32 + lane;
-    if (idx < n) pos[idx] = base + vals[j];
-  }
-}
-
-// ---------------------------------------------------------------------------
-// reduce-then-scan variant of the offsets (no waiting between tiles): one
-// kernel sums each tile's degrees, one block scans the tile sums, a third
-// kernel writes pos[].  Used where tiles carry little work, so that a
-// look-back chain would dominate.
-// ---------------------------------------------------------------------------
+// Reduce-then-scan, no waiting between tiles: one kernel sums each tile's
+// degrees, one block scans the tile sums, a third kernel writes pos[] (tiles
+// carry little work, so that a look-back chain would dominate).
 template <class K>
 __device__ __forceinline__ uint64_t group_degree(const K* dkeys, uint64_t idx, int jshift, uint64_t jmask,
                                                  const uint32_t* off, uint64_t n_nodes, uint32_t gmax,
@@ -469,7 +410,7 @@ __global__ void __launch_bounds__(NT)
 // ---------------------------------------------------------------------------
 // merge_diff: full ∪ cand and the delta over merge-path tiles
 // ---------------------------------------------------------------------------
-constexpr int MD_ITEMS = 6;
+constexpr int MD_ITEMS = 8;
 constexpr uint32_t MD_TILE = NT * MD_ITEMS;
 constexpr int MD_PER = MD_ITEMS + 1;  // merged positions a thread (a tile holds up to MD_TILE + 1)
 
@@ -498,30 +439,37 @@ __global__ void __launch_bounds__(NT) k_md_bounds(const K* __restrict__ A, uint6
   }
 }
 
-// Two passes over the same tiles, reduce-then-scan (no tile waits on
-// another): PASS 0 counts each tile's full-out rows and Δ' rows into
-// tile_full / tile_delta; after their exclusive scan, PASS 1 recomputes the tile
-// and writes its rows at the scanned offsets.  A thread finds its place on the
-// tile's merge path with one binary search and then merges MD_PER rows in
-// turn (a binary search for every row, 2 x 11 shared-memory reads each, bound
-// the earlier form); the rows leave through shared memory, coalesced.  Delta
-// round of 2 M rows against 3.2 M candidates of 16 bytes, one B200: both
-// passes 225 -> 140 us.
-template <class K, class W, bool TROP, bool WRITE_FULL, bool WRITE_DELTA, bool INPLACE, int PASS>
-__global__ void __launch_bounds__(NT)
+// One pass over the tiles, claimed in order: a tile merges, counts its full-out
+// and Δ' rows, publishes both counts and learns the rows before it by a bounded
+// look-back (a warp each, while the others stage the rows).  A thread finds its
+// place on the tile's merge path with one binary search and then merges MD_PER
+// rows in turn; the rows leave through shared memory, coalesced.  Bound by
+// the reads and writes and the look-back's latency.  Delta round of 2 M rows
+// against 3.2 M candidates of 16 bytes, one B200: a binary search per row in
+// a counting and a writing pass 225 us, this merge in two passes 140, in one
+// 125, with the rows in place and output rows by their 16-bit number (half the
+// shared memory, 40 registers, six blocks an SM instead of four) 105; tiles of
+// 1,024 / 1,536 / 2,048 / 2,560 / 3,584 rows 126 / 105 / 105 / 106 / 122, and
+// six merges of sparse paths over 200 k nodes 595 / 518 / 461 / 475 / 591.
+template <class K, class W, bool TROP, bool WRITE_FULL, bool WRITE_DELTA, bool INPLACE>
+__global__ void __launch_bounds__(NT, 6)
     k_merge_diff(const K* __restrict__ A, W* Aw, uint64_t na, const K* __restrict__ B,
                  const W* __restrict__ Bw, uint64_t nb, K* __restrict__ fout, W* __restrict__ fout_w,
                  K* __restrict__ dout, W* __restrict__ dout_w, const uint64_t* __restrict__ splits,
-                 uint64_t* tile_full, uint64_t* tile_delta, uint32_t* status) {
+                 uint64_t* full_states, uint64_t* delta_states, uint32_t* tile_counter, uint64_t* d_counts,
+                 uint32_t* status) {
   extern __shared__ __align__(16) unsigned char s_raw[];
   constexpr uint32_t CAP = MD_TILE + 2;
-  // keys of A, then of B; on the way out the full rows' keys, then Δ's (at
-  // most acnt + bcnt and bcnt of them); the weights beside them
+  // the rows of A, then of B; and per output row (the full ones, then Δ's: at
+  // most acnt + bcnt and bcnt of them) the row it is
   K* s_k = reinterpret_cast<K*>(s_raw);
-  W* s_w = reinterpret_cast<W*>(s_k + 2 * CAP);
+  W* s_w = reinterpret_cast<W*>(s_k + CAP);
+  uint16_t* s_row = reinterpret_cast<uint16_t*>(s_raw + CAP * (sizeof(K) + (TROP ? sizeof(W) : 0)));
   __shared__ uint32_t s_scan[NT / 32 + 1];
+  __shared__ uint64_t s_before[2];
+  __shared__ uint32_t s_tile;
   const int tid = threadIdx.x;
-  const uint32_t tile = blockIdx.x;
+  const uint32_t tile = claim_tile(tile_counter, &s_tile);
   const uint64_t i0 = splits[2 * tile], j0 = splits[2 * tile + 1];
   const uint64_t i1 = splits[2 * tile + 2], j1 = splits[2 * tile + 3];
   // Impossible for sorted unique inputs; checked so unsorted input cannot
@@ -553,31 +501,27 @@ __global__ void __launch_bounds__(NT)
     if (a[mid] <= b[d - mid - 1]) lo = mid + 1; else hi = mid;
   }
   uint32_t i = lo, j = d - lo;
-  K kk[MD_PER];
-  W ww[MD_PER];
+  uint32_t row[MD_PER];
   uint32_t fm = 0, dm = 0;  // positions that go to the full relation / to Δ'
 #pragma unroll
   for (int q = 0; q < MD_PER; q++) {
-    kk[q] = K(0);
-    ww[q] = W(0);
+    row[q] = 0;
     if (d + q >= n) continue;
     if (i < acnt && (j >= bcnt || a[i] <= b[j])) {
-      kk[q] = a[i];
+      row[q] = i;
       fm |= 1u << q;
       if constexpr (TROP) {
-        ww[q] = aw[i];
-        if (j < bcnt && b[j] == a[i] && bw[j] < ww[q]) ww[q] = bw[j];
+        if (j < bcnt && b[j] == a[i] && bw[j] < aw[i]) row[q] = acnt + j;  // the same key, the lower weight
       }
       i++;
     } else {
       const bool match = i > 0 && a[i - 1] == b[j];
-      kk[q] = b[j];
+      row[q] = acnt + j;
       bool changed = !match;
       if constexpr (TROP) {
-        ww[q] = bw[j];
         if (match && bw[j] < aw[i - 1]) {
           changed = true;
-          if constexpr (INPLACE && PASS == 1) Aw[i0 + i - 1] = bw[j];
+          if constexpr (INPLACE) Aw[i0 + i - 1] = bw[j];
         }
       }
       if (!match) fm |= 1u << q;
@@ -589,38 +533,32 @@ __global__ void __launch_bounds__(NT)
   uint32_t tot;
   const uint32_t ex = block_excl_sum<NT>((uint32_t)__popc(fm) | ((uint32_t)__popc(dm) << 16), s_scan, &tot);
   const uint32_t ftot = tot & 0xffffu, dtot = tot >> 16;
-  if constexpr (PASS == 0) {
-    if (tid == 0) {
-      tile_full[tile] = ftot;
-      tile_delta[tile] = dtot;
+  if (tid < 64) {
+    const int side = tid >> 5;  // 0: full rows, 1: Δ' rows
+    const uint32_t own = side ? dtot : ftot;
+    const uint64_t before = warp_lookback(side ? delta_states : full_states, tile, own, status);
+    if ((tid & 31) == 0) {
+      s_before[side] = before;
+      if (tile == gridDim.x - 1) d_counts[side] = before + own;
     }
-    return;
   }
-  // every thread has read its rows (the scan's barriers); stage and write
   uint32_t f = ex & 0xffffu, e = ftot + (ex >> 16);
 #pragma unroll
   for (int q = 0; q < MD_PER; q++) {
-    if (WRITE_FULL && ((fm >> q) & 1u)) {
-      s_k[f] = kk[q];
-      if constexpr (TROP) s_w[f] = ww[q];
-      f++;
-    }
-    if (WRITE_DELTA && ((dm >> q) & 1u)) {
-      s_k[e] = kk[q];
-      if constexpr (TROP) s_w[e] = ww[q];
-      e++;
-    }
+    if (WRITE_FULL && ((fm >> q) & 1u)) s_row[f++] = (uint16_t)row[q];
+    if (WRITE_DELTA && ((dm >> q) & 1u)) s_row[e++] = (uint16_t)row[q];
   }
   __syncthreads();
-  const uint64_t fex = tile_full[tile], dex = tile_delta[tile];
+  const uint64_t fex = s_before[0], dex = s_before[1];
   if constexpr (WRITE_FULL) {
     for (uint32_t k = tid; k < ftot; k += NT) {
       if (fex + k >= na + nb) {
         atomicOr(status, ST_BOUNDS);
         break;
       }
-      fout[fex + k] = s_k[k];
-      if constexpr (TROP) fout_w[fex + k] = s_w[k];
+      const uint32_t r = s_row[k];
+      fout[fex + k] = s_k[r];
+      if constexpr (TROP) fout_w[fex + k] = s_w[r];
     }
   }
   if constexpr (WRITE_DELTA) {
@@ -629,8 +567,9 @@ __global__ void __launch_bounds__(NT)
         atomicOr(status, ST_BOUNDS);
         break;
       }
-      dout[dex + k] = s_k[ftot + k];
-      if constexpr (TROP) dout_w[dex + k] = s_w[ftot + k];
+      const uint32_t r = s_row[ftot + k];
+      dout[dex + k] = s_k[r];
+      if constexpr (TROP) dout_w[dex + k] = s_w[r];
     }
   }
 }
@@ -1060,32 +999,24 @@ static void launch_merge(strata_ctx* ctx, const K* full, W* full_w, uint64_t nf,
     return;
   }
   const uint32_t tiles = (uint32_t)ceil_div(nf + nc, MD_TILE);
-  // per-tile counts (full, Δ'), each array tiles + 1 long for the scan total;
-  // then the merge-path splits
-  DBuf<uint64_t> buf(ctx, 2ull * (tiles + 1) + 2ull * (tiles + 1));
-  uint64_t* fcount = buf.p;
-  uint64_t* dcount = buf.p + tiles + 1;
-  uint64_t* splits = buf.p + 2ull * (tiles + 1);
+  // look-back states (full, Δ') and the tile counter, zeroed; then the merge-path splits
+  DBuf<uint64_t> buf(ctx, 2ull * tiles + 1 + 2ull * (tiles + 1));
+  uint64_t* states = buf.p;
+  uint64_t* splits = buf.p + 2ull * tiles + 1;
+  SK_CUDA(cudaMemsetAsync(states, 0, (2ull * tiles + 1) * 8, ctx->stream));
   k_md_bounds<K><<<(unsigned)ceil_div((uint64_t)tiles + 1, NT / 32), NT, 0, ctx->stream>>>(full, nf, cand, nc, tiles,
                                                                                            splits);
   after_launch(ctx, "k_md_bounds");
   constexpr uint32_t CAP = MD_TILE + 2;
-  const size_t smem = 2 * CAP * (sizeof(K) + (TROP ? sizeof(W) : 0));
-  auto count = k_merge_diff<K, W, TROP, WF, WD, IP, 0>;
-  auto write = k_merge_diff<K, W, TROP, WF, WD, IP, 1>;
-  SK_CUDA(cudaFuncSetAttribute(count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  SK_CUDA(cudaFuncSetAttribute(write, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const size_t smem = CAP * (sizeof(K) + (TROP ? sizeof(W) : 0) + 2 * sizeof(uint16_t));
+  auto kern = k_merge_diff<K, W, TROP, WF, WD, IP>;
+  SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int kh = kprof_begin(ctx, K_MERGE_DIFF);
-  count<<<tiles, NT, smem, ctx->stream>>>(full, full_w, nf, cand, cand_w, nc, fout, fout_w, dout, dout_w, splits,
-                                          fcount, dcount, ctx->d_status);
-  scan_tile_sums(ctx, buf.p, tiles, 2);
-  write<<<tiles, NT, smem, ctx->stream>>>(full, full_w, nf, cand, cand_w, nc, fout, fout_w, dout, dout_w, splits,
-                                          fcount, dcount, ctx->d_status);
+  kern<<<tiles, NT, smem, ctx->stream>>>(full, full_w, nf, cand, cand_w, nc, fout, fout_w, dout, dout_w, splits, states,
+                                         states + tiles, reinterpret_cast<uint32_t*>(states + 2ull * tiles), d_counts,
+                                         ctx->d_status);
   kprof_end(ctx, kh, (nf + nc) * (sizeof(K) + (TROP ? sizeof(W) : 0)));  // reads; writes added on read-back
   after_launch(ctx, "k_merge_diff");
-  ctx->launches += 1;  // the counting pass
-  SK_CUDA(cudaMemcpyAsync(d_counts, fcount + tiles, sizeof(uint64_t), cudaMemcpyDeviceToDevice, ctx->stream));
-  SK_CUDA(cudaMemcpyAsync(d_counts + 1, dcount + tiles, sizeof(uint64_t), cudaMemcpyDeviceToDevice, ctx->stream));
 }
 
 template <class K, class W, bool TROP>
