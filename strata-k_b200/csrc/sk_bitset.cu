@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(BS_NT, 3) k_bs_round(BsView v) {
         if (lane < 16) seen_of[lane] = 0u;
         __syncwarp();
         if (act) {
-          ent[ci] = make_uint4(y * W, sm, row, 0u);
+          ent[ci] = make_uint4(y, sm, row, 0u);
           atomicOr(&seen_of[row], sm);
         }
         __syncwarp();
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(BS_NT, 3) k_bs_round(BsView v) {
             if ((uint32_t)q < nq) {
               const uint4 en = ent[j + q];
               if ((en.y >> lane) & 1u) {
-                d[q] = dcol[en.x];
+                d[q] = dcol[(uint64_t)en.x * W];
                 mv.delta(true);
               }
             }
