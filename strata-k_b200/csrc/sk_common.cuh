@@ -149,11 +149,12 @@ inline uint64_t reusable_device_bytes(strata_ctx* ctx) {
 }
 
 // `share` of reusable_device_bytes; or `need` itself when the context holds
-// that much unused already (with a tenth to spare): the device query takes
-// 0.1 ms to several ms, and the need then takes nothing new from the device.
+// that much unused already, each buffer rounded up to its size class (at most
+// an eighth more): the device query takes 0.1 ms to several ms, and the need
+// then takes nothing new from the device.
 inline uint64_t device_budget(strata_ctx* ctx, double share, uint64_t need) {
   const uint64_t held = held_device_bytes(ctx);
-  if (need <= held - held / 10) return need;
+  if (need + need / 8 <= held) return need;
   return (uint64_t)((double)reusable_device_bytes(ctx) * share);
 }
 
