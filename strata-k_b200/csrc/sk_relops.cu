@@ -1127,9 +1127,11 @@ FixScan fix_scan(strata_ctx* ctx, const uint32_t* a, const int64_t* aw, const ui
                  const uint32_t* x, const uint32_t* y, const int64_t* w, const uint8_t* winf, uint64_t m) {
   // Ids below 2^20 in up to 2^20 rows are counted in the same pass (a 128 KB
   // bitmap, one wait); otherwise the bitmap's size needs the maxima first,
-  // and hub ids are better marked in shared memory (count_distinct_ids).
+  // and hub ids are better marked in shared memory (count_distinct_ids).  So
+  // too under a memory cap that has no room for the 128 KB.
   constexpr uint64_t kIds = 1ull << 20;
-  const uint64_t limit = na + m <= kIds ? kIds : 0;
+  const bool room = !ctx->cap || ctx->in_use + size_class((6 + kIds / 64) * 8) <= ctx->cap;
+  const uint64_t limit = na + m <= kIds && room ? kIds : 0;
   DBuf<uint64_t> buf(ctx, 6 + limit / 64);
   SK_CUDA(cudaMemsetAsync(buf.p, 0, (6 + limit / 64) * 8, ctx->stream));
   auto* out = reinterpret_cast<unsigned long long*>(buf.p);
@@ -1145,7 +1147,10 @@ FixScan fix_scan(strata_ctx* ctx, const uint32_t* a, const int64_t* aw, const ui
   read_u64(ctx, buf.p, h, 6);
   FixScan r{(uint32_t)h[0], (uint32_t)h[1], (uint32_t)h[2], h[3], h[4], h[5]};
   const uint64_t ids = std::max(h[0], std::max(h[1], h[2])) + 1;
-  if (ids > limit) r.universe = count_distinct_ids(ctx, a, na, x, m, y, m, ids);
+  if (ids > limit) {
+    buf.release();
+    r.universe = count_distinct_ids(ctx, a, na, x, m, y, m, ids);
+  }
   return r;
 }
 
