@@ -709,8 +709,10 @@ strata_circuits* circuits_upload(strata_ctx* ctx, const std::vector<const std::v
     c->a = dev_upload(ctx, A, qnode[nq]);
     c->b = dev_upload(ctx, B, qnode[nq]);
     c->ch = dev_upload(ctx, CH.get(), total_ch);
-    c->qnode = dev_upload(ctx, qnode);
-    c->qchild = dev_upload(ctx, qch);
+    std::vector<uint32_t> firsts(qnode.begin(), qnode.end());  // below 2^32, checked above
+    firsts.insert(firsts.end(), qch.begin(), qch.end());
+    c->qnode = dev_upload(ctx, firsts);
+    c->qchild = c->qnode + nq + 1;
     c->root = dev_upload(ctx, root);
     c->qlevel = dev_upload(ctx, qlevel);
     c->lvl = dev_upload(ctx, lvl);
@@ -799,7 +801,7 @@ strata_circuits* circuit_parts_upload(strata_ctx* ctx, uint32_t n_parts, Circuit
 
 void circuits_free(strata_ctx* ctx, strata_circuits* c) {
   if (!c) return;
-  for (void* p : {(void*)c->kind, (void*)c->a, (void*)c->b, (void*)c->ch, (void*)c->qnode, (void*)c->qchild, (void*)c->root,
+  for (void* p : {(void*)c->kind, (void*)c->a, (void*)c->b, (void*)c->ch, (void*)c->qnode, (void*)c->root,
                   (void*)c->qlevel, (void*)c->lvl, (void*)c->val, (void*)c->val_lo, (void*)c->adj})
     if (p) dev_free(ctx, p);
   delete c;

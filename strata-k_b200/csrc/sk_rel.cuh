@@ -31,8 +31,8 @@ struct strata_circuits {
   uint32_t* a = nullptr;        // leaf index, or first child (index into `ch`)
   uint32_t* b = nullptr;        // child count
   uint32_t* ch = nullptr;       // children (global node indices)
-  uint64_t* qnode = nullptr;    // first node of query q (n_queries + 1)
-  uint64_t* qchild = nullptr;   // first entry of `ch` of query q (n_queries + 1)
+  uint32_t* qnode = nullptr;    // first node of query q (n_queries + 1)
+  uint32_t* qchild = nullptr;   // first entry of `ch` of query q (n_queries + 1); behind qnode in its block
   uint32_t* root = nullptr;     // root node of query q (global index)
   uint64_t* qlevel = nullptr;   // first level of query q in `lvl` (n_queries + 1)
   uint32_t* lvl = nullptr;      // level boundaries: node offsets relative to qnode[q]

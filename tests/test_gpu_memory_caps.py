@@ -28,3 +28,27 @@ def test_small_tropical_calls(engine, n, m, cap):
         assert got.stats["universe"] == len(np.unique(np.concatenate([edges[0], edges[1], [0, 3]])))
         if n == 20:
             assert _same(small.shortest_paths_trop(edges), engine.shortest_paths_trop(edges))
+
+
+def test_compiled_circuits():
+    # per node a kind, two words and three floats; per child and level a word;
+    # per query two first entries and a root of 4 bytes and a 64-bit level start
+    import torch
+    from strata_b200 import Engine
+    nq = 1023
+
+    def cls(b):  # size classes of the context's blocks
+        step = 256 if b <= 1 << 20 else 1 << (b.bit_length() - 4)
+        return -(-b // step) * step
+    with Engine(0) as eng:
+        one = eng.compile_circuits([[[1, 2], [2, 3]]], 3)
+        nodes, levels = one.shape()
+        assert nodes == 19  # three decisions of five nodes, four constants
+        one.free()
+        held = eng.mem()[0]
+        circ = eng.compile_circuits([[[1, 2], [2, 3]]] * nq, 3)
+        assert eng.mem()[0] - held <= (cls(nq * nodes) + 5 * cls(4 * nq * nodes) + cls(4 * nq * 18) + cls(8 * (nq + 1)) +
+                                       cls(4 * nq) + cls(8 * (nq + 1)) + cls(4 * nq * (levels + 1)))
+        p = torch.full((3,), 0.5, device="cuda")
+        assert torch.equal(circ.forward(p), torch.full((nq,), 0.375, device="cuda"))
+        circ.free()
