@@ -231,6 +231,19 @@ inline void dev_free(strata_ctx* ctx, void* p) {
   ctx->sizes.erase(it);
 }
 
+// Runs f; false where its device memory could not be had (f's buffers are
+// given back by then), so that the caller can take a form that needs less.
+template <class F>
+bool with_memory(F&& f) {
+  try {
+    f();
+  } catch (const SkError& e) {
+    if (e.code != STRATA_E_OOM) throw;
+    return false;
+  }
+  return true;
+}
+
 // Owning device buffer (RAII, stream-ordered free).
 template <class T>
 struct DBuf {

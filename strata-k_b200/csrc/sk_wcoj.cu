@@ -881,7 +881,9 @@ inline uint32_t hub_step(uint64_t n, uint64_t n_nodes) {
 
 inline int hub_q(uint64_t n_nodes) { return n_nodes <= 4096 ? 1 : 2; }
 
-// The plan applies: default probe, sizes in range, and its memory within the context's cap.
+// The plan applies: default probe, sizes in range, and its memory within the
+// context's cap.  Without a cap the device may still be too full for it: then
+// its first allocation to fail ends it and the edges are probed instead.
 inline bool hub_fits(strata_ctx* ctx, uint64_t n, uint64_t n_min, uint64_t n_nodes, size_t key_bytes) {
   if (ctx->tune_tri_probe != 0 || n < n_min || n_nodes > kHubMaxNodes) return false;
   return !ctx->cap || ctx->in_use + n * (3 * key_bytes + 4) + hub_bytes(n, n_nodes, hub_q(n_nodes)) <= ctx->cap;
@@ -983,11 +985,14 @@ uint64_t pattern_impl(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uin
   DBuf<K> keys(ctx, n + 1), uniq;
   uniq.ctx = ctx;
   if (hub_fits(ctx, n, kHubMinDirected, n_nodes, sizeof(K))) {
-    DBuf<uint32_t> deg;
-    deg.ctx = ctx;
-    const HubSample hs = hub_sample(ctx, x, y, n, n_nodes, false, deg);
-    const double cand = (double)hs.candidates * hs.step * hs.step;
-    if (cand >= (double)kHubMinCandidates * (double)n && hs.covered(n_nodes)) {
+    bool counted = false;
+    uint64_t r = 0;
+    const bool had = with_memory([&] {
+      DBuf<uint32_t> deg;
+      deg.ctx = ctx;
+      const HubSample hs = hub_sample(ctx, x, y, n, n_nodes, false, deg);
+      const double cand = (double)hs.candidates * hs.step * hs.step;
+      if (cand < (double)kHubMinCandidates * (double)n || !hs.covered(n_nodes)) return;
       const bool whole = u_lo == 0 && u_hi == n_nodes;
       DBuf<uint32_t> label, order;
       label.ctx = order.ctx = ctx;
@@ -995,8 +1000,11 @@ uint64_t pattern_impl(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uin
       k_hub_pack<K><<<blocks(n), 256, 0, ctx->stream>>>(x, y, n, label.p, b, 0, keys.p);
       after_launch(ctx, "k_hub_pack");
       const uint64_t m = sort_unique<K>(ctx, keys, n, 2 * b, uniq);
-      return hub_count<K>(ctx, uniq.p, m, b, n_nodes, whole ? nullptr : order.p, (uint32_t)u_lo, (uint32_t)u_hi);
-    }
+      r = hub_count<K>(ctx, uniq.p, m, b, n_nodes, whole ? nullptr : order.p, (uint32_t)u_lo, (uint32_t)u_hi);
+      counted = true;
+    });
+    if (had && counted) return r;
+    uniq.release();
   }
   pack_pairs<K, int32_t, false>(ctx, x, y, nullptr, nullptr, n, b, keys.p, nullptr);
   const uint64_t m = sort_unique<K>(ctx, keys, n, 2 * b, uniq);
@@ -1042,17 +1050,22 @@ uint64_t tri_undirected_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t*
   if (hub_fits(ctx, n, kHubMinUndirected, n_nodes, sizeof(K))) {
     // Any total order of the vertices counts each triangle of the simple
     // graph once; the labels are one, so a single sort orients and dedups.
-    DBuf<uint32_t> deg, label;
-    deg.ctx = label.ctx = ctx;
-    const HubSample hs = hub_sample(ctx, a, b, n, n_nodes, true, deg);
-    hub_labels(ctx, deg.p, n_nodes, label, nullptr);
-    DBuf<K> keys(ctx, n + 1);
-    k_hub_pack<K><<<blocks(n), 256, 0, ctx->stream>>>(a, b, n, label.p, bits, 1, keys.p);
-    after_launch(ctx, "k_hub_pack");
-    const uint64_t m = drop_loops<K>(ctx, ori, sort_unique<K>(ctx, keys, n, 2 * bits, ori), bits);
-    if (m == 0) return 0;
-    if (!hs.covered(n_nodes)) return tri_from_sorted<K>(ctx, ori.p, m, bits, n_nodes);
-    return hub_count<K>(ctx, ori.p, m, bits, n_nodes, nullptr, 0, 0);
+    uint64_t r = 0;
+    const bool had = with_memory([&] {
+      DBuf<uint32_t> deg, label;
+      deg.ctx = label.ctx = ctx;
+      const HubSample hs = hub_sample(ctx, a, b, n, n_nodes, true, deg);
+      hub_labels(ctx, deg.p, n_nodes, label, nullptr);
+      DBuf<K> keys(ctx, n + 1);
+      k_hub_pack<K><<<blocks(n), 256, 0, ctx->stream>>>(a, b, n, label.p, bits, 1, keys.p);
+      after_launch(ctx, "k_hub_pack");
+      const uint64_t m = drop_loops<K>(ctx, ori, sort_unique<K>(ctx, keys, n, 2 * bits, ori), bits);
+      if (m == 0) return;
+      r = hs.covered(n_nodes) ? hub_count<K>(ctx, ori.p, m, bits, n_nodes, nullptr, 0, 0)
+                              : tri_from_sorted<K>(ctx, ori.p, m, bits, n_nodes);
+    });
+    if (had) return r;
+    ori.release();
   }
   const uint64_t m = oriented_edges<K>(ctx, a, b, n, bits, n_nodes, true, ori);
   if (m == 0) return 0;
