@@ -867,6 +867,13 @@ uint64_t tri_from_sorted(strata_ctx* ctx, const K* keys, uint64_t m, int bits, u
 // eight times the mean in-degree.
 constexpr uint64_t kHubMinDirected = 1ull << 18, kHubMinUndirected = 1ull << 15;
 constexpr uint64_t kHubMinCandidates = 48;
+// Undirected graphs without skew take the labels for the sort they save (one
+// of the edges instead of two) while the sort of the ids costs less: up to
+// eight ids an edge.  Uniform graphs of 600 k edges over as many vertices, us a
+// call, labels / none: 0.6 M ids 1,280 / 1,363, 4.8 M 4,167 / 4,201, 9.6 M
+// 7,469 / 7,414; 4 M edges, 32 M ids 26,309 / 26,041, 100 M 73,298 / 71,894.
+// With skew the rows pay at any width (40 k edges over 10^8 ids 4,771 / 65,681).
+constexpr uint64_t kHubSortIds = 8;
 constexpr uint64_t kHubMaxNodes = 1ull << 27;  // above, the per-vertex tables outgrow their use
 
 // Device bytes the plan needs beside the edge keys (an upper bound on the rows).
@@ -1050,11 +1057,14 @@ uint64_t tri_undirected_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t*
   if (hub_fits(ctx, n, kHubMinUndirected, n_nodes, sizeof(K))) {
     // Any total order of the vertices counts each triangle of the simple
     // graph once; the labels are one, so a single sort orients and dedups.
+    bool counted = false;
     uint64_t r = 0;
     const bool had = with_memory([&] {
       DBuf<uint32_t> deg, label;
       deg.ctx = label.ctx = ctx;
       const HubSample hs = hub_sample(ctx, a, b, n, n_nodes, true, deg);
+      if (!hs.covered(n_nodes) && n_nodes > kHubSortIds * n) return;
+      counted = true;
       hub_labels(ctx, deg.p, n_nodes, label, nullptr);
       DBuf<K> keys(ctx, n + 1);
       k_hub_pack<K><<<blocks(n), 256, 0, ctx->stream>>>(a, b, n, label.p, bits, 1, keys.p);
@@ -1064,7 +1074,7 @@ uint64_t tri_undirected_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t*
       r = hs.covered(n_nodes) ? hub_count<K>(ctx, ori.p, m, bits, n_nodes, nullptr, 0, 0)
                               : tri_from_sorted<K>(ctx, ori.p, m, bits, n_nodes);
     });
-    if (had) return r;
+    if (had && counted) return r;
     ori.release();
   }
   const uint64_t m = oriented_edges<K>(ctx, a, b, n, bits, n_nodes, true, ori);
