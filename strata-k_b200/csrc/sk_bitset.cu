@@ -683,11 +683,13 @@ struct InstSpec {
 
 inline uint64_t inst_w4(const InstSpec& s) { return std::max<uint64_t>(1, ceil_div(s.cols, 128)); }
 inline uint64_t inst_vecs(const InstSpec& s) { return (uint64_t)s.rows * inst_w4(s); }
+// Matrices, row and edge arrays: what the size rules (8 GB, one instance per
+// budget) go by.
 inline uint64_t inst_bytes(const InstSpec& s) {
   return 3 * inst_vecs(s) * 16 + (uint64_t)s.rows * (2 + 4 + 16) + (s.e1 - s.e0) * 4 + 64;
 }
-
-// With the Δ summaries of rows wider than 32 words (inst_bytes has room for narrower ones).
+// What an instance takes: also the Δ summaries of rows wider than 32 words
+// (inst_bytes has room for narrower ones).
 inline uint64_t wave_bytes(const InstSpec& s) {
   return inst_bytes(s) + (uint64_t)s.rows * 8 * (ceil_div(inst_w4(s), 32) - 1);
 }
@@ -1196,8 +1198,9 @@ void tc_bool_batch(strata_ctx* ctx, uint32_t n_inst, const uint32_t* nodes, cons
 // do not fit (the caller falls back to another plan).
 bool tc_bool_bitset_fits(strata_ctx* ctx, uint64_t n_src, uint64_t n_dst, uint64_t m) {
   const InstSpec s{(uint32_t)n_src, (uint32_t)n_dst, 0, m};
-  const uint64_t need = inst_bytes(s);
-  return n_src < (1ull << 32) && n_dst < (1ull << 32) && need <= (8ull << 30) && need <= bs_budget(ctx, need);
+  // asked for by name (plan 3), the rounds are tried up to the size rule itself
+  const uint64_t need = ctx->plan == 3 ? inst_bytes(s) : wave_bytes(s);
+  return n_src < (1ull << 32) && n_dst < (1ull << 32) && inst_bytes(s) <= (8ull << 30) && need <= bs_budget(ctx, need);
 }
 
 // ---- one small closure in one block --------------------------------------------

@@ -685,16 +685,27 @@ strata_rel* fix_tc_bool(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats* st
     const bool fits = tc_bool_bitset_fits(ctx, L.n_nodes_src, L.n_nodes, e.n);
     if (ctx->plan == 3 && !fits) fail(STRATA_E_UNSUPPORTED, "the bit-row plan needs its bit matrices within 8 GB");
     if (fits) {
-      if (!L.wide_key) return run_tc_bitset<uint32_t>(ctx, e, L, st, et, l_start);
-      return run_tc_bitset<uint64_t>(ctx, e, L, st, et, l_start);
+      auto bits = [&] {
+        return L.wide_key ? run_tc_bitset<uint64_t>(ctx, e, L, st, et, l_start)
+                          : run_tc_bitset<uint32_t>(ctx, e, L, st, et, l_start);
+      };
+      if (ctx->plan == 3) return bits();
+      // buffers rounded up and the relation itself come on top of what was
+      // checked: where they do not fit, a tuple plan may
+      strata_rel* rel = nullptr;
+      if (with_memory([&] { rel = bits(); })) return rel;
     }
   }
+  auto tuples = [&](bool dense) {
+    return L.wide_key ? run_tc_shape<uint64_t, int32_t, false>(ctx, e, L.b0, L.b1, L.bsrc, L.n_nodes, 0, 0, st, et,
+                                                               l_start, L.n_nodes_src, dense)
+                      : run_tc_shape<uint32_t, int32_t, false>(ctx, e, L.b0, L.b1, L.bsrc, L.n_nodes, 0, 0, st, et,
+                                                               l_start, L.n_nodes_src, dense);
+  };
   const bool dense = want_dense(ctx, false, true, L.n_nodes_src, L.n_nodes);
-  if (!L.wide_key)
-    return run_tc_shape<uint32_t, int32_t, false>(ctx, e, L.b0, L.b1, L.bsrc, L.n_nodes, 0, 0, st, et, l_start,
-                                                  L.n_nodes_src, dense);
-  return run_tc_shape<uint64_t, int32_t, false>(ctx, e, L.b0, L.b1, L.bsrc, L.n_nodes, 0, 0, st, et, l_start,
-                                                L.n_nodes_src, dense);
+  if (!dense || ctx->plan == 2) return tuples(dense);
+  strata_rel* rel = nullptr;
+  return with_memory([&] { rel = tuples(true); }) ? rel : tuples(false);
 }
 
 strata_rel* fix_trop_paths(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats* st) {

@@ -52,3 +52,19 @@ def test_compiled_circuits():
         p = torch.full((3,), 0.5, device="cuda")
         assert torch.equal(circ.forward(p), torch.full((nq,), 0.375, device="cuda"))
         circ.free()
+
+
+def test_closure_gives_way_to_the_tuple_plan(engine):
+    # 4,500 disjoint edges of 9,000 nodes: bit rows of 31 MB for a relation of 36 KB
+    from strata_b200 import Engine
+    n = 9000
+    s = np.arange(0, n, 2, dtype=np.uint32)
+    want = engine.transitive_closure_bool((s, s + 1))
+    assert np.array_equal(want.src, s) and np.array_equal(want.dst, s + 1)
+    mats = 3 * (n - 1) * -(-n // 128) * 16
+    for cap in [mats // 2] + [int(mats * f) for f in (1.005, 1.01, 1.05, 1.1, 1.15, 1.3)]:
+        with Engine(0, mem_cap=cap) as small:
+            small.set_plan(1)
+            assert _same(small.transitive_closure_bool((s, s + 1)), want)
+        with Engine(0, mem_cap=cap) as small:
+            assert _same(small.transitive_closure_bool((s, s + 1)), want), cap
