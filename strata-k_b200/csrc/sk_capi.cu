@@ -896,7 +896,7 @@ strata_status strata_op_sort(strata_ctx* ctx, int key_bytes, int val_bytes, cons
     K* kalt = ka.p;
     V* vp = static_cast<V*>(d_vals_out);
     V* valt = va.p;
-    sk::radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, val_bytes != 0, n, key_bits, true,
+    sk::radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, val_bytes != 0, n, key_bits, sk::kSortLook,
                          apart ? static_cast<const K*>(d_keys_in) : nullptr,
                          apart && val_bytes ? static_cast<const V*>(d_vals_in) : nullptr);
     if (kp != d_keys_out) {

@@ -138,7 +138,7 @@ uint64_t derive(strata_ctx* ctx, const K* dk, const W* dw, uint64_t nd, const Cs
   K* ka = s.ck2.p;
   V* vp = reinterpret_cast<V*>(s.cw.p);
   V* va = reinterpret_cast<V*>(s.cw2.p);
-  radix_sort<K, V>(ctx, &kp, &ka, &vp, &va, TROP, T, key_bits, false);
+  radix_sort<K, V>(ctx, &kp, &ka, &vp, &va, TROP, T, key_bits, kSortAll);
   pt.end(t);
   a.sort_b += 2 * T * (ksz + wsz) * (uint64_t)((key_bits + 7) / 8);
   a.sort_l += (uint32_t)(ctx->launches - l1);
@@ -200,10 +200,12 @@ void fix_loop(strata_ctx* ctx, Rel<K, W>& full, Rel<K, W>& delta, const Csr<W>& 
   *rounds_out = rounds;
 }
 
-// The sorted unique relation (Trop: least weight per key) of columns (c0, c1).
+// The sorted unique relation (Trop: least weight per key) of columns (c0, c1),
+// whose ids differ in the bits v0, v1 (the input scan found them): ids that
+// share their high bits, or one source for all rows, take fewer sort passes.
 template <class K, class W, bool TROP>
 void normalize(strata_ctx* ctx, const uint32_t* c0, const uint32_t* c1, const int64_t* w, const uint8_t* inf,
-               uint64_t n, int shift, int key_bits, Rel<K, W>& out) {
+               uint64_t n, int shift, uint32_t v0, uint32_t v1, int key_bits, Rel<K, W>& out) {
   using V = typename SortVal<W>::type;
   out.reserve(n + 1, TROP);
   DBuf<uint64_t> cnt(ctx, 1);
@@ -220,8 +222,8 @@ void normalize(strata_ctx* ctx, const uint32_t* c0, const uint32_t* c1, const in
     K* kalt = ka.p;
     V* vp = reinterpret_cast<V*>(kw.p);
     V* valt = reinterpret_cast<V*>(wa.p);
-    // packed ids: every digit of the key's bits varies, so no look at the keys
-    radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, TROP, n, key_bits, false);
+    const uint64_t vary = (c0 ? (uint64_t)v0 << shift : 0ull) | v1;
+    radix_sort<K, V>(ctx, &kp, &kalt, &vp, &valt, TROP, n, key_bits, vary);
     reduce_runs<K, W, TROP>(ctx, kp, reinterpret_cast<W*>(vp), n, out.k.p, TROP ? out.w.p : nullptr, cnt.p);
   }
   read_u64(ctx, cnt.p, &out.n, 1);
@@ -236,7 +238,8 @@ void build_edge_csr(strata_ctx* ctx, const EdgeCols& e, int join_col, int jbits,
   const uint32_t* c1 = join_col == 0 ? e.dst : e.src;
   Rel<KC, W> r;
   r.k.ctx = r.w.ctx = ctx;
-  normalize<KC, W, TROP>(ctx, c0, c1, e.w, e.inf, e.n, vbits, jbits + vbits, r);
+  normalize<KC, W, TROP>(ctx, c0, c1, e.w, e.inf, e.n, vbits, join_col == 0 ? e.vsrc : e.vdst,
+                         join_col == 0 ? e.vdst : e.vsrc, jbits + vbits, r);
   csr.off.ctx = csr.nbr.ctx = csr.w.ctx = ctx;
   csr.off.reserve(n_nodes + 1);
   csr.nbr.reserve(r.n + 1);
@@ -536,7 +539,7 @@ strata_rel* run_tc_shape(strata_ctx* ctx, const EdgeCols& e, int b0, int b1, int
   // path0 = normalize(edge): every edge is derived by the base rule.
   Rel<K, W> full, delta;
   full.k.ctx = full.w.ctx = delta.k.ctx = delta.w.ctx = ctx;
-  normalize<K, W, TROP>(ctx, e.src, e.dst, e.w, e.inf, e.n, b1, key_bits, full);
+  normalize<K, W, TROP>(ctx, e.src, e.dst, e.w, e.inf, e.n, b1, e.vsrc, e.vdst, key_bits, full);
   // In-CSR: Y -> X (join on the edge's dst), key bits b1 + bsrc.
   Csr<W> csr;
   if (b1 + bsrc <= 32)
@@ -585,15 +588,7 @@ struct Layout {
   bool wide_key;
 };
 
-// The largest ids of the edge columns alone (a Bool closure needs no more).
-FixScan edge_maxima(strata_ctx* ctx, const EdgeCols& e) {
-  FixScan r{};
-  max_u32_pair(ctx, e.src, e.dst, e.n, &r.max_x, &r.max_y);
-  return r;
-}
-
-Layout tc_layout(const FixScan& fs) {
-  const uint32_t ms = fs.max_x, md = fs.max_y;
+Layout tc_layout(uint32_t ms, uint32_t md) {
   Layout L;
   L.b0 = std::max(1, bits_for(ms));
   L.b1 = std::max(1, bits_for(md));
@@ -667,7 +662,8 @@ strata_rel* run_tc_bitset(strata_ctx* ctx, const EdgeCols& e, const Layout& L, s
 
 }  // namespace
 
-strata_rel* fix_tc_bool(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats* st) {
+strata_rel* fix_tc_bool(strata_ctx* ctx, const EdgeCols& cols, strata_fix_stats* st) {
+  EdgeCols e = cols;
   if (st) std::memset(st, 0, sizeof(*st));
   reset_status(ctx);
   const uint64_t l_start = ctx->launches;
@@ -677,7 +673,10 @@ strata_rel* fix_tc_bool(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats* st
     strata_rel* rel = new strata_rel();
     return rel;
   }
-  const Layout L = tc_layout(edge_maxima(ctx, e));
+  const ColScan cs = col_scan(ctx, e.src, e.dst, e.n);  // a Bool closure needs no more of its inputs
+  e.vsrc = cs.a.vary();
+  e.vdst = cs.b.vary();
+  const Layout L = tc_layout(cs.a.max, cs.b.max);
   if (ctx->plan == 3 || ctx->plan == 0) {
     // profiling runs keep the rounds as kernels of their own
     if (!ctx->profiling && tc_bool_small_fits(ctx, L.n_nodes_src, L.n_nodes, e.n))
@@ -708,7 +707,8 @@ strata_rel* fix_tc_bool(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats* st
   return with_memory([&] { rel = tuples(true); }) ? rel : tuples(false);
 }
 
-strata_rel* fix_trop_paths(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats* st) {
+strata_rel* fix_trop_paths(strata_ctx* ctx, const EdgeCols& cols, strata_fix_stats* st) {
+  EdgeCols e = cols;
   if (st) std::memset(st, 0, sizeof(*st));
   reset_status(ctx);
   const uint64_t l_start = ctx->launches;
@@ -721,7 +721,9 @@ strata_rel* fix_trop_paths(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats*
     return rel;
   }
   const FixScan fs = fix_scan(ctx, nullptr, nullptr, nullptr, 0, e.src, e.dst, e.w, e.inf, e.n);
-  const Layout L = tc_layout(fs);
+  e.vsrc = fs.x.vary();
+  e.vdst = fs.y.vary();
+  const Layout L = tc_layout(fs.x.max, fs.y.max);
   const uint64_t universe = fs.universe;
   const uint64_t cap = universe + 2;
   const bool narrow = !ctx->force_wide && narrow_ok(universe, fs.mag_w, 0);
@@ -746,7 +748,7 @@ strata_rel* fix_trop_paths(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats*
 namespace {
 
 template <class K, class W>
-strata_rel* run_mssp(strata_ctx* ctx, const uint32_t* sources, const int64_t* src_w,
+strata_rel* run_mssp(strata_ctx* ctx, const uint32_t* sources, uint32_t vsources, const int64_t* src_w,
                      const uint8_t* src_inf, uint64_t ns, const EdgeCols& e, int b0, int b1,
                      int besrc, uint64_t n_nodes_src, uint64_t universe, uint64_t cap,
                      strata_fix_stats* st, EventTimer& et, uint64_t l_start, uint64_t n0, uint64_t n1,
@@ -758,7 +760,7 @@ strata_rel* run_mssp(strata_ctx* ctx, const uint32_t* sources, const int64_t* sr
   // src as a unary Trop relation keyed by S (min over duplicate facts).
   Rel<K, W> srcu;
   srcu.k.ctx = srcu.w.ctx = ctx;
-  normalize<K, W, true>(ctx, nullptr, sources, src_w, src_inf, ns, 0, b0, srcu);
+  normalize<K, W, true>(ctx, nullptr, sources, src_w, src_inf, ns, 0, 0, vsources, b0, srcu);
   // Out-CSR: Y -> Z with weights (join on the edge's src), key bits besrc + b1.
   Csr<W> csr;
   if (besrc + b1 <= 32)
@@ -821,7 +823,8 @@ strata_rel* run_mssp(strata_ctx* ctx, const uint32_t* sources, const int64_t* sr
 }  // namespace
 
 strata_rel* fix_mssp(strata_ctx* ctx, const uint32_t* sources, const int64_t* src_w,
-                     const uint8_t* src_inf, uint64_t ns, const EdgeCols& e, strata_fix_stats* st) {
+                     const uint8_t* src_inf, uint64_t ns, const EdgeCols& cols, strata_fix_stats* st) {
+  EdgeCols e = cols;
   if (st) std::memset(st, 0, sizeof(*st));
   reset_status(ctx);
   const uint64_t l_start = ctx->launches;
@@ -837,7 +840,9 @@ strata_rel* fix_mssp(strata_ctx* ctx, const uint32_t* sources, const int64_t* sr
     return rel;
   }
   const FixScan fs = fix_scan(ctx, sources, src_w, src_inf, ns, e.src, e.dst, e.w, e.inf, e.n);
-  const uint32_t mS = fs.max_a, mes = fs.max_x, med = fs.max_y;
+  const uint32_t mS = fs.a.max, mes = fs.x.max, med = fs.y.max;
+  e.vsrc = fs.x.vary();
+  e.vdst = fs.y.vary();
   const int b0 = std::max(1, bits_for(mS));
   const int b1 = std::max(1, bits_for(med));
   const int besrc = std::max(1, bits_for(mes));
@@ -850,15 +855,15 @@ strata_rel* fix_mssp(strata_ctx* ctx, const uint32_t* sources, const int64_t* sr
   const bool dense = want_dense(ctx, true, narrow, n0, n1);
   if (b0 + b1 <= 32) {
     if (narrow)
-      return run_mssp<uint32_t, int32_t>(ctx, sources, src_w, src_inf, ns, e, b0, b1, besrc, nn, universe, cap, st,
+      return run_mssp<uint32_t, int32_t>(ctx, sources, fs.a.vary(), src_w, src_inf, ns, e, b0, b1, besrc, nn, universe, cap, st,
                                          et, l_start, n0, n1, dense);
-    return run_mssp<uint32_t, int64_t>(ctx, sources, src_w, src_inf, ns, e, b0, b1, besrc, nn, universe, cap, st,
+    return run_mssp<uint32_t, int64_t>(ctx, sources, fs.a.vary(), src_w, src_inf, ns, e, b0, b1, besrc, nn, universe, cap, st,
                                        et, l_start, n0, n1, dense);
   }
   if (narrow)
-    return run_mssp<uint64_t, int32_t>(ctx, sources, src_w, src_inf, ns, e, b0, b1, besrc, nn, universe, cap, st, et,
+    return run_mssp<uint64_t, int32_t>(ctx, sources, fs.a.vary(), src_w, src_inf, ns, e, b0, b1, besrc, nn, universe, cap, st, et,
                                        l_start, n0, n1, dense);
-  return run_mssp<uint64_t, int64_t>(ctx, sources, src_w, src_inf, ns, e, b0, b1, besrc, nn, universe, cap, st, et,
+  return run_mssp<uint64_t, int64_t>(ctx, sources, fs.a.vary(), src_w, src_inf, ns, e, b0, b1, besrc, nn, universe, cap, st, et,
                                      l_start, n0, n1, dense);
 }
 

@@ -16,13 +16,15 @@ constexpr uint64_t kMaxSortKeys = (1ull << 32) - 1;
 // Stable LSD radix sort (onesweep) of `n` keys on their low `bits` bits, with
 // optional values (V = uint32_t or uint64_t; has_vals selects them).  keys/alt
 // (and vals/valt) are a double buffer: on return `*keys` (and `*vals`) point at
-// the sorted data and `*alt` at the scratch half.  With `look` the bits in
-// which the keys differ are read back first (one synchronization) and only
-// those are sorted.  With kin (and vin) the data comes from there, untouched,
-// and the result lies in the buffers that *keys and *vals name on entry.
+// the sorted data and `*alt` at the scratch half.  Only the bits of `vary`, the
+// bits in which keys may differ, are sorted; with kSortLook they are read from
+// the keys first (one synchronization).  With kin (and vin) the data comes from
+// there, untouched, and the result lies in the buffers that *keys and *vals
+// name on entry.
+constexpr uint64_t kSortLook = 0, kSortAll = ~0ull;
 template <class K, class V>
-void radix_sort(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has_vals,
-                uint64_t n, int bits, bool look = true, const K* kin = nullptr, const V* vin = nullptr);
+void radix_sort(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has_vals, uint64_t n, int bits,
+                uint64_t vary, const K* kin = nullptr, const V* vin = nullptr);
 
 // Keys-per-thread choices of the onesweep tile for 4- or 8-byte keys
 // (strata_ctx_set_knob); returns how many, writes up to max_out.
@@ -181,9 +183,18 @@ void build_csr(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint64_t n
 uint64_t count_distinct_ids(strata_ctx* ctx, const uint32_t* a, uint64_t na, const uint32_t* b,
                             uint64_t nb, const uint32_t* c, uint64_t nc, uint64_t limit);
 
-// max over columns (synchronizing).
-void max_u32_pair(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, uint32_t* ma, uint32_t* mb);
-uint32_t max_u32(strata_ctx* ctx, const uint32_t* a, uint64_t n, const uint32_t* b = nullptr);  // over a and b
+// What one column's ids have in common: the largest, the bits that some have
+// set and the bits that some have clear.
+struct IdBits {
+  uint32_t max, some, none;
+  uint32_t vary() const { return some & none; }  // the bits in which they differ
+};
+// Two columns in one pass (synchronizing); `loops`: some row has a[i] == b[i].
+struct ColScan {
+  IdBits a, b;
+  bool loops;
+};
+ColScan col_scan(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n);
 
 // Pack two u32 columns into keys (c0 << shift) | c1, optional weight conversion
 // from (int64 w, u8 inf) to W codes (inf -> WInf<W>, finite v -> v - ctx->wshift).
@@ -202,11 +213,11 @@ void unpack_pairs(strata_ctx* ctx, const K* keys, const W* w, uint64_t n, int sh
 // there is none (both 0).  NULL w: every weight is Finite(0).
 bool weight_range(strata_ctx* ctx, const int64_t* w, const uint8_t* inf, uint64_t n, int64_t* mn, int64_t* mx);
 
-// Max |finite weight| over (w, inf) columns (synchronizing); 0 when n == 0.
-// A fixpoint's inputs in one pass: largest ids, largest |finite weight| of the
-// sources' and the edges' columns, and the number of distinct ids.
+// A fixpoint's inputs in one pass (synchronizing): the ids and the largest
+// |finite weight| of the sources' and the edges' columns (0 without rows), and
+// the number of distinct ids.
 struct FixScan {
-  uint32_t max_a, max_x, max_y;
+  IdBits a, x, y;
   uint64_t mag_a, mag_w, universe;
 };
 FixScan fix_scan(strata_ctx* ctx, const uint32_t* a, const int64_t* aw, const uint8_t* ainf, uint64_t na,

@@ -451,8 +451,10 @@ void prov_tc_capture(strata_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
   check_cuda(cudaEventRecord(e0, ctx->stream), "cudaEventRecord");
   const uint64_t l0 = ctx->launches;
   // ---- out-CSR sorted by (X, Y), edge fact ids as values; distinct edges
-  if (m && (max_u32(ctx, d_src, m) >= n || max_u32(ctx, d_dst, m) >= n))
-    fail(STRATA_E_INVALID, "an edge endpoint is outside [0, n)");
+  if (m) {
+    const ColScan cs = col_scan(ctx, d_src, d_dst, m);
+    if (cs.a.max >= n || cs.b.max >= n) fail(STRATA_E_INVALID, "an edge endpoint is outside [0, n)");
+  }
   const int b = std::max(1, bits_for(n ? n - 1 : 0));
   DBuf<uint64_t> keys(ctx, m + 1), kalt(ctx, m + 1);
   DBuf<uint32_t> idx(ctx, m + 1), ialt(ctx, m + 1), nbr(ctx, m + 1), off(ctx, (uint64_t)n + 1), flag(ctx, 2);
@@ -465,7 +467,7 @@ void prov_tc_capture(strata_ctx* ctx, uint32_t n, const uint32_t* d_src, const u
     uint64_t* ka = kalt.p;
     uint32_t* vp = idx.p;
     uint32_t* va = ialt.p;
-    radix_sort<uint64_t, uint32_t>(ctx, &kp, &ka, &vp, &va, true, m, 2 * b, false);
+    radix_sort<uint64_t, uint32_t>(ctx, &kp, &ka, &vp, &va, true, m, 2 * b, kSortAll);
     k_edge_check<<<(unsigned)ceil_div(m, 256), 256, 0, ctx->stream>>>(kp, d_prob, m, flag.p);
     after_launch(ctx, "k_edge_check");
     build_csr<uint64_t>(ctx, kp, m, b, n, off.p, nbr.p);

@@ -16,10 +16,11 @@
 //     written out in runs (coalesced per digit), values fetched through the
 //     source slot — no per-key value state stays in registers;
 //   * only the significant `bits` of the key are sorted (a 26-bit key takes 4
-//     passes, not 64), and where the host may look at the keys first only the
-//     bits that differ between them: a digit is up to eight such bits, from two
-//     separate windows of the key where one ends and the next begins (a packed
-//     pair (c0 << 32) | c1 of 19-bit ids takes 5 passes, not 6 or 8).
+//     passes, not 64), and of those only the ones that differ between the keys,
+//     where the caller knows them or lets the sort look: a digit is up to eight
+//     such bits, from two separate windows of the key where one ends and the
+//     next begins (a packed pair (c0 << 32) | c1 of 19-bit ids takes 5 passes,
+//     not 6 or 8).
 #include "sk_ops.cuh"
 #include "sk_prims.cuh"
 
@@ -381,16 +382,6 @@ __global__ void __launch_bounds__(NT, 4) k_onesweep(const K* __restrict__ kin, K
 
 namespace {
 
-// `bits` low bits in contiguous 8-bit digits.
-std::vector<Digit> plain_digits(int bits) {
-  std::vector<Digit> g;
-  for (int s = 0; s < bits; s += 8) {
-    const int l = std::min(8, bits - s);
-    g.push_back(Digit{s, 0, l, l, (1u << l) - 1, 0u});
-  }
-  return g;
-}
-
 // Digits over the set bits of `vary`, lowest first: a window of at most eight
 // bits from the lowest one left (up to its last varying bit), then a second
 // window where the first leaves room.
@@ -418,24 +409,19 @@ std::vector<Digit> varying_digits(uint64_t vary) {
 // *keys / *vals (the result is there on return).
 template <class K, class V, int ITEMS>
 void radix_sort_impl(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has_vals,
-                     uint64_t n, int bits, bool look, const K* kin, const V* vin) {
+                     uint64_t n, int bits, uint64_t vary, const K* kin, const V* vin) {
   constexpr uint32_t TILE = NT * ITEMS;
   const K* src = kin ? kin : *keys;
   const V* vsrc = vin ? vin : *vals;
-  std::vector<Digit> dg;
-  if (look) {
+  if (vary == kSortLook) {
     DBuf<uint64_t> m(ctx, 1);
     SK_CUDA(cudaMemsetAsync(m.p, 0, 8, ctx->stream));
     k_radix_varying<K><<<(unsigned)std::min<uint64_t>(ceil_div(n, NT * 8), (uint64_t)ctx->num_sms * 8), NT, 0,
                          ctx->stream>>>(src, n, reinterpret_cast<unsigned long long*>(m.p));
     after_launch(ctx, "k_radix_varying");
-    uint64_t vary;
     read_u64(ctx, m.p, &vary, 1);
-    if (bits < 64) vary &= (1ull << bits) - 1;
-    dg = varying_digits(vary);
-  } else {
-    dg = plain_digits(bits);
   }
+  const std::vector<Digit> dg = varying_digits(bits < 64 ? vary & ((1ull << bits) - 1) : vary);
   const int passes = (int)dg.size();
   if (passes == 0) {
     if (kin) SK_CUDA(cudaMemcpyAsync(*keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -539,7 +525,7 @@ int radix_items_choices(int key_bytes, int* out, int max_out) {
 
 template <class K, class V>
 void radix_sort(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has_vals,
-                uint64_t n, int bits, bool look, const K* kin, const V* vin) {
+                uint64_t n, int bits, uint64_t vary, const K* kin, const V* vin) {
   if (n <= 1 || bits <= 0) {
     if (kin && n) SK_CUDA(cudaMemcpyAsync(*keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, ctx->stream));
     if (vin && n && has_vals)
@@ -549,7 +535,7 @@ void radix_sort(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has
   if (n > kMaxSortKeys) fail(STRATA_E_UNSUPPORTED, "radix sort call limited to 2^32-1 keys");
   if (bits > (int)(8 * sizeof(K))) bits = 8 * sizeof(K);
   auto run = [&](auto items) {
-    radix_sort_impl<K, V, decltype(items)::value>(ctx, keys, alt, vals, valt, has_vals, n, bits, look, kin, vin);
+    radix_sort_impl<K, V, decltype(items)::value>(ctx, keys, alt, vals, valt, has_vals, n, bits, vary, kin, vin);
   };
   if constexpr (sizeof(K) == 4) {
     switch (ctx->tune_items4) {
@@ -568,7 +554,8 @@ void radix_sort(strata_ctx* ctx, K** keys, K** alt, V** vals, V** valt, bool has
 }
 
 #define SK_INST_SORT(K, V)                                                                   \
-  template void radix_sort<K, V>(strata_ctx*, K**, K**, V**, V**, bool, uint64_t, int, bool, const K*, const V*);
+  template void radix_sort<K, V>(strata_ctx*, K**, K**, V**, V**, bool, uint64_t, int, uint64_t, const K*, \
+                                 const V*);
 SK_INST_SORT(uint32_t, uint32_t)
 SK_INST_SORT(uint32_t, uint64_t)
 SK_INST_SORT(uint64_t, uint32_t)

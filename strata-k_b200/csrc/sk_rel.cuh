@@ -69,6 +69,7 @@ struct EdgeCols {
   const int64_t* w = nullptr;
   const uint8_t* inf = nullptr;
   uint64_t n = 0;
+  uint32_t vsrc = ~0u, vdst = ~0u;  // the bits in which the ids of a column may differ
 };
 
 strata_rel* fix_tc_bool(strata_ctx* ctx, const EdgeCols& e, strata_fix_stats* st);

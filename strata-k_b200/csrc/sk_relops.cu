@@ -633,25 +633,58 @@ __global__ void k_popcount(const uint32_t* __restrict__ bitmap, uint64_t words, 
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
-// The largest value of a (out[0]) and of b, when given (out[1]), over n rows.
-__global__ void k_max_u32(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, uint64_t n, uint32_t* out) {
-  uint32_t m = 0, mb = 0;
+// One thread's IdBits.
+struct IdAcc {
+  uint32_t max = 0, some = 0, none = 0;
+  __device__ void add(uint32_t v) {
+    max = v > max ? v : max;
+    some |= v;
+    none |= ~v;
+  }
+};
+// Add the block's columns to out (every thread takes part; once per kernel).
+// Blocks meet at a few words, so each adds once: a warp at a time it was
+// 20 us more for 400 k rows.
+template <int N>
+__device__ __forceinline__ void add_columns(const IdAcc (&col)[N], IdBits* out) {
+  __shared__ uint32_t s[3 * N][NT / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    const uint32_t m = __reduce_max_sync(kFull, col[q].max);
+    const uint32_t b = __reduce_or_sync(kFull, col[q].some), z = __reduce_or_sync(kFull, col[q].none);
+    if (lane == 0) {
+      s[3 * q][warp] = m;
+      s[3 * q + 1][warp] = b;
+      s[3 * q + 2][warp] = z;
+    }
+  }
+  __syncthreads();
+  for (int k = warp; k < 3 * N; k += NT / 32) {
+    const uint32_t x = lane < NT / 32 ? s[k][lane] : 0u;
+    const uint32_t m = __reduce_max_sync(kFull, x), b = __reduce_or_sync(kFull, x);
+    if (lane != 0) continue;
+    IdBits* o = out + k / 3;
+    if (k % 3 == 0) atomicMax(&o->max, m);
+    else atomicOr(k % 3 == 1 ? &o->some : &o->none, b);
+  }
+}
+
+struct ColOut {
+  IdBits c[2];
+  uint32_t loops, pad;
+};
+__global__ void k_col_scan(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, uint64_t n, ColOut* out) {
+  IdAcc c[2];
+  bool loop = false;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    m = a[i] > m ? a[i] : m;
-    if (b) mb = b[i] > mb ? b[i] : mb;
+    const uint32_t u = a[i], v = b[i];
+    c[0].add(u);
+    c[1].add(v);
+    loop |= u == v;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const uint32_t t = __shfl_xor_sync(kFull, m, o);
-    m = t > m ? t : m;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const uint32_t t = __shfl_xor_sync(kFull, mb, o);
-    mb = t > mb ? t : mb;
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(&out[0], m);
-    if (mb) atomicMax(&out[1], mb);
-  }
+  add_columns(c, out->c);
+  if (loop) out->loops = 1u;
 }
 
 template <class K>
@@ -670,17 +703,22 @@ __device__ __forceinline__ W pack_weight(const int64_t* w, const uint8_t* inf, u
   return (W)code;
 }
 
-// Everything a fixpoint's set-up asks of its inputs in one pass: the largest
-// ids of the source column a (may be absent) and the edge columns x, y
-// (out[0..2]), the largest |finite weight| of a's and the edges' (out[3], out[4]),
-// and, in a bitmap of ids below `limit`, which ids occur (k_popcount
-// then counts them into out[5]).
+// Everything a fixpoint's set-up asks of its inputs in one pass: the ids of
+// the source column a (may be absent) and of the edge columns x, y, the largest
+// |finite weight| of a's and the edges', and, in a bitmap of ids below
+// `limit`, which ids occur (k_popcount then counts them).
+struct FixOut {
+  unsigned long long mag_a, mag_w, ids;
+  IdBits c[3];  // a, x, y
+  uint32_t pad;
+};
 __global__ void k_fix_scan(const uint32_t* __restrict__ a, const int64_t* __restrict__ aw,
                            const uint8_t* __restrict__ ainf, uint64_t na, const uint32_t* __restrict__ x,
                            const uint32_t* __restrict__ y, const int64_t* __restrict__ w,
                            const uint8_t* __restrict__ winf, uint64_t m, uint32_t* bitmap, uint64_t limit,
-                           unsigned long long* out) {
-  unsigned long long mx[5] = {0, 0, 0, 0, 0};
+                           FixOut* out) {
+  unsigned long long mg[2] = {0, 0};
+  IdAcc c[3];
   auto mark = [&](uint32_t v) {
     if (v >= limit) return;
     const uint32_t bit = 1u << (v & 31);
@@ -690,31 +728,32 @@ __global__ void k_fix_scan(const uint32_t* __restrict__ a, const int64_t* __rest
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x, t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (uint64_t i = t0; i < na; i += stride) {
     const uint32_t v = a[i];
-    mx[0] = v > mx[0] ? v : mx[0];
+    c[0].add(v);
     mark(v);
     if (aw && !(ainf && ainf[i])) {
       const unsigned long long g = mag(aw[i]);
-      mx[3] = g > mx[3] ? g : mx[3];
+      mg[0] = g > mg[0] ? g : mg[0];
     }
   }
   for (uint64_t i = t0; i < m; i += stride) {
     const uint32_t u = x[i], v = y[i];
-    mx[1] = u > mx[1] ? u : mx[1];
-    mx[2] = v > mx[2] ? v : mx[2];
+    c[1].add(u);
+    c[2].add(v);
     mark(u);
     mark(v);
     if (w && !(winf && winf[i])) {
       const unsigned long long g = mag(w[i]);
-      mx[4] = g > mx[4] ? g : mx[4];
+      mg[1] = g > mg[1] ? g : mg[1];
     }
   }
+  add_columns(c, out->c);
 #pragma unroll
-  for (int q = 0; q < 5; q++) {
+  for (int q = 0; q < 2; q++) {
     for (int o = 16; o > 0; o >>= 1) {
-      const unsigned long long t = __shfl_xor_sync(kFull, mx[q], o);
-      mx[q] = t > mx[q] ? t : mx[q];
+      const unsigned long long t = __shfl_xor_sync(kFull, mg[q], o);
+      mg[q] = t > mg[q] ? t : mg[q];
     }
-    if ((threadIdx.x & 31) == 0 && mx[q]) atomicMax(&out[q], mx[q]);
+    if ((threadIdx.x & 31) == 0 && mg[q]) atomicMax(q ? &out->mag_w : &out->mag_a, mg[q]);
   }
 }
 
@@ -1104,23 +1143,17 @@ uint64_t count_distinct_ids(strata_ctx* ctx, const uint32_t* a, uint64_t na, con
   return r;
 }
 
-void max_u32_pair(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, uint32_t* ma, uint32_t* mb) {
-  *ma = *mb = 0;
-  if (n == 0) return;
-  DBuf<uint64_t> m(ctx, 1);
-  SK_CUDA(cudaMemsetAsync(m.p, 0, 8, ctx->stream));
-  k_max_u32<<<grid_for(ctx, n), NT, 0, ctx->stream>>>(a, b, n, reinterpret_cast<uint32_t*>(m.p));
-  after_launch(ctx, "k_max_u32");
-  uint64_t r;
-  read_u64(ctx, m.p, &r, 1);
-  *ma = (uint32_t)r;
-  *mb = (uint32_t)(r >> 32);
-}
-
-uint32_t max_u32(strata_ctx* ctx, const uint32_t* a, uint64_t n, const uint32_t* b) {
-  uint32_t ma, mb;
-  max_u32_pair(ctx, a, b, n, &ma, &mb);
-  return std::max(ma, mb);
+ColScan col_scan(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n) {
+  constexpr int words = sizeof(ColOut) / 8;
+  DBuf<uint64_t> m(ctx, words);
+  SK_CUDA(cudaMemsetAsync(m.p, 0, sizeof(ColOut), ctx->stream));
+  k_col_scan<<<grid_for(ctx, n), NT, 0, ctx->stream>>>(a, b, n, reinterpret_cast<ColOut*>(m.p));
+  after_launch(ctx, "k_col_scan");
+  uint64_t h[words];
+  read_u64(ctx, m.p, h, words);
+  ColOut r;
+  std::memcpy(&r, h, sizeof(r));
+  return ColScan{r.c[0], r.c[1], r.loops != 0};
 }
 
 FixScan fix_scan(strata_ctx* ctx, const uint32_t* a, const int64_t* aw, const uint8_t* ainf, uint64_t na,
@@ -1130,23 +1163,26 @@ FixScan fix_scan(strata_ctx* ctx, const uint32_t* a, const int64_t* aw, const ui
   // and hub ids are better marked in shared memory (count_distinct_ids).  So
   // too under a memory cap that has no room for the 128 KB.
   constexpr uint64_t kIds = 1ull << 20;
-  const bool room = !ctx->cap || ctx->in_use + size_class((6 + kIds / 64) * 8) <= ctx->cap;
+  constexpr int words = sizeof(FixOut) / 8;
+  const bool room = !ctx->cap || ctx->in_use + size_class((words + kIds / 64) * 8) <= ctx->cap;
   const uint64_t limit = na + m <= kIds && room ? kIds : 0;
-  DBuf<uint64_t> buf(ctx, 6 + limit / 64);
-  SK_CUDA(cudaMemsetAsync(buf.p, 0, (6 + limit / 64) * 8, ctx->stream));
-  auto* out = reinterpret_cast<unsigned long long*>(buf.p);
-  uint32_t* bitmap = reinterpret_cast<uint32_t*>(buf.p + 6);
+  DBuf<uint64_t> buf(ctx, words + limit / 64);
+  SK_CUDA(cudaMemsetAsync(buf.p, 0, (words + limit / 64) * 8, ctx->stream));
+  auto* out = reinterpret_cast<FixOut*>(buf.p);
+  uint32_t* bitmap = reinterpret_cast<uint32_t*>(buf.p + words);
   k_fix_scan<<<grid_for(ctx, std::max(na, m)), NT, 0, ctx->stream>>>(a, aw, ainf, na, x, y, w, winf, m, bitmap, limit,
                                                                      out);
   after_launch(ctx, "k_fix_scan");
   if (limit) {
-    k_popcount<<<grid_for(ctx, limit / 32), NT, 0, ctx->stream>>>(bitmap, limit / 32, out + 5);
+    k_popcount<<<grid_for(ctx, limit / 32), NT, 0, ctx->stream>>>(bitmap, limit / 32, &out->ids);
     after_launch(ctx, "k_popcount");
   }
-  uint64_t h[6];
-  read_u64(ctx, buf.p, h, 6);
-  FixScan r{(uint32_t)h[0], (uint32_t)h[1], (uint32_t)h[2], h[3], h[4], h[5]};
-  const uint64_t ids = std::max(h[0], std::max(h[1], h[2])) + 1;
+  uint64_t h[words];
+  read_u64(ctx, buf.p, h, words);
+  FixOut o;
+  std::memcpy(&o, h, sizeof(o));
+  FixScan r{o.c[0], o.c[1], o.c[2], o.mag_a, o.mag_w, o.ids};
+  const uint64_t ids = (uint64_t)std::max(r.a.max, std::max(r.x.max, r.y.max)) + 1;
   if (ids > limit) {
     buf.release();
     r.universe = count_distinct_ids(ctx, a, na, x, m, y, m, ids);

@@ -532,7 +532,7 @@ TsvResult tsv_load(strata_ctx* ctx, const char* text, uint64_t text_len, uint32_
     uint64_t* ha = h2.p;
     pp = pos.p;
     uint32_t* pa = pos2.p;
-    radix_sort<uint64_t, uint32_t>(ctx, &hp, &ha, &pp, &pa, true, n_cells, 64, false);
+    radix_sort<uint64_t, uint32_t>(ctx, &hp, &ha, &pp, &pa, true, n_cells, 64, kSortAll);
     SK_CUDA(cudaMemsetAsync(coll.p, 0, 4, ctx->stream));
     k_cell_verify<<<gridn(n_cells, NT), NT, 0, ctx->stream>>>(B.p, coff.p, clen.p, hp, pp, n_cells, head.p, coll.p);
     after_launch(ctx, "k_cell_verify");

@@ -775,15 +775,15 @@ __global__ void k_tri_list_sum(const K* __restrict__ keys, uint64_t m, int bits,
 }
 
 // Sort + dedup packed keys in `keys` (n), result in out (returns count).
-// `look`: the keys may vary in few of their bits (packed ids vary in all).
+// `vary`: the bits in which they may differ (sk_ops.cuh).
 template <class K>
-uint64_t sort_unique(strata_ctx* ctx, DBuf<K>& keys, uint64_t n, int bits, DBuf<K>& out, bool look = false) {
+uint64_t sort_unique(strata_ctx* ctx, DBuf<K>& keys, uint64_t n, int bits, uint64_t vary, DBuf<K>& out) {
   DBuf<K> alt(ctx, n + 1);
   K* kp = keys.p;
   K* ka = alt.p;
   uint32_t* vp = nullptr;
   uint32_t* va = nullptr;
-  radix_sort<K, uint32_t>(ctx, &kp, &ka, &vp, &va, false, n, bits, look);
+  radix_sort<K, uint32_t>(ctx, &kp, &ka, &vp, &va, false, n, bits, vary);
   out.reserve(n + 1);
   DBuf<uint64_t> cnt(ctx, 1);
   reduce_runs<K, int32_t, false>(ctx, kp, nullptr, n, out.p, nullptr, cnt.p);
@@ -933,7 +933,7 @@ void hub_labels(strata_ctx* ctx, const uint32_t* deg, uint64_t n_nodes, DBuf<uin
   k_hub_sort_keys<<<blocks(n_nodes), 256, 0, ctx->stream>>>(deg, n_nodes, k.p, id.p);
   after_launch(ctx, "k_hub_sort_keys");
   uint32_t *kp = k.p, *kalt = ka.p, *vp = id.p, *valt = ia.p;
-  radix_sort<uint32_t, uint32_t>(ctx, &kp, &kalt, &vp, &valt, true, n_nodes, 32, true);
+  radix_sort<uint32_t, uint32_t>(ctx, &kp, &kalt, &vp, &valt, true, n_nodes, 32, kSortLook);
   label.reserve(n_nodes);
   k_hub_labels<<<blocks(n_nodes), 256, 0, ctx->stream>>>(vp, n_nodes, label.p);
   after_launch(ctx, "k_hub_labels");
@@ -984,9 +984,35 @@ uint64_t hub_count(strata_ctx* ctx, const K* keys, uint64_t m, int bits, uint64_
   return r;
 }
 
+// The ids of two edge columns: bits of the largest, one past it, and the bits
+// in which the packed keys may differ.
+struct Ids {
+  int bits;
+  uint64_t n_nodes;
+  uint32_t vx, vy;    // bits in which the ids of a column differ
+  uint32_t any, hole; // of both columns together; the bits not set in all of them
+  bool loops;
+  uint64_t pattern() const { return (uint64_t)vx << bits | vy; }
+  // either column's id in either half; a self-loop's key is all ones
+  uint64_t undirected(bool with_loops) const {
+    const uint64_t v = with_loops && loops ? hole & ((1ull << bits) - 1) : any;
+    return v << bits | v;
+  }
+};
+
+Ids id_space(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n) {
+  const ColScan c = col_scan(ctx, a, b, n);
+  const uint32_t m = std::max(c.a.max, c.b.max);
+  const uint32_t hole = c.a.none | c.b.none;
+  return Ids{std::max(1, bits_for(m)), (uint64_t)m + 1, c.a.vary(), c.b.vary(), (c.a.some | c.b.some) & hole, hole,
+             c.loops};
+}
+
 template <class K>
-uint64_t pattern_impl(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uint64_t n, int b,
-                      uint64_t n_nodes, uint64_t u_lo = 0, uint64_t u_hi = ~0ull) {
+uint64_t pattern_impl(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uint64_t n, const Ids& I,
+                      uint64_t u_lo = 0, uint64_t u_hi = ~0ull) {
+  const int b = I.bits;
+  const uint64_t n_nodes = I.n_nodes;
   if (u_hi > n_nodes) u_hi = n_nodes;
   if (u_lo >= u_hi) return 0;
   DBuf<K> keys(ctx, n + 1), uniq;
@@ -1006,7 +1032,7 @@ uint64_t pattern_impl(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uin
       hub_labels(ctx, deg.p, n_nodes, label, whole ? nullptr : &order);
       k_hub_pack<K><<<blocks(n), 256, 0, ctx->stream>>>(x, y, n, label.p, b, 0, keys.p);
       after_launch(ctx, "k_hub_pack");
-      const uint64_t m = sort_unique<K>(ctx, keys, n, 2 * b, uniq);
+      const uint64_t m = sort_unique<K>(ctx, keys, n, 2 * b, kSortAll, uniq);
       r = hub_count<K>(ctx, uniq.p, m, b, n_nodes, whole ? nullptr : order.p, (uint32_t)u_lo, (uint32_t)u_hi);
       counted = true;
     });
@@ -1014,20 +1040,22 @@ uint64_t pattern_impl(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uin
     uniq.release();
   }
   pack_pairs<K, int32_t, false>(ctx, x, y, nullptr, nullptr, n, b, keys.p, nullptr);
-  const uint64_t m = sort_unique<K>(ctx, keys, n, 2 * b, uniq);
+  const uint64_t m = sort_unique<K>(ctx, keys, n, 2 * b, I.pattern(), uniq);
   return tri_from_sorted<K>(ctx, uniq.p, m, b, n_nodes, u_lo, u_hi);
 }
 
 // Canonicalize, dedup, drop self-loops, orient by (degree, id).  Leaves the
 // oriented sorted keys in `out` and returns their count.
 template <class K>
-uint64_t oriented_edges(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, int bits,
-                        uint64_t n_nodes, bool by_degree, DBuf<K>& out) {
+uint64_t oriented_edges(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, const Ids& I,
+                        bool by_degree, DBuf<K>& out) {
+  const int bits = I.bits;
+  const uint64_t n_nodes = I.n_nodes;
   DBuf<K> keys(ctx, n + 1), uniq;
   uniq.ctx = ctx;
   k_canon<K><<<blocks(n), 256, 0, ctx->stream>>>(a, b, n, bits, keys.p);
   after_launch(ctx, "k_canon");
-  const uint64_t m = drop_loops<K>(ctx, uniq, sort_unique<K>(ctx, keys, n, 2 * bits, uniq), bits);
+  const uint64_t m = drop_loops<K>(ctx, uniq, sort_unique<K>(ctx, keys, n, 2 * bits, I.undirected(true), uniq), bits);
   if (!by_degree || m == 0) {
     out = std::move(uniq);
     return m;
@@ -1043,15 +1071,16 @@ uint64_t oriented_edges(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, u
   K* ka = alt.p;
   uint32_t* vp = nullptr;
   uint32_t* va = nullptr;
-  radix_sort<K, uint32_t>(ctx, &kp, &ka, &vp, &va, false, m, 2 * bits, false);
+  radix_sort<K, uint32_t>(ctx, &kp, &ka, &vp, &va, false, m, 2 * bits, I.undirected(false));
   if (kp == uniq.p) out = std::move(uniq);
   else out = std::move(alt);
   return m;
 }
 
 template <class K>
-uint64_t tri_undirected_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, int bits,
-                             uint64_t n_nodes) {
+uint64_t tri_undirected_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, const Ids& I) {
+  const int bits = I.bits;
+  const uint64_t n_nodes = I.n_nodes;
   DBuf<K> ori;
   ori.ctx = ctx;
   if (hub_fits(ctx, n, kHubMinUndirected, n_nodes, sizeof(K))) {
@@ -1069,7 +1098,7 @@ uint64_t tri_undirected_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t*
       DBuf<K> keys(ctx, n + 1);
       k_hub_pack<K><<<blocks(n), 256, 0, ctx->stream>>>(a, b, n, label.p, bits, 1, keys.p);
       after_launch(ctx, "k_hub_pack");
-      const uint64_t m = drop_loops<K>(ctx, ori, sort_unique<K>(ctx, keys, n, 2 * bits, ori), bits);
+      const uint64_t m = drop_loops<K>(ctx, ori, sort_unique<K>(ctx, keys, n, 2 * bits, kSortAll, ori), bits);
       if (m == 0) return;
       r = hs.covered(n_nodes) ? hub_count<K>(ctx, ori.p, m, bits, n_nodes, nullptr, 0, 0)
                               : tri_from_sorted<K>(ctx, ori.p, m, bits, n_nodes);
@@ -1077,16 +1106,18 @@ uint64_t tri_undirected_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t*
     if (had && counted) return r;
     ori.release();
   }
-  const uint64_t m = oriented_edges<K>(ctx, a, b, n, bits, n_nodes, true, ori);
+  const uint64_t m = oriented_edges<K>(ctx, a, b, n, I, true, ori);
   if (m == 0) return 0;
   return tri_from_sorted<K>(ctx, ori.p, m, bits, n_nodes);
 }
 
 template <class K>
-uint64_t k4_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, int bits, uint64_t n_nodes) {
+uint64_t k4_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, const Ids& I) {
+  const int bits = I.bits;
+  const uint64_t n_nodes = I.n_nodes;
   DBuf<K> ori;
   ori.ctx = ctx;
-  const uint64_t m = oriented_edges<K>(ctx, a, b, n, bits, n_nodes, true, ori);
+  const uint64_t m = oriented_edges<K>(ctx, a, b, n, I, true, ori);
   if (m == 0) return 0;
   DBuf<uint32_t> off(ctx, n_nodes + 1), nbr(ctx, m + 1);
   build_csr<K>(ctx, ori.p, m, bits, n_nodes, off.p, nbr.p);
@@ -1126,10 +1157,12 @@ uint64_t k4_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t
 }
 
 template <class K>
-uint64_t bpi_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, int bits, uint64_t n_nodes) {
+uint64_t bpi_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n, const Ids& I) {
+  const int bits = I.bits;
+  const uint64_t n_nodes = I.n_nodes;
   DBuf<K> ori;
   ori.ctx = ctx;
-  const uint64_t m = oriented_edges<K>(ctx, a, b, n, bits, n_nodes, false, ori);
+  const uint64_t m = oriented_edges<K>(ctx, a, b, n, I, false, ori);
   if (m == 0) return 0;
   DBuf<uint32_t> off(ctx, n_nodes + 1), nbr(ctx, m + 1);
   build_csr<K>(ctx, ori.p, m, bits, n_nodes, off.p, nbr.p);
@@ -1142,24 +1175,14 @@ uint64_t bpi_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_
   return r;
 }
 
-struct Ids {
-  int bits;
-  uint64_t n_nodes;
-};
-
-Ids id_space(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n) {
-  const uint32_t m = max_u32(ctx, a, n, b);
-  return Ids{std::max(1, bits_for(m)), (uint64_t)m + 1};
-}
-
 }  // namespace
 
 uint64_t count_triangle_pattern(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uint64_t n) {
   reset_status(ctx);
   if (n == 0) return 0;
   const Ids I = id_space(ctx, x, y, n);
-  if (2 * I.bits <= 32) return pattern_impl<uint32_t>(ctx, x, y, n, I.bits, I.n_nodes);
-  return pattern_impl<uint64_t>(ctx, x, y, n, I.bits, I.n_nodes);
+  if (2 * I.bits <= 32) return pattern_impl<uint32_t>(ctx, x, y, n, I);
+  return pattern_impl<uint64_t>(ctx, x, y, n, I);
 }
 
 uint64_t count_triangle_pattern_range(strata_ctx* ctx, const uint32_t* x, const uint32_t* y, uint64_t n,
@@ -1167,32 +1190,32 @@ uint64_t count_triangle_pattern_range(strata_ctx* ctx, const uint32_t* x, const 
   reset_status(ctx);
   if (n == 0 || u_lo >= u_hi) return 0;
   const Ids I = id_space(ctx, x, y, n);
-  if (2 * I.bits <= 32) return pattern_impl<uint32_t>(ctx, x, y, n, I.bits, I.n_nodes, u_lo, u_hi);
-  return pattern_impl<uint64_t>(ctx, x, y, n, I.bits, I.n_nodes, u_lo, u_hi);
+  if (2 * I.bits <= 32) return pattern_impl<uint32_t>(ctx, x, y, n, I, u_lo, u_hi);
+  return pattern_impl<uint64_t>(ctx, x, y, n, I, u_lo, u_hi);
 }
 
 uint64_t count_triangles_undirected(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n) {
   reset_status(ctx);
   if (n == 0) return 0;
   const Ids I = id_space(ctx, a, b, n);
-  if (2 * I.bits <= 32) return tri_undirected_impl<uint32_t>(ctx, a, b, n, I.bits, I.n_nodes);
-  return tri_undirected_impl<uint64_t>(ctx, a, b, n, I.bits, I.n_nodes);
+  if (2 * I.bits <= 32) return tri_undirected_impl<uint32_t>(ctx, a, b, n, I);
+  return tri_undirected_impl<uint64_t>(ctx, a, b, n, I);
 }
 
 uint64_t count_4cliques_undirected(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n) {
   reset_status(ctx);
   if (n == 0) return 0;
   const Ids I = id_space(ctx, a, b, n);
-  if (2 * I.bits <= 32) return k4_impl<uint32_t>(ctx, a, b, n, I.bits, I.n_nodes);
-  return k4_impl<uint64_t>(ctx, a, b, n, I.bits, I.n_nodes);
+  if (2 * I.bits <= 32) return k4_impl<uint32_t>(ctx, a, b, n, I);
+  return k4_impl<uint64_t>(ctx, a, b, n, I);
 }
 
 uint64_t binary_plan_intermediate(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t n) {
   reset_status(ctx);
   if (n == 0) return 0;
   const Ids I = id_space(ctx, a, b, n);
-  if (2 * I.bits <= 32) return bpi_impl<uint32_t>(ctx, a, b, n, I.bits, I.n_nodes);
-  return bpi_impl<uint64_t>(ctx, a, b, n, I.bits, I.n_nodes);
+  if (2 * I.bits <= 32) return bpi_impl<uint32_t>(ctx, a, b, n, I);
+  return bpi_impl<uint64_t>(ctx, a, b, n, I);
 }
 
 uint64_t intern_terms(strata_ctx* ctx, const uint64_t* keys, uint64_t n, uint32_t* ids) {
@@ -1208,7 +1231,7 @@ uint64_t intern_terms(strata_ctx* ctx, const uint64_t* keys, uint64_t n, uint32_
   DBuf<uint64_t> copy(ctx, n + 1), table;
   table.ctx = ctx;
   SK_CUDA(cudaMemcpyAsync(copy.p, keys, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-  const uint64_t m = sort_unique<uint64_t>(ctx, copy, n, std::max(1, bits_for(maxk)), table, true);
+  const uint64_t m = sort_unique<uint64_t>(ctx, copy, n, std::max(1, bits_for(maxk)), kSortLook, table);
   k_intern_map<<<blocks(n), 256, 0, ctx->stream>>>(keys, n, table.p, m, ids);
   after_launch(ctx, "k_intern_map");
   sync_and_check(ctx);
