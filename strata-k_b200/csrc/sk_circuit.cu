@@ -406,43 +406,56 @@ __global__ void __launch_bounds__(CK_NT) k_circuit_adjoint(strata_circuits c, co
 }
 
 // ---- circuits staged in shared memory -----------------------------------------
-// Structure and values of one query's circuit, node and child ids local.
-constexpr uint32_t kStageNodes = 1536;  // nodes, and children, of a staged circuit
+// Structure and values of one query's circuit, node and child ids local, in a
+// block's dynamic shared memory sized for the set's largest circuit.
 struct StageMem {
-  float hi[kStageNodes], lo[kStageNodes], adj[kStageNodes];
-  uint32_t a[kStageNodes];        // leaf, or first child | children << 16
-  uint16_t ch[kStageNodes];
-  uint8_t kind[kStageNodes];
+  float *hi, *lo, *adj;  // adj: gradients only
+  uint32_t* a;           // leaf, or first child | children << 16
+  uint16_t* ch;
+  uint8_t* kind;
 };
 
-__device__ __forceinline__ ff stage_value(const StageMem* m, uint32_t i) { return ff{m->hi[i], m->lo[i]}; }
+inline __host__ __device__ uint32_t stage_even(uint64_t n) { return (uint32_t)((n + 1) & ~1ull); }
+inline size_t stage_bytes(uint64_t nodes, uint64_t children, bool grad) {
+  return stage_even(nodes) * (size_t)(grad ? 16 : 12) + stage_even(children) * (size_t)2 + nodes;
+}
+__device__ __forceinline__ StageMem stage_mem(unsigned char* base, uint32_t nodes, uint32_t children, bool grad) {
+  StageMem m;
+  const uint32_t n = stage_even(nodes);
+  m.hi = reinterpret_cast<float*>(base);
+  m.lo = m.hi + n;
+  m.a = reinterpret_cast<uint32_t*>(m.lo + n);
+  m.adj = reinterpret_cast<float*>(m.a + n);
+  m.ch = reinterpret_cast<uint16_t*>(grad ? m.adj + n : m.adj);
+  m.kind = reinterpret_cast<uint8_t*>(m.ch + stage_even(children));
+  return m;
+}
+
+__device__ __forceinline__ ff stage_value(const StageMem& m, uint32_t i) { return ff{m.hi[i], m.lo[i]}; }
 
 // Copy a circuit of n nodes and its children into shared memory.
-__device__ __forceinline__ void stage_circuit(const strata_circuits& c, StageMem* m, uint64_t n0, uint64_t ch0,
+__device__ __forceinline__ void stage_circuit(const strata_circuits& c, const StageMem& m, uint64_t n0, uint64_t ch0,
                                               uint32_t n, uint32_t nch) {
   for (uint32_t i = threadIdx.x; i < n; i += CK_NT) {
     const uint8_t kd = c.kind[n0 + i];
-    m->kind[i] = kd;
-    m->a[i] = kd == 2 || kd == 3 ? (uint32_t)(c.a[n0 + i] - ch0) | (c.b[n0 + i] << 16) : c.a[n0 + i];
+    m.kind[i] = kd;
+    m.a[i] = kd == 2 || kd == 3 ? (uint32_t)(c.a[n0 + i] - ch0) | (c.b[n0 + i] << 16) : c.a[n0 + i];
   }
-  for (uint32_t i = threadIdx.x; i < nch; i += CK_NT) m->ch[i] = (uint16_t)(c.ch[ch0 + i] - n0);
+  for (uint32_t i = threadIdx.x; i < nch; i += CK_NT) m.ch[i] = (uint16_t)(c.ch[ch0 + i] - n0);
   __syncthreads();
 }
 
 // The same sweeps as k_circuit_forward and k_circuit_adjoint (the values bit by
-// bit) on a circuit copied into shared memory, for sets whose largest circuit
-// has at most kStageNodes nodes and children: each level is a few dependent
+// bit) on a circuit copied into shared memory: each level is a few dependent
 // shared-memory reads instead of four dependent global ones, which is what
 // bounds the sweep (1,024 queries of up to 8 path proofs, one B200: values 37
-// -> 19 us, values and gradients 37 + 65 -> 46 us).  Larger circuits need the
-// first-level cache for their values: with the stage's shared memory set aside
-// 96 queries of 16,000 nodes took 308 us instead of 220.
+// -> 19 us, values and gradients 37 + 65 -> 46 us).
 template <bool GRAD>
 __global__ void __launch_bounds__(CK_NT) k_circuit_staged(strata_circuits c, const float* __restrict__ p, float* out32,
                                                           double* out64, const float* __restrict__ seed,
                                                           double* g_out) {
   extern __shared__ __align__(16) unsigned char s_stage[];
-  StageMem* m = reinterpret_cast<StageMem*>(s_stage);
+  const StageMem m = stage_mem(s_stage, c.max_nodes, c.max_children, GRAD);
   const uint32_t q = blockIdx.x;
   const uint64_t n0 = c.qnode[q], ch0 = c.qchild[q], l0 = c.qlevel[q];
   const uint32_t n = (uint32_t)(c.qnode[q + 1] - n0), nch = (uint32_t)(c.qchild[q + 1] - ch0);
@@ -451,7 +464,7 @@ __global__ void __launch_bounds__(CK_NT) k_circuit_staged(strata_circuits c, con
   stage_circuit(c, m, n0, ch0, n, nch);
   for (uint32_t L = 0; L < levels; L++) {
     for (uint32_t i = lvl[L] + threadIdx.x; i < lvl[L + 1]; i += CK_NT) {
-      const uint32_t kd = m->kind[i], a = m->a[i];
+      const uint32_t kd = m.kind[i], a = m.a[i];
       const uint32_t f = a & 0xffffu, nc = a >> 16;  // of an And / Or node
       ff x;
       if (kd == 0) {
@@ -460,41 +473,41 @@ __global__ void __launch_bounds__(CK_NT) k_circuit_staged(strata_circuits c, con
         x = ff_two_sum(1.0f, -p[a]);  // 1 - p, exactly
       } else if (kd == 2) {
         x = ff{1.0f, 0.0f};
-        for (uint32_t j = 0; j < nc; j++) x = ff_mul(x, stage_value(m, m->ch[f + j]));
+        for (uint32_t j = 0; j < nc; j++) x = ff_mul(x, stage_value(m, m.ch[f + j]));
       } else if (kd == 3) {
         x = ff{0.0f, 0.0f};
-        for (uint32_t j = 0; j < nc; j++) x = ff_add(x, stage_value(m, m->ch[f + j]));
+        for (uint32_t j = 0; j < nc; j++) x = ff_add(x, stage_value(m, m.ch[f + j]));
       } else {
         x = ff{kd == 4 ? 1.0f : 0.0f, 0.0f};
       }
-      m->hi[i] = x.hi;
-      m->lo[i] = x.lo;
-      if constexpr (GRAD) m->adj[i] = 0.0f;
+      m.hi[i] = x.hi;
+      m.lo[i] = x.lo;
+      if constexpr (GRAD) m.adj[i] = 0.0f;
     }
     __syncthreads();
   }
   if constexpr (!GRAD) {
     if (threadIdx.x == 0) {
-      const uint32_t kd = m->kind[root], f = m->a[root] & 0xffffu, nc = m->a[root] >> 16;
+      const uint32_t kd = m.kind[root], f = m.a[root] & 0xffffu, nc = m.a[root] >> 16;
       double x = ff_to_f64(stage_value(m, root));
       if (kd == 2) {
         x = 1.0;
-        for (uint32_t j = 0; j < nc; j++) x = x * ff_to_f64(stage_value(m, m->ch[f + j]));
+        for (uint32_t j = 0; j < nc; j++) x = x * ff_to_f64(stage_value(m, m.ch[f + j]));
       } else if (kd == 3) {
         x = 0.0;
-        for (uint32_t j = 0; j < nc; j++) x = x + ff_to_f64(stage_value(m, m->ch[f + j]));
+        for (uint32_t j = 0; j < nc; j++) x = x + ff_to_f64(stage_value(m, m.ch[f + j]));
       }
       if (out32) out32[q] = (float)x;
       if (out64) out64[q] = x;
     }
   } else {
-    if (threadIdx.x == 0) m->adj[root] = seed ? seed[q] : 1.0f;
+    if (threadIdx.x == 0) m.adj[root] = seed ? seed[q] : 1.0f;
     __syncthreads();
     for (uint32_t L = levels; L > 0; L--) {
       for (uint32_t i = lvl[L - 1] + threadIdx.x; i < lvl[L]; i += CK_NT) {
-        const float gi = m->adj[i];
+        const float gi = m.adj[i];
         if (gi == 0.0f) continue;
-        const uint32_t kd = m->kind[i], a = m->a[i];
+        const uint32_t kd = m.kind[i], a = m.a[i];
         const uint32_t f = a & 0xffffu, nc = a >> 16;
         if (kd == 0) {
           atomicAdd(&g_out[a], (double)gi);
@@ -502,22 +515,22 @@ __global__ void __launch_bounds__(CK_NT) k_circuit_staged(strata_circuits c, con
           atomicAdd(&g_out[a], -(double)gi);
         } else if (kd == 2) {
           for (uint32_t j = 0; j < nc; j++) {
-            const uint32_t cj = m->ch[f + j], kj = m->kind[cj];
+            const uint32_t cj = m.ch[f + j], kj = m.kind[cj];
             if (kj == 0 || kj == 1) {
               ff sib{1.0f, 0.0f};  // a leaf child: its term in FP64
               for (uint32_t k = 0; k < nc; k++)
-                if (k != j) sib = ff_mul(sib, stage_value(m, m->ch[f + k]));
+                if (k != j) sib = ff_mul(sib, stage_value(m, m.ch[f + k]));
               const double t = (double)gi * ff_to_f64(sib);
-              atomicAdd(&g_out[m->a[cj]], kj == 0 ? t : -t);
+              atomicAdd(&g_out[m.a[cj]], kj == 0 ? t : -t);
             } else {
               float sib = 1.0f;
               for (uint32_t k = 0; k < nc; k++)
-                if (k != j) sib = sib * m->hi[m->ch[f + k]];
-              atomicAdd(&m->adj[cj], gi * sib);
+                if (k != j) sib = sib * m.hi[m.ch[f + k]];
+              atomicAdd(&m.adj[cj], gi * sib);
             }
           }
         } else if (kd == 3) {
-          for (uint32_t j = 0; j < nc; j++) atomicAdd(&m->adj[m->ch[f + j]], gi);
+          for (uint32_t j = 0; j < nc; j++) atomicAdd(&m.adj[m.ch[f + j]], gi);
         }
       }
       __syncthreads();
@@ -525,12 +538,24 @@ __global__ void __launch_bounds__(CK_NT) k_circuit_staged(strata_circuits c, con
   }
 }
 
+// Whether a set takes the staged form: while two blocks of its largest circuit
+// fit an SM, or one where there are no more queries than SMs.  One B200, values
+// and gradients in us, staged / not, 1,024 queries of which one (or all) has
+// the given nodes: 1,800 91 / 153 (231 / 275), 3,000 104 / 162 (290 / 372),
+// 4,700 149 / 180 (709 / 828); one block an SM: 6,800 225 / 199 (643 / 962).
+// 128 queries of 9,500 nodes 168 / 280.
+bool staged(const strata_ctx* ctx, const strata_circuits& c, bool grad) {
+  const size_t limit = c.n_queries <= (uint32_t)ctx->num_sms ? 226 * 1024 : 112 * 1024;
+  return stage_bytes(c.max_nodes, c.max_children, grad) <= limit && c.max_nodes < 65536 && c.max_children < 65536;
+}
+
 template <bool GRAD>
 void launch_staged(strata_ctx* ctx, const strata_circuits& c, const float* p, float* out32, double* out64,
                    const float* seed, double* grad) {
   auto* kern = k_circuit_staged<GRAD>;
-  SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StageMem)));
-  kern<<<c.n_queries, CK_NT, sizeof(StageMem), ctx->stream>>>(c, p, out32, out64, seed, grad);
+  const size_t smem = stage_bytes(c.max_nodes, c.max_children, GRAD);
+  SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<c.n_queries, CK_NT, smem, ctx->stream>>>(c, p, out32, out64, seed, grad);
   after_launch(ctx, "k_circuit_staged");
 }
 
@@ -701,8 +726,10 @@ strata_circuits* circuits_upload(strata_ctx* ctx, const std::vector<const std::v
   c->n_leaves = n_leaves;
   c->n_nodes = qnode[nq];
   c->max_levels = max_levels;
-  for (uint32_t q = 0; q < nq; q++)
-    c->max_query = std::max<uint64_t>(c->max_query, std::max(qnode[q + 1] - qnode[q], qch[q + 1] - qch[q]));
+  for (uint32_t q = 0; q < nq; q++) {
+    c->max_nodes = std::max<uint32_t>(c->max_nodes, (uint32_t)(qnode[q + 1] - qnode[q]));
+    c->max_children = std::max<uint32_t>(c->max_children, (uint32_t)(qch[q + 1] - qch[q]));
+  }
   c->n_children = total_ch;
   try {
     c->kind = dev_upload(ctx, kind.get(), qnode[nq]);
@@ -810,7 +837,7 @@ void circuits_free(strata_ctx* ctx, strata_circuits* c) {
 void circuits_forward(strata_ctx* ctx, const strata_circuits* c, const float* d_p, float* out32, double* out64) {
   if (!c->n_queries) return;
   const int kh = kprof_begin(ctx, K_CIRCUIT);
-  if (c->max_query <= kStageNodes) {
+  if (staged(ctx, *c, false)) {
     launch_staged<false>(ctx, *c, d_p, out32, out64, nullptr, nullptr);
   } else {
     k_circuit_forward<<<c->n_queries, CK_NT, 0, ctx->stream>>>(*c, d_p, out32, out64);
@@ -829,7 +856,7 @@ void circuits_adjoint(strata_ctx* ctx, const strata_circuits* c, const float* d_
   if (c->n_queries) {
     // the per-query rows keep the order of their node sums (FP32 atomics in
     // global memory): they are compared in FP64
-    if (!per_query && c->max_query <= kStageNodes) {
+    if (!per_query && staged(ctx, *c, true)) {
       const int kh = kprof_begin(ctx, K_CIRCUIT);
       launch_staged<true>(ctx, *c, d_p, nullptr, nullptr, seed, grad);
       kprof_end(ctx, kh, c->n_nodes * (1 + 4 + 4 + 4 + 4) + c->n_children * 12);

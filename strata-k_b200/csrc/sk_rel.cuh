@@ -25,7 +25,7 @@ struct strata_circuits {
   uint32_t n_leaves = 0;
   uint64_t n_nodes = 0;
   uint32_t max_levels = 0;
-  uint64_t max_query = 0;       // nodes, or children, of the largest query
+  uint32_t max_nodes = 0, max_children = 0;  // of any one query
   // device arrays
   uint8_t* kind = nullptr;      // 0 leaf, 1 neg leaf, 2 and, 3 or, 4 true, 5 false
   uint32_t* a = nullptr;        // leaf index, or first child (index into `ch`)
