@@ -448,11 +448,23 @@ __global__ void __launch_bounds__(NT) k_md_bounds(const K* __restrict__ A, uint6
 // against 3.2 M candidates of 16 bytes, one B200: a binary search per row in
 // a counting and a writing pass 225 us, this merge in two passes 140, in one
 // 125, with the rows in place and output rows by their 16-bit number (half the
-// shared memory, 40 registers, six blocks an SM instead of four) 105; tiles of
+// shared memory: five blocks an SM instead of four) 105; tiles of
 // 1,024 / 1,536 / 2,048 / 2,560 / 3,584 rows 126 / 105 / 105 / 106 / 122, and
 // six merges of sparse paths over 200 k nodes 595 / 518 / 461 / 475 / 591.
+template <class K, class W, bool TROP>
+constexpr uint32_t md_smem() {  // the rows, and two 16-bit row numbers each
+  return (MD_TILE + 2) * (uint32_t)(sizeof(K) + (TROP ? sizeof(W) : 0) + 2 * sizeof(uint16_t));
+}
+// Resident blocks that registers are kept for: as many as the 228 KB of an SM
+// hold with 1 KB of reserve and the static part each, six at most.
+template <class K, class W, bool TROP>
+constexpr int md_blocks() {
+  const int fit = (int)(228u * 1024u / (md_smem<K, W, TROP>() + 1024u + 64u));
+  return fit < 6 ? fit : 6;
+}
+static_assert(md_blocks<uint64_t, int64_t, true>() == 5 && md_blocks<uint64_t, int32_t, true>() == 6, "");
 template <class K, class W, bool TROP, bool WRITE_FULL, bool WRITE_DELTA, bool INPLACE>
-__global__ void __launch_bounds__(NT, 6)
+__global__ void __launch_bounds__(NT, md_blocks<K, W, TROP>())
     k_merge_diff(const K* __restrict__ A, W* Aw, uint64_t na, const K* __restrict__ B,
                  const W* __restrict__ Bw, uint64_t nb, K* __restrict__ fout, W* __restrict__ fout_w,
                  K* __restrict__ dout, W* __restrict__ dout_w, const uint64_t* __restrict__ splits,
@@ -1046,8 +1058,7 @@ static void launch_merge(strata_ctx* ctx, const K* full, W* full_w, uint64_t nf,
   k_md_bounds<K><<<(unsigned)ceil_div((uint64_t)tiles + 1, NT / 32), NT, 0, ctx->stream>>>(full, nf, cand, nc, tiles,
                                                                                            splits);
   after_launch(ctx, "k_md_bounds");
-  constexpr uint32_t CAP = MD_TILE + 2;
-  const size_t smem = CAP * (sizeof(K) + (TROP ? sizeof(W) : 0) + 2 * sizeof(uint16_t));
+  const size_t smem = md_smem<K, W, TROP>();
   auto kern = k_merge_diff<K, W, TROP, WF, WD, IP>;
   SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int kh = kprof_begin(ctx, K_MERGE_DIFF);
