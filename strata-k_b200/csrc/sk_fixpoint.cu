@@ -328,6 +328,10 @@ struct DenseIdx {
   DenseLayout lay{};
   uint64_t entries = 0;
   uint64_t words() const { return entries / 32; }
+  void release_heads() {
+    for (auto* b : {&hidx, &hmask, &hseg}) b->release();
+    hpos.release();
+  }
 };
 
 // Bytes the index needs (D and Dprev at `wbytes` per entry for Trop, the
@@ -402,9 +406,10 @@ uint64_t dense_round_keys(strata_ctx* ctx, const K* dk, const W* dw, uint64_t nd
   return cands;
 }
 
+constexpr int kGroupRounds = 8;  // enqueued between two looks at their totals
 template <bool TROP, class W>
 void fix_loop_queued(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, DenseIdx<W>& X, uint64_t cap,
-                     PhaseTimer& pt, Acct& a, uint64_t* rounds_out);
+                     DBuf<uint64_t>& totals, PhaseTimer& pt, Acct& a, uint64_t* rounds_out);
 
 // Semi-naive rounds with Δ in the marks: word heads (which clear the marks
 // and snapshot Δ's weights), then the expand marks Δ'.  A round runs while
@@ -412,12 +417,22 @@ void fix_loop_queued(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, Den
 template <bool TROP, class W>
 void fix_loop_dense(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, DenseIdx<W>& X, uint64_t bound,
                     uint64_t cap, PhaseTimer& pt, Acct& a, uint64_t* rounds_out) {
-  // the queued rounds hold a head per marks word: under a memory cap only where those fit
-  const uint64_t heads = X.words() + 1;
-  if (dense_rounds_queued(X.lay, csr.m) &&
-      (!ctx->cap || ctx->in_use + 3 * size_class(heads * 4) + size_class(heads * 8) + size_class(4096) <= ctx->cap)) {
-    fix_loop_queued<TROP, W>(ctx, csr, js, X, cap, pt, a, rounds_out);
-    return;
+  // the queued rounds hold a head per marks word: only where that memory can be had
+  if (dense_rounds_queued(X.lay, csr.m)) {
+    DBuf<uint64_t> totals;
+    totals.ctx = ctx;
+    const uint64_t heads = X.words() + 1;
+    if (with_memory([&] {
+          X.hidx.reserve(heads);
+          X.hmask.reserve(heads);
+          X.hseg.reserve(heads);
+          X.hpos.reserve(heads);
+          totals.reserve(kGroupRounds * 4 + 1);
+        })) {
+      fix_loop_queued<TROP, W>(ctx, csr, js, X, cap, totals, pt, a, rounds_out);
+      return;
+    }
+    X.release_heads();
   }
   DBuf<uint64_t> splits;
   splits.ctx = ctx;
@@ -462,29 +477,22 @@ void fix_loop_dense(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, Dens
   *rounds_out = rounds;
 }
 
-// The same rounds in groups: the host enqueues up to kGroup rounds and looks
+// The same rounds in groups: the host enqueues up to kGroupRounds and looks
 // at their totals once.  A round whose Δ is empty costs two empty launches.
 // At the cap the last round's Δ is only counted (its expand would run past
 // the point where the interpreter stops).
 template <bool TROP, class W>
 void fix_loop_queued(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, DenseIdx<W>& X, uint64_t cap,
-                     PhaseTimer& pt, Acct& a, uint64_t* rounds_out) {
-  constexpr int kGroup = 8;
-  const uint64_t hcap = X.words() + 1;
-  X.hidx.reserve(hcap);
-  X.hmask.reserve(hcap);
-  X.hseg.reserve(hcap);
-  X.hpos.reserve(hcap);
-  DBuf<uint64_t> totals(ctx, kGroup * 4 + 1);
+                     DBuf<uint64_t>& totals, PhaseTimer& pt, Acct& a, uint64_t* rounds_out) {
   const uint64_t wsz = TROP ? sizeof(W) : 0;
   uint64_t rounds = 0;
   for (bool more = true; more;) {
     const uint64_t l0 = ctx->launches;
     const int t = pt.begin(&a.join_ms);
     // rounds that may still run: the (cap + 1)-th is counted, not expanded
-    const uint64_t left = TROP && cap ? cap + 1 - rounds : kGroup;
-    const int count = (int)std::min<uint64_t>(kGroup, left);
-    const int expands = TROP && cap && left <= (uint64_t)kGroup ? count - 1 : count;
+    const uint64_t left = TROP && cap ? cap + 1 - rounds : kGroupRounds;
+    const int count = (int)std::min<uint64_t>(kGroupRounds, left);
+    const int expands = TROP && cap && left <= (uint64_t)kGroupRounds ? count - 1 : count;
     const size_t rec0 = ctx->krecs.size();
     dense_queue_rounds<TROP, W>(ctx, X.marks.p, X.lay, csr.off.p, csr.n_nodes, X.hidx.p, X.hmask.p, X.hpos.p,
                                 X.hseg.p, TROP ? X.D.p : nullptr, TROP ? X.Dprev.p : nullptr, js.out_pshift,
@@ -511,8 +519,7 @@ void fix_loop_queued(strata_ctx* ctx, const Csr<W>& csr, const JoinSpec& js, Den
       fail(STRATA_E_NEG_CYCLE, "negative-weight cycle: tropical stratum diverges");
   }
   // a head per word is more than the rounds one by one would hold: not while the result is built
-  for (auto* b : {&X.hidx, &X.hmask, &X.hseg}) b->release();
-  X.hpos.release();
+  X.release_heads();
   *rounds_out = rounds;
 }
 

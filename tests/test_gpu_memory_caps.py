@@ -68,3 +68,39 @@ def test_closure_gives_way_to_the_tuple_plan(engine):
             assert _same(small.transitive_closure_bool((s, s + 1)), want)
         with Engine(0, mem_cap=cap) as small:
             assert _same(small.transitive_closure_bool((s, s + 1)), want), cap
+
+
+def _calls():
+    s, d, w = _graph(2500, 2700)  # queued rounds: heads for 2,500 * 79 words
+    t = _graph(700, 2000, 2)
+    rng = np.random.default_rng(4)
+    hub = tuple((rng.random(60_000) ** 3 * 3000).astype(np.uint32) for _ in range(2))  # hub rows from 2^15 edges on
+    small = _graph(300, 700, 5)[:2]  # one-block closure
+    rows = _graph(3000, 5000, 6)[:2]
+    return {"sparse paths": lambda e: e.shortest_paths_trop((s, d, w)), "paths": lambda e: e.shortest_paths_trop(t),
+            "mssp": lambda e: e.mssp_trop([1, 2, 3], (s, d, w)), "small closure": lambda e: e.transitive_closure_bool(small),
+            "closure": lambda e: e.transitive_closure_bool(rows), "triangles": lambda e: e.count_triangles(hub)}
+
+
+@pytest.mark.parametrize("name", list(_calls()))
+def test_more_memory_never_fails(engine, name):
+    # a form chosen because its estimate fits, and that then does not, would
+    # fail above a cap at which a smaller form ran
+    from strata_b200 import Engine
+    from strata_b200.gpu import OutOfMemory
+    call = _calls()[name]
+    want = call(engine)
+    with Engine(0) as eng:
+        call(eng)
+        peak = eng.mem()[1]
+    ran = False
+    for cap in np.geomspace(peak / 40, peak * 1.1, 60).astype(int).tolist() + [peak]:
+        with Engine(0, mem_cap=cap) as eng:
+            try:
+                got = call(eng)
+            except OutOfMemory:
+                assert not ran, (cap, peak)
+                continue
+            ran = True
+            assert got == want if isinstance(want, int) else _same(got, want)
+    assert ran
