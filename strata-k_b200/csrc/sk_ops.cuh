@@ -167,14 +167,15 @@ template <class K, class W, bool TROP>
 void diff_improve(strata_ctx* ctx, const K* cand, const W* cand_w, uint64_t nc, const K* full,
                   W* full_w, uint64_t nf, K* out, W* out_w, uint64_t* d_count);
 
-// CSR offsets from keys sorted by (join << vbits) | v:
-// off[j] = first index with join >= j, for j in [0, n_nodes]; nbr[i] = key & vmask.
-// The two halves of build_csr; op_w (optional): the rows' operator-surface
-// weights, checked on the way (a finite one without a code sets the status).
+// A CSR over keys sorted by (join << vbits) | v, in two halves.
+// off[j] = first index with join >= j, for j in [0, n_nodes].
 template <class K>
 void csr_offsets(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint64_t n_nodes, uint32_t* off);
+// nbr[i] = v of key i.  op_w (optional): the rows' operator-surface weights,
+// checked on the way (a finite one without a code sets the status).
 template <class K>
 void csr_neighbours(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint32_t* nbr, const int64_t* op_w);
+// Both halves, without weights.
 template <class K>
 void build_csr(strata_ctx* ctx, const K* keys, uint64_t m, int vbits, uint64_t n_nodes,
                uint32_t* off, uint32_t* nbr);
