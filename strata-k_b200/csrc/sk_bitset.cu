@@ -1321,7 +1321,7 @@ uint64_t tc_bool_small(strata_ctx* ctx, const uint32_t* d_src, const uint32_t* d
   out.reserve(n_src * n_dst + 1);
   DBuf<uint64_t> res(ctx, 2);
   const size_t smem = small_smem(n_src, ceil_div(n_dst, 32), m);
-  SK_CUDA(cudaFuncSetAttribute(k_bs_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(k_bs_small, kSmallSmem);
   k_bs_small<<<1, SM_NT, smem, ctx->stream>>>(d_src, d_dst, (uint32_t)m, (uint32_t)n_src, (uint32_t)n_dst, b1, out.p,
                                               res.p);
   after_launch(ctx, "k_bs_small");

@@ -544,8 +544,9 @@ __global__ void __launch_bounds__(CK_NT) k_circuit_staged(strata_circuits c, con
 // the given nodes: 1,800 91 / 153 (231 / 275), 3,000 104 / 162 (290 / 372),
 // 4,700 149 / 180 (709 / 828); one block an SM: 6,800 225 / 199 (643 / 962).
 // 128 queries of 9,500 nodes 168 / 280.
+constexpr size_t kStageOne = 226 * 1024, kStageTwo = 112 * 1024;  // of shared memory, one and two blocks an SM
 bool staged(const strata_ctx* ctx, const strata_circuits& c, bool grad) {
-  const size_t limit = c.n_queries <= (uint32_t)ctx->num_sms ? 226 * 1024 : 112 * 1024;
+  const size_t limit = c.n_queries <= (uint32_t)ctx->num_sms ? kStageOne : kStageTwo;
   return stage_bytes(c.max_nodes, c.max_children, grad) <= limit && c.max_nodes < 65536 && c.max_children < 65536;
 }
 
@@ -554,7 +555,7 @@ void launch_staged(strata_ctx* ctx, const strata_circuits& c, const float* p, fl
                    const float* seed, double* grad) {
   auto* kern = k_circuit_staged<GRAD>;
   const size_t smem = stage_bytes(c.max_nodes, c.max_children, GRAD);
-  SK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  allow_smem(kern, kStageOne);
   kern<<<c.n_queries, CK_NT, smem, ctx->stream>>>(c, p, out32, out64, seed, grad);
   after_launch(ctx, "k_circuit_staged");
 }

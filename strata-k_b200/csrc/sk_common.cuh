@@ -329,6 +329,15 @@ inline void read_u64(strata_ctx* ctx, const uint64_t* d, uint64_t* out, int coun
   std::memcpy(out, ctx->h_scalar, sizeof(uint64_t) * count);
 }
 
+// Let launches of `kern` ask for up to `most` bytes of dynamic shared memory.
+// The limit belongs to the kernel on the device, for every context and thread:
+// a call states the most that any call may ask for, never its own need, which
+// could fall below another thread's between that one's check and its launch.
+template <class F>
+inline void allow_smem(F* kern, size_t most) {
+  check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most), "cudaFuncSetAttribute");
+}
+
 inline void after_launch(strata_ctx* ctx, const char* name) {
   ctx->launches++;
   cudaError_t e = cudaGetLastError();

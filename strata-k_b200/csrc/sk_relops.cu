@@ -1132,9 +1132,9 @@ uint64_t count_distinct_ids(strata_ctx* ctx, const uint32_t* a, uint64_t na, con
   const uint32_t* cols[3] = {a, b, c};
   const uint64_t ns[3] = {na, nb, nc};
   const size_t smem = words * 4;
-  const bool private_bm = smem <= 160 * 1024;
-  if (private_bm)
-    SK_CUDA(cudaFuncSetAttribute(k_mark_ids_smem, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  constexpr size_t kPrivate = 160 * 1024;
+  const bool private_bm = smem <= kPrivate;
+  if (private_bm) allow_smem(k_mark_ids_smem, kPrivate);
   for (int q = 0; q < 3; q++) {
     if (!cols[q] || !ns[q]) continue;
     if (private_bm) {

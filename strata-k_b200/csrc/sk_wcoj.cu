@@ -1139,7 +1139,7 @@ uint64_t k4_impl(strata_ctx* ctx, const uint32_t* a, const uint32_t* b, uint64_t
   const uint64_t grid_cap = (uint64_t)ctx->num_sms * 8;
   auto launch = [&](uint32_t d_lo, uint32_t d_hi, uint32_t cap, int warps, uint32_t* counter) {
     const size_t smem = (size_t)warps * 2 * cap * 4;
-    SK_CUDA(cudaFuncSetAttribute(k_k4_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(k_k4_warp, kSmemLimit);
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(ceil_div(n_nodes, warps), grid_cap));
     k_k4_warp<<<grid, warps * 32, smem, ctx->stream>>>(off.p, nbr.p, n_nodes, d_lo, d_hi, cap, counter,
                                                        reinterpret_cast<unsigned long long*>(acc.p));
