@@ -43,6 +43,7 @@
 #include <exception>
 #include <map>
 #include <memory>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -646,27 +647,37 @@ static void compile_query(const uint64_t* proof_off, const uint64_t* lit_off, co
   out.levels = top + 1;
 }
 
-// fn(i) for i in [0, n) on the host threads, the first exception rethrown.
+// fn(i) for i in [0, n) on this thread and as many more as the host gives, the
+// first exception rethrown.  No thread is left joinable: a thread that cannot
+// be started would otherwise end the program.
 template <class Fn>
 static void host_parallel(uint32_t n, Fn fn) {
   const unsigned hw = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
   const unsigned T = std::min<unsigned>(hw, std::max<uint32_t>(1, n));
   std::atomic<uint32_t> next{0};
   std::vector<std::exception_ptr> errs(T);
-  std::vector<std::thread> th;
-  for (unsigned t = 0; t < T; t++)
-    th.emplace_back([&, t]() {
-      try {
-        while (true) {
-          const uint32_t q = next.fetch_add(1);
-          if (q >= n) break;
-          fn(q);
-        }
-      } catch (...) {
-        errs[t] = std::current_exception();
-        next.store(n);
+  auto work = [&](unsigned t) {
+    try {
+      while (true) {
+        const uint32_t q = next.fetch_add(1);
+        if (q >= n) break;
+        fn(q);
       }
-    });
+    } catch (...) {
+      errs[t] = std::current_exception();
+      next.store(n);
+    }
+  };
+  std::vector<std::thread> th;
+  th.reserve(T);
+  for (unsigned t = 1; t < T; t++) {
+    try {
+      th.emplace_back(work, t);
+    } catch (const std::system_error&) {
+      break;
+    }
+  }
+  work(0);
   for (auto& x : th) x.join();
   for (auto& e : errs)
     if (e) std::rethrow_exception(e);
